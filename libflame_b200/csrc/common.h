@@ -187,11 +187,20 @@ int status_read(int* info);
 //   mode LOWER: only C(i,j) with i - j >= diag_off are written (SYRK-style),
 //   tiles entirely above are skipped.
 // ---------------------------------------------------------------------------
+// Space for the partial products of a split-K GEMM, owned by the caller (one
+// per stream that may run such a GEMM).
+struct GemmSplit {
+  double* p = nullptr;
+  size_t elems = 0;
+};
 enum GemmMode : int { GEMM_FULL = 0, GEMM_LOWER = 1 };
 int gemm_f64(cudaStream_t st, bool ta, bool tb, long m, long n, long k, double alpha,
              const double* A, long lda, const double* B, long ldb, double beta, double* C,
              long ldc, GemmMode mode = GEMM_FULL, long diag_off = 0,
-             const int* guard = nullptr, int guard_limit = 0x7fffffff, long kmax = 0);
+             const int* guard = nullptr, int guard_limit = 0x7fffffff, long kmax = 0,
+             const GemmSplit* split = nullptr);
+// split (full mode, no guard): an output of few tiles is split over k to fill
+// the GPU, its partial products in the caller's space (as many slices as fit).
 // kmax > 0 (full mode only): split k so that no CTA runs more than about
 // kmax of it, for GEMMs whose long-running tiles would keep SMs from a
 // cluster kernel waiting on the other stream.

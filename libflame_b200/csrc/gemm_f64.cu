@@ -494,7 +494,8 @@ int tile_bm() {
 
 int gemm_f64(cudaStream_t st, bool ta, bool tb, long m, long n, long k, double alpha,
              const double* A, long lda, const double* B, long ldb, double beta, double* C,
-             long ldc, GemmMode mode, long diag_off, const int* guard, int guard_limit, long kmax) {
+             long ldc, GemmMode mode, long diag_off, const int* guard, int guard_limit, long kmax,
+             const GemmSplit* split) {
   if (m <= 0 || n <= 0) return FLA_SUCCESS;
   if (k <= 0 || alpha == 0.0) {
     // C := beta*C only; k == 0 never occurs on the factorization path with
@@ -559,7 +560,22 @@ int gemm_f64(cudaStream_t st, bool ta, bool tb, long m, long n, long k, double a
   long S = 1, kc = 0, ldp = 0, zs = 0;
   double* Pz = nullptr;
   const bool capped = mode == GEMM_FULL && !guard && kmax > 0 && k > kmax;
-  if (mode == GEMM_FULL && !guard && (((tiles * 2 <= sms || narrow) && k >= 2048) || capped)) {
+  if (split && mode == GEMM_FULL && !guard) {
+    // The caller's space: slices down to 128 of k (eight stages: below that
+    // a tile's prologue and epilogue outweigh its products), as many as fill
+    // the four CTAs an SM holds.
+    ldp = (m + 1) & ~1L;
+    zs = ldp * n;
+    S = std::min<long>(std::min<long>(4L * sms / tiles, k / 128), (long)(split->elems / (size_t)zs));
+    if (S > 1) {
+      kc = ((k + S - 1) / S + BK - 1) / BK * BK;
+      S = (k + kc - 1) / kc;
+      Pz = split->p;
+      grid.z = (unsigned)S;
+    } else {
+      S = 1;
+    }
+  } else if (mode == GEMM_FULL && !guard && (((tiles * 2 <= sms || narrow) && k >= 2048) || capped)) {
     S = std::min<long>(std::min<long>(((narrow ? 4L : 2L) * sms + tiles - 1) / tiles, k / 512), 64);
     if (capped) S = std::min<long>(std::max<long>(S, (k + kmax - 1) / kmax), 64);
     if (S > 1) {

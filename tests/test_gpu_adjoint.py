@@ -40,6 +40,28 @@ def test_chol_adjoint_closed_form(cuda, flame, oracle, n):
     assert np.array_equal(np.triu(to_host(Bd), 1), np.triu(to_dev(cuda, Lbar).cpu().numpy(), 1))
 
 
+# Orders at which the block below is ragged, the products over the rows below
+# a block are split over k (from 256 rows) and the last block has one column;
+# an odd leading dimension is realigned behind the call.  Tolerance: as above.
+@pytest.mark.parametrize("n", [257, 385, 1001, 2305])
+def test_chol_adjoint_split_products(cuda, flame, n):
+    torch = cuda
+    g = torch.Generator(device="cuda").manual_seed(n)
+    G = torch.randn((n, n), dtype=torch.float64, device="cuda", generator=g)
+    L = torch.linalg.cholesky(G @ G.t() / n + torch.eye(n, dtype=torch.float64, device="cuda"))
+    Lbar = torch.randn((n, n), dtype=torch.float64, device="cuda", generator=g)
+    Ld, Bd = L.t().contiguous().clone().t(), Lbar.t().contiguous().clone().t()
+    Ld += torch.triu(torch.full_like(L, float("nan")), 1)  # never read
+    assert flame.chol_adjoint(Ld, Bd) == flame.FLA_SUCCESS, flame.last_error()
+    P = torch.tril(L.t() @ torch.tril(Lbar))
+    P.diagonal().mul_(0.5)
+    Li = torch.linalg.solve_triangular(L, torch.eye(n, dtype=torch.float64, device="cuda"), upper=False)
+    S = 0.5 * Li.t() @ (P + P.t()) @ Li
+    Ab = torch.tril(Bd)
+    assert ((0.5 * (Ab + Ab.t()) - S).norm() / S.norm()).item() < 1e-10
+    assert torch.equal(torch.triu(Bd, 1), torch.triu(Lbar, 1))
+
+
 def test_chol_adjoint_finite_differences(cuda, flame, oracle):
     n, h = 96, 1e-6
     rng = seeded(17)
