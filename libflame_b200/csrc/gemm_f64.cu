@@ -298,6 +298,173 @@ __global__ void __launch_bounds__(Tile<BM_, BN_>::THREADS, Tile<BM_, BN_>::MINB)
   }
 }
 
+
+// The same product for outputs of few tiles, where one 64 x 64 tile per SM
+// leaves most SMs idle and a chain of such products (the factorizations'
+// panel joins and lookahead updates, the solves) waits for one tile's k
+// loop: 32 x 32 tiles, four times as many CTAs, and the four warps of a CTA
+// share each 16 of k (warp w takes 4w..4w+3 for the whole tile), so these cost
+// each SM sub-partition 16 DMMAs instead of 64.  The four partial tiles are
+// added through shared memory in warp order.  Four stages of 32 k (64 KB,
+// three CTAs per SM): a depth of 128 is in flight at once, and a barrier wait
+// is paid every 32 k only.  C is read into registers
+// before the k loop.  Measured, one call between events (an empty one is
+// about 5 us), 64 x 64 tiles against these: 896 x 128 x 128 16.8 -> 8.9 us,
+// 768 x 256 x 256 25.1 -> 12.8, 1536 x 256 x 128 16.7 -> 11.2; past the
+// limit 2048 x 768 x 128 (384 tiles) 25.9 -> 31.6.
+constexpr int SM_T = 32, SM_STAGES = 4, SM_BK = 2 * BK;
+constexpr int SM_A_BYTES = SM_T * BK * 8, SM_HALF_BYTES = 2 * SM_A_BYTES, SM_STAGE_BYTES = 2 * SM_HALF_BYTES;
+constexpr int SM_SMEM = SM_STAGES * SM_STAGE_BYTES + 2048 /*align*/ + 256 /*barriers*/;
+template <bool A_K, bool B_K>
+__global__ void __launch_bounds__(128) dgemm_small_kernel(const __grid_constant__ CUtensorMap mapA,
+                                                          const __grid_constant__ CUtensorMap mapB,
+                                                          double* __restrict__ C, long ldc, int M, int N, int K,
+                                                          double alpha, double beta, int mode, long diag_off, int* err,
+                                                          const int* guard, int guard_limit, int k_chunk,
+                                                          long c_zstride) {
+  extern __shared__ unsigned char smem_raw[];
+  if (guard && *((volatile const int*)guard) < guard_limit) return;
+  const int tile_m = blockIdx.x * SM_T, tile_n = blockIdx.y * SM_T;
+  if (mode == GEMM_LOWER && (long)tile_m + SM_T - 1 - tile_n < diag_off) return;
+  const uintptr_t base = (reinterpret_cast<uintptr_t>(smem_raw) + 2047) & ~uintptr_t(2047);
+  unsigned char* sm = reinterpret_cast<unsigned char*>(base);
+  const uint32_t sm_base = smem_u32(sm);
+  const uint32_t full0 = sm_base + SM_STAGES * SM_STAGE_BYTES, empty0 = full0 + 8 * SM_STAGES;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int ks = blockIdx.z * k_chunk;
+  const int Kz = k_chunk ? min(K - ks, k_chunk) : K;
+  C += (long)blockIdx.z * c_zstride;
+  const int KT = (Kz + SM_BK - 1) / SM_BK;
+  if (tid == 0) {
+    for (int s = 0; s < SM_STAGES; ++s) {
+      mbar_init(full0 + 8 * s, 1);
+      mbar_init(empty0 + 8 * s, 4);
+    }
+    fence_barrier_init();
+  }
+  __syncthreads();
+  // stage: two 16-wide k halves, each A (32 x 16) then B; a half past the end
+  // of k reads zeros (the map's fill), one inside another slice its values,
+  // so slices are multiples of SM_BK
+  auto issue = [&](int kt) {
+    const int st = kt % SM_STAGES;
+    const uint32_t fb_ = full0 + 8 * st;
+    mbar_arrive_expect_tx(fb_, SM_STAGE_BYTES);
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const uint32_t dA = sm_base + st * SM_STAGE_BYTES + u * SM_HALF_BYTES, dB = dA + SM_A_BYTES;
+      const int k0 = ks + kt * SM_BK + u * BK;
+      if (A_K) {
+        tma_load_2d(dA, &mapA, k0, tile_m, fb_);  // box {16 k, 32 m}
+      } else {
+        tma_load_2d(dA, &mapA, tile_m, k0, fb_);
+        tma_load_2d(dA + BK * 128, &mapA, tile_m + 16, k0, fb_);
+      }
+      if (B_K) {
+        tma_load_2d(dB, &mapB, k0, tile_n, fb_);
+      } else {
+        tma_load_2d(dB, &mapB, tile_n, k0, fb_);
+        tma_load_2d(dB + BK * 128, &mapB, tile_n + 16, k0, fb_);
+      }
+    }
+  };
+  int issued = 0;
+  if (tid == 0)
+    for (; issued < SM_STAGES && issued < KT; ++issued) issue(issued);
+  // this thread's elements of C: row tile_m + lane, columns tile_n + warp + 4 q
+  const int row = tile_m + lane;
+  double cv[8];
+  bool ok_c[8];
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    const int col = tile_n + warp + 4 * q;
+    ok_c[q] = row < M && col < N && (mode != GEMM_LOWER || (long)row - (long)col >= diag_off);
+    cv[q] = (ok_c[q] && beta != 0.0) ? C[(long)row + (long)col * ldc] : 0.0;
+  }
+  const int g = lane >> 2, t = lane & 3;
+  uint32_t aoff[4], boff[4];
+#pragma unroll
+  for (int f = 0; f < 4; ++f) {
+    const int ra = A_K ? (8 * f + perm8_tab(g)) : (16 * (f >> 1) + perm16_tab(f & 1, g));
+    const int rb = B_K ? (8 * f + perm8_tab(g)) : (16 * (f >> 1) + perm16_tab(f & 1, g));
+    const uint32_t xa = A_K ? (uint32_t)(warp << 5) : (uint32_t)((warp << 9) | ((warp & 1) << 6));
+    const uint32_t xb = B_K ? (uint32_t)(warp << 5) : (uint32_t)((warp << 9) | ((warp & 1) << 6));
+    aoff[f] = (A_K ? base_kcontig(ra, t) : base_rcontig(ra, t)) ^ xa;
+    boff[f] = SM_A_BYTES + ((B_K ? base_kcontig(rb, t) : base_rcontig(rb, t)) ^ xb);
+  }
+  double acc[4][4][2];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+  bool ok = true;
+  for (int kt = 0; kt < KT; ++kt) {
+    const int s = kt % SM_STAGES;
+    if (!mbar_wait(full0 + 8 * s, (kt / SM_STAGES) & 1, err, 12)) { ok = false; break; }
+    const uint32_t tS = sm_base + s * SM_STAGE_BYTES;
+    double a[2][4], b[2][4];
+#pragma unroll
+    for (int u = 0; u < 2; ++u)
+#pragma unroll
+      for (int f = 0; f < 4; ++f) {
+        a[u][f] = lds_f64(tS + u * SM_HALF_BYTES + aoff[f]);
+        b[u][f] = lds_f64(tS + u * SM_HALF_BYTES + boff[f]);
+      }
+#pragma unroll
+    for (int u = 0; u < 2; ++u)
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) dmma_884(acc[i][j][0], acc[i][j][1], a[u][i], b[u][j]);
+    if (kt + SM_STAGES < KT) {
+      // this stage is refilled (see dgemm_tma_kernel for the fences)
+      __threadfence_block();
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive(empty0 + 8 * s);
+      if (tid == 0) {
+        if (!mbar_wait(empty0 + 8 * s, (kt / SM_STAGES) & 1, err, 11)) { ok = false; break; }
+        issue(issued);
+        ++issued;
+      }
+    }
+  }
+  if (!__syncthreads_and(ok ? 1 : 0)) {
+    if (tid == 0)
+      for (int kt = (issued > SM_STAGES ? issued - SM_STAGES : 0); kt < issued; ++kt)
+        mbar_wait(full0 + 8 * (kt % SM_STAGES), (kt / SM_STAGES) & 1, nullptr, 0);
+    return;
+  }
+  // partial tiles through shared memory (every stage has been read): warp w's
+  // at sC + w * 32 * LDC
+  constexpr int LDC = SM_T + 2;
+  double* sC = reinterpret_cast<double*>(sm);
+  {
+    double* p = sC + warp * SM_T * LDC;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int ra = A_K ? (8 * i + perm8_tab(g)) : (16 * (i >> 1) + perm16_tab(i & 1, g));
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const int h = 2 * t + e;
+          const int cb = B_K ? (8 * j + perm8_tab(h)) : (16 * (j >> 1) + perm16_tab(j & 1, h));
+          p[ra + cb * LDC] = acc[i][j][e];
+        }
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    if (!ok_c[q]) continue;
+    const int cl = warp + 4 * q;
+    const double* p = sC + lane + cl * LDC;
+    const double v = alpha * ((p[0] + p[SM_T * LDC]) + (p[2 * SM_T * LDC] + p[3 * SM_T * LDC]));
+    C[(long)row + (long)(tile_n + cl) * ldc] = beta != 0.0 ? fma(beta, cv[q], v) : v;
+  }
+}
+
 // Fallback for operands the TMA path cannot address (a base or leading
 // dimension that is not 16-byte aligned; only small odd-sized blocks at the
 // edge of a factorization reach it): 32x32 C tiles, 16-deep k slices in SMEM,
@@ -390,6 +557,19 @@ void launch(dim3 grid, cudaStream_t st, const CUtensorMap& mA, const CUtensorMap
   dgemm_tma_kernel<A_K, B_K, BM_, BN_><<<grid, Tile<BM_, BN_>::THREADS, Tile<BM_, BN_>::SMEM_BYTES, st>>>(
       mA, mB, C, ldc, (int)m, (int)n, (int)k, alpha, beta, mode, diag_off, err, guard, guard_limit, k_chunk,
       c_zstride);
+}
+
+template <bool A_K, bool B_K>
+void launch_small(dim3 grid, cudaStream_t st, const CUtensorMap& mA, const CUtensorMap& mB, double* C, long ldc,
+                  long m, long n, long k, double alpha, double beta, GemmMode mode, long diag_off, int* err,
+                  const int* guard, int guard_limit, int k_chunk, long c_zstride) {
+  static bool done = false;
+  if (!done) {
+    cudaFuncSetAttribute(dgemm_small_kernel<A_K, B_K>, cudaFuncAttributeMaxDynamicSharedMemorySize, SM_SMEM);
+    done = true;
+  }
+  dgemm_small_kernel<A_K, B_K><<<grid, 128, SM_SMEM, st>>>(mA, mB, C, ldc, (int)m, (int)n, (int)k, alpha, beta, mode,
+                                                           diag_off, err, guard, guard_limit, k_chunk, c_zstride);
 }
 
 // C := alpha * sum_z P_z + beta * C over the S partial products of a split-K
@@ -490,6 +670,15 @@ int tile_bm() {
   return bm;
 }
 
+long small_tiles() {
+  static long v = -1;
+  if (v < 0) {
+    v = 3L * ctx().num_sms / 4;
+    if (const char* e = std::getenv("FLA_B200_GEMM_SMALL_TILES")) v = std::atol(e);
+  }
+  return v;
+}
+
 }  // namespace
 
 int gemm_f64(cudaStream_t st, bool ta, bool tb, long m, long n, long k, double alpha,
@@ -541,59 +730,57 @@ int gemm_f64(cudaStream_t st, bool ta, bool tb, long m, long n, long k, double a
   // products with at most 32 columns and a long k (the refinement residual
   // R = B - A X): 128 x 32 tiles, k split to fill the GPU
   const bool narrow = (n <= 32 && mode == GEMM_FULL && !guard && k >= 2048);
-  const int BMv = narrow ? 128 : tile_bm();
-  const int BNv = narrow ? 32 : BN;
-  bool okA = ta ? make_map(&mA, A, k, m, lda, 16, BMv) : make_map(&mA, A, m, k, lda, 16, BK);
-  bool okB = tb ? make_map(&mB, B, n, k, ldb, 16, BK) : make_map(&mB, B, k, n, ldb, 16, BNv);
-  if (!okA || !okB) {
-    set_last_error("gemm_f64: cuTensorMapEncodeTiled failed");
-    return FLA_FAILURE;
-  }
-  dim3 grid((unsigned)((m + BMv - 1) / BMv), (unsigned)((n + BNv - 1) / BNv));
-  int* err = ctx().d_status + ST_ERROR;
   // Split K when the output has too few tiles to occupy the GPU and K is
   // long (the W = U^T B products of the QR updates and of FLA_Apply_Q_UT):
   // slices of K go to blockIdx.z, each into its own partial product, and one
   // reduction adds them in a fixed order.
-  const long tiles = (long)grid.x * grid.y;
+  const int bm_ = narrow ? 128 : tile_bm(), bn_ = narrow ? 32 : BN;
+  const long tiles = ((m + bm_ - 1) / bm_) * ((n + bn_ - 1) / bn_);
   const int sms = ctx().num_sms;
-  long S = 1, kc = 0, ldp = 0, zs = 0;
+  long S = 1, kc = 0, ldp = (m + 1) & ~1L, zs = ldp * n;
   double* Pz = nullptr;
   const bool capped = mode == GEMM_FULL && !guard && kmax > 0 && k > kmax;
   if (split && mode == GEMM_FULL && !guard) {
     // The caller's space: slices down to 128 of k (eight stages: below that
     // a tile's prologue and epilogue outweigh its products), as many as fill
     // the four CTAs an SM holds.
-    ldp = (m + 1) & ~1L;
-    zs = ldp * n;
     S = std::min<long>(std::min<long>(4L * sms / tiles, k / 128), (long)(split->elems / (size_t)zs));
-    if (S > 1) {
-      kc = ((k + S - 1) / S + BK - 1) / BK * BK;
-      S = (k + kc - 1) / kc;
-      Pz = split->p;
-      grid.z = (unsigned)S;
-    } else {
-      S = 1;
-    }
   } else if (mode == GEMM_FULL && !guard && (((tiles * 2 <= sms || narrow) && k >= 2048) || capped)) {
     S = std::min<long>(std::min<long>(((narrow ? 4L : 2L) * sms + tiles - 1) / tiles, k / 512), 64);
     if (capped) S = std::min<long>(std::max<long>(S, (k + kmax - 1) / kmax), 64);
-    if (S > 1) {
-      kc = ((k + S - 1) / S + BK - 1) / BK * BK;
-      S = (k + kc - 1) / kc;
-      ldp = (m + 1) & ~1L;
-      zs = ldp * n;
-      Pz = (double*)ws_get(st == ctx().side ? WS_SPLITK_SIDE : WS_SPLITK, sizeof(double) * (size_t)(S * zs));
-      if (!Pz) return FLA_FAILURE;
-      grid.z = (unsigned)S;
-    }
   }
+  if (S > 1) {
+    kc = ((k + S - 1) / S + SM_BK - 1) / SM_BK * SM_BK;
+    S = (k + kc - 1) / kc;
+  }
+  if (S > 1) {
+    Pz = split ? split->p
+               : (double*)ws_get(st == ctx().side ? WS_SPLITK_SIDE : WS_SPLITK, sizeof(double) * (size_t)(S * zs));
+    if (!Pz) return FLA_FAILURE;
+  } else {
+    S = 1;
+    kc = 0;
+  }
+  // Few 64 x 64 tiles: 32 x 32 ones (dgemm_small_kernel) while their CTAs fit
+  // on the GPU at once (three per SM).
+  const bool small = !narrow && tiles * (tile_bm() / 64) * S <= small_tiles();
+  const int BMv = small ? SM_T : bm_, BNv = small ? SM_T : bn_;
+  bool okA = ta ? make_map(&mA, A, k, m, lda, 16, BMv) : make_map(&mA, A, m, k, lda, 16, BK);
+  bool okB = tb ? make_map(&mB, B, n, k, ldb, 16, BK) : make_map(&mB, B, k, n, ldb, 16, BNv);
+  if (!okA || !okB) {
+    set_last_error("gemm_f64: cuTensorMapEncodeTiled failed");
+    return FLA_FAILURE;
+  }
+  dim3 grid((unsigned)((m + BMv - 1) / BMv), (unsigned)((n + BNv - 1) / BNv), (unsigned)S);
+  int* err = ctx().d_status + ST_ERROR;
   double* Cl = S > 1 ? Pz : C;
   const long ldcl = S > 1 ? ldp : ldc;
   const double al = S > 1 ? 1.0 : alpha, be = S > 1 ? 0.0 : beta;
   const int pslot = prof_begin(st);
 #define FB_GEMM_LAUNCH(AK, BK_)                                                                                  \
-  (narrow ? launch<AK, BK_, 128, 32>(grid, st, mA, mB, Cl, ldcl, m, n, k, al, be, mode, diag_off, err, guard,   \
+  (small ? launch_small<AK, BK_>(grid, st, mA, mB, Cl, ldcl, m, n, k, al, be, mode, diag_off, err, guard,         \
+                                 guard_limit, (int)kc, zs)                                                      \
+   : narrow ? launch<AK, BK_, 128, 32>(grid, st, mA, mB, Cl, ldcl, m, n, k, al, be, mode, diag_off, err, guard,   \
                                      guard_limit, (int)kc, zs)                                                  \
    : BMv == 64 ? launch<AK, BK_, 64>(grid, st, mA, mB, Cl, ldcl, m, n, k, al, be, mode, diag_off, err, guard,   \
                                      guard_limit, (int)kc, zs)                                                  \
