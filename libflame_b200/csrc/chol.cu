@@ -28,7 +28,7 @@ namespace {
 
 constexpr int NB = 128;        // outer block
 constexpr int IB = 32;         // inner block
-constexpr int LDS = NB + 1;    // SMEM leading dimension (odd: spreads banks)
+constexpr int LDS = NB + 4;    // SMEM leading dimension (= 4 mod 16: conflict-free DMMA fragments)
 constexpr int POTRF_THREADS = 256;
 constexpr int POTRF_SMEM = NB * LDS * 8;
 // Block columns of at most this many rows below the diagonal block are
@@ -48,67 +48,70 @@ __device__ __forceinline__ bool guard_failed(const int* info) {
 }
 
 // Factor the b x b (b <= 128) lower-triangular diagonal block at A (ld) in
-// place.  gcol = global index of its first column (for the info word).
-// Per 32-column chunk: (a) warp 0 factors the 32 x 32 diagonal block with
-// one row per lane in registers, (b) one thread per row below solves
-// X := X inv(L11)^T with its row in registers, (c) the trailing lower
-// triangle of the block is updated, each thread a register tile of
-// interleaved rows and columns (the shared-memory loads of one warp are
-// broadcasts or consecutive words).  The update of the next chunk's 32
-// columns comes first; warp 0 then factors the next diagonal block while
-// the other seven warps update the columns beyond it.
-// The pivot chain of (a) carries register values only: the next pivot is
-// formed by its own lane from its own multiplier (fma(-l, l, a), the value
-// the shared-memory column broadcast gives) and shuffled; each pivot's
-// reciprocal square root is one rsqrt, its square root d * rsqrt(d).
+// place.  gcol = global index of its first column for the info word.
+// Bound by the pivot chain of one warp: per column a reciprocal square root,
+// two products and a shuffle.  Everything else of a 32-column chunk runs
+// beside that chain:
+//   (a) warp 0 factors the 32 x 32 diagonal block, one row per lane in
+//       registers, and publishes each column in shared memory with a counter;
+//       warps 1-3 solve the rows below (one row per thread in registers,
+//       X := X inv(L11)^T, dtrsm's R,L,T,N order), one column behind warp 0;
+//       warps 4-7 subtract the previous chunk's products from the columns
+//       beyond this chunk;
+//   (b) all warps subtract this chunk's products from the next 32 columns.
+// The products run on the FP64 tensor cores.  The pivot chain carries register
+// values only: the next pivot is formed by its own lane from its own
+// multiplier (fma(-l, l, a)) and shuffled; each pivot's reciprocal square root
+// is one rsqrt, its square root d * rsqrt(d).
+// Measured (128 x 128): 40 us with the solve and the products between the
+// chunks' chains, 27 us in this form.
 __device__ __forceinline__ void cp_async8(double* dst, const double* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
 }
 
-// S[r + c*LDS] -= sum_k S[r + (jb+k)*LDS] S[c + (jb+k)*LDS] (k < w) for the
-// rows r in [r_lo, b) and columns c in [c_lo, c_hi), c <= r: thread (tx, ty)
-// of a TX x TY grid owns rows r_lo + ty + TY a (a < RA) and columns c_lo +
-// tx + TX q (q < CQ).
-template <int TX, int TY, int RA, int CQ>
-__device__ __forceinline__ void syrk_tile(double* S, int jb, int w, int r_lo, int c_lo, int c_hi, int b, int t) {
-  const int tx = t % TX, ty = t / TX;
-  double acc[RA][CQ];
+// S(r, c) -= sum_{k < IB} S(r, jb + k) S(c, jb + k) for 8 x 8 tiles: rows
+// r_lo + 8 i, columns c_lo + 8 j (i < nti, j < ntj), tiles on or below the
+// diagonal only (r_lo, c_lo multiples of 8), dealt to the warps w, w + nw, ...
+// Entries above the diagonal of a diagonal tile are written too: nothing
+// reads them.
+__device__ __forceinline__ void syrk_tiles(double* S, int jb, int r_lo, int nti, int c_lo, int ntj, int w, int nw,
+                                           int lane) {
+  const int g = lane >> 2, t = lane & 3;
+  for (int e = w; e < nti * ntj; e += nw) {
+    const int r = r_lo + 8 * (e % nti), c = c_lo + 8 * (e / nti);
+    if (r < c) continue;
+    const double* pa = S + r + g + (jb + t) * LDS;
+    const double* pb = S + c + g + (jb + t) * LDS;
+    double d0[2] = {0.0, 0.0}, d1[2] = {0.0, 0.0};
 #pragma unroll
-  for (int a = 0; a < RA; ++a)
-#pragma unroll
-    for (int q = 0; q < CQ; ++q) acc[a][q] = 0.0;
-  int ri[RA], ci[CQ];
-#pragma unroll
-  for (int a = 0; a < RA; ++a) ri[a] = min(r_lo + ty + TY * a, b - 1);
-#pragma unroll
-  for (int q = 0; q < CQ; ++q) ci[q] = min(c_lo + tx + TX * q, b - 1);
-  for (int k = 0; k < w; ++k) {
-    const double* col = S + (jb + k) * LDS;
-    double xr[RA], xc[CQ];
-#pragma unroll
-    for (int a = 0; a < RA; ++a) xr[a] = col[ri[a]];
-#pragma unroll
-    for (int q = 0; q < CQ; ++q) xc[q] = col[ci[q]];
-#pragma unroll
-    for (int a = 0; a < RA; ++a)
-#pragma unroll
-      for (int q = 0; q < CQ; ++q) acc[a][q] += xr[a] * xc[q];
-  }
-#pragma unroll
-  for (int a = 0; a < RA; ++a)
-#pragma unroll
-    for (int q = 0; q < CQ; ++q) {
-      const int r = r_lo + ty + TY * a, c = c_lo + tx + TX * q;
-      if (r < b && c < c_hi && c <= r) S[r + c * LDS] -= acc[a][q];
+    for (int k = 0; k < IB; k += 8) {
+      dmma_884(d0[0], d0[1], pa[k * LDS], pb[k * LDS]);
+      dmma_884(d1[0], d1[1], pa[(k + 4) * LDS], pb[(k + 4) * LDS]);
     }
+    double* o = S + r + g + (c + 2 * t) * LDS;
+    o[0] -= d0[0] + d1[0];
+    o[LDS] -= d0[1] + d1[1];
+  }
+}
+
+__device__ __forceinline__ void publish(int* cnt, int v) {
+  asm volatile("st.release.cta.shared.b32 [%0], %1;" ::"r"(smem_u32(cnt)), "r"(v) : "memory");
+}
+__device__ __forceinline__ int published(const int* cnt) {
+  int v;
+  asm volatile("ld.acquire.cta.shared.b32 %0, [%1];" : "=r"(v) : "r"(smem_u32(cnt)) : "memory");
+  return v;
 }
 
 // (a): warp 0 factors the w x w diagonal block at (jb, jb).  Every update is
 // unconditional (no divergent branches in the chain): a lane only ever reads
 // a[c] of its own row for c <= lane, and entries above the diagonal or past
 // w never reach those.  After a failing pivot the rest of the block is not
-// meaningful; the failing column is what is reported.
-__device__ __forceinline__ void potrf_diag32(double* S, int jb, int w, int lane, double* s_rinv, double* s_col,
+// meaningful; the failing column is what is reported.  Column j goes to S
+// (lanes below the diagonal and the pivot), its reciprocal pivot to s_rinv[j],
+// then *cnt := base + j + 1.  Columns are published for all of IB, so the
+// readers' waits always end.
+__device__ __forceinline__ void potrf_diag32(double* S, int jb, int w, int lane, double* s_rinv, int* cnt, int base,
                                              int* s_fail) {
   double a[IB];
 #pragma unroll
@@ -121,78 +124,81 @@ __device__ __forceinline__ void potrf_diag32(double* S, int jb, int w, int lane,
     if (!(d > 0.0) && fail < 0 && j < w) fail = j;  // <= 0 or NaN
     const double rinv = rsqrt(d), sd = d * rinv;
     a[j] = lane == j ? sd : (lane > j ? a[j] * rinv : a[j]);
-    if (lane == 0) s_rinv[j] = rinv;
     const double lj = a[j];
+    double* col = S + jb + (jb + j) * LDS;
+    if (lane >= j) col[lane] = lj;
+    if (lane == 0) s_rinv[j] = rinv;
     if (j + 1 < IB) {
       // lane j + 1's next pivot from its own multiplier, then the broadcast
       const double dn = fma(-lj, lj, a[j + 1]);
       d = __shfl_sync(0xffffffffu, dn, j + 1);
-      double* col = s_col + (j & 1) * IB;  // double-buffered column
-      col[lane] = lj;
-      __syncwarp();
-#pragma unroll
-      for (int c = j + 1; c < IB; ++c) a[c] = fma(-lj, col[c], a[c]);
     }
-  }
+    __syncwarp();
+    if (lane == 0) publish(cnt, base + j + 1);
 #pragma unroll
-  for (int c = 0; c < IB; ++c)
-    if (c <= lane && lane < w) S[(jb + lane) + (jb + c) * LDS] = a[c];
+    for (int c = j + 1; c < IB; ++c) a[c] = fma(-lj, col[c], a[c]);
+  }
   if (lane == 0 && fail >= 0) *s_fail = jb + fail;
 }
 
+// (a): row r below the diagonal block at (jb, jb), in step with warp 0.
+// The wait is for another warp of this CTA, which needs nothing from the
+// waiting one; it is bounded all the same (*err set when it runs out).
+__device__ __forceinline__ void potrf_row(double* S, int jb, int r, const double* s_rinv, const int* cnt, int base,
+                                          int* err) {
+  double x[IB];
+#pragma unroll
+  for (int c = 0; c < IB; ++c) x[c] = S[r + (jb + c) * LDS];
+  int seen = base;
+#pragma unroll
+  for (int j = 0; j < IB; ++j) {
+    for (int spin = 0; seen < base + j + 1; seen = published(cnt))
+      if (++spin > (1 << 20)) {
+        atomicExch(err, 61);
+        return;
+      }
+    x[j] *= s_rinv[j];
+    S[r + (jb + j) * LDS] = x[j];
+#pragma unroll
+    for (int c = j + 1; c < IB; ++c) x[c] = fma(-x[j], S[(jb + c) + (jb + j) * LDS], x[c]);
+  }
+}
+
 __global__ void __launch_bounds__(POTRF_THREADS, 1) potrf_diag_kernel(double* A, long ld, int b, int gcol,
-                                                                   int* info) {
-  extern __shared__ double S[];  // S[r + c*LDS]
-  __shared__ int s_fail;
-  __shared__ double s_rinv[IB];
-  __shared__ double s_col[2 * IB];
+                                                                   int* info, int* err) {
+  extern __shared__ __align__(16) double S[];  // S[r + c*LDS]
+  __shared__ int s_fail, s_cnt;
+  __shared__ double s_rinv[2][IB];
   if (guard_failed(info)) return;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   // load the lower triangle (and diagonal) with asynchronous copies, all in
-  // flight at once; the upper part of S is never read
+  // flight at once; the rest of the square only feeds entries nobody reads
   for (int c = warp; c < b; c += POTRF_THREADS / 32)
     for (int r = c + lane; r < b; r += 32) cp_async8(S + r + c * LDS, A + r + (long)c * ld);
   asm volatile("cp.async.wait_all;" ::: "memory");
-  if (tid == 0) s_fail = -1;
+  if (tid == 0) {
+    s_fail = -1;
+    s_cnt = 0;
+  }
   __syncthreads();
-  if (warp == 0) potrf_diag32(S, 0, min(IB, b), lane, s_rinv, s_col, &s_fail);
-  __syncthreads();
-  for (int jb = 0;;) {
-    if (s_fail >= 0) break;
-    const int w = min(IB, b - jb);
-    const int r0 = jb + w;  // first row below the diagonal block
-    // (b) rows below: X := X inv(L11)^T, one thread per row (right-looking,
-    //     multiply by the reciprocal of the pivot like dtrsm R,L,T,N).
-    //     Columns past w only collect values that are never stored.
-    for (int r = r0 + tid; r < b; r += POTRF_THREADS) {
-      double x[IB];
-#pragma unroll
-      for (int c = 0; c < IB; ++c) x[c] = c < w ? S[r + (jb + c) * LDS] : 0.0;
-#pragma unroll
-      for (int j = 0; j < IB; ++j) {
-        x[j] *= s_rinv[j];
-#pragma unroll
-        for (int c = j + 1; c < IB; ++c) x[c] -= x[j] * S[(jb + c) + (jb + j) * LDS];
-      }
-#pragma unroll
-      for (int c = 0; c < IB; ++c)
-        if (c < w) S[r + (jb + c) * LDS] = x[c];
-    }
-    __syncthreads();
-    if (r0 >= b) break;
-    const int w2 = min(IB, b - r0);
-    // (c) first the next chunk's columns (all rows below r0) ...
-    syrk_tile<32, 8, 12, 1>(S, jb, w, r0, r0, r0 + w2, b, tid);
-    __syncthreads();
-    // ... then warp 0 factors the next diagonal block while the other warps
-    // update the columns beyond it
+  const int b8 = (b + 7) & ~7;
+  for (int jb = 0; jb < b; jb += IB) {
+    const int w = min(IB, b - jb), r0 = jb + w;  // r0: first row below the block
+    // (a); the counter runs on over the chunks (base jb), s_rinv alternates
+    double* rinv = s_rinv[(jb / IB) & 1];
     if (warp == 0) {
-      potrf_diag32(S, r0, w2, lane, s_rinv, s_col, &s_fail);
-    } else if (r0 + w2 < b) {
-      syrk_tile<16, 14, 5, 4>(S, jb, w, r0 + w2, r0 + w2, b, b, tid - 32);
+      potrf_diag32(S, jb, w, lane, rinv, &s_cnt, jb, &s_fail);
+    } else if (warp < 4) {
+      const int r = r0 + (warp - 1) * 32 + lane;
+      if (r < b) potrf_row(S, jb, r, rinv, &s_cnt, jb, err);
+    } else if (jb > 0 && r0 < b) {
+      syrk_tiles(S, jb - IB, r0, (b8 - r0) / 8, r0, (b8 - r0) / 8, warp - 4, 4, lane);
     }
     __syncthreads();
-    jb = r0;
+    if (s_fail >= 0) break;
+    // (b) the next chunk's columns
+    if (r0 < b) syrk_tiles(S, jb, r0, (b8 - r0) / 8, r0, min(IB, b8 - r0) / 8, warp, POTRF_THREADS / 32, lane);
+    __syncthreads();
   }
   // write back the lower triangle (the strictly upper part of A is untouched)
   for (int c = warp; c < b; c += POTRF_THREADS / 32)
@@ -271,7 +277,7 @@ int chol_lower_enqueue(DMat A, cudaStream_t st) {
   auto sub = [&](long k, cudaStream_t s) -> int {
     const int b = (int)std::min<long>(NB, n - k);
     int ps = prof_begin(s);
-    potrf_diag_kernel<<<1, POTRF_THREADS, POTRF_SMEM, s>>>(at(k, k), ld, b, (int)k, info);
+    potrf_diag_kernel<<<1, POTRF_THREADS, POTRF_SMEM, s>>>(at(k, k), ld, b, (int)k, info, cx.d_status + ST_ERROR);
     prof_end(ps, s, PROF_DIAG, (double)b * b * b / 3.0);
     count_launch();
     FB_CK(cudaGetLastError());
@@ -338,7 +344,8 @@ int chol_lower_enqueue(DMat A, cudaStream_t st) {
 int potrf_diag_dev(double* A, long ld, int b, int gcol, cudaStream_t st) {
   set_attrs();
   int ps = prof_begin(st);
-  potrf_diag_kernel<<<1, POTRF_THREADS, POTRF_SMEM, st>>>(A, ld, b, gcol, ctx().d_status + ST_INFO);
+  potrf_diag_kernel<<<1, POTRF_THREADS, POTRF_SMEM, st>>>(A, ld, b, gcol, ctx().d_status + ST_INFO,
+                                                            ctx().d_status + ST_ERROR);
   prof_end(ps, st, PROF_DIAG, (double)b * b * b / 3.0);
   count_launch();
   FB_CK(cudaGetLastError());
