@@ -27,6 +27,7 @@ struct Context {
   int* d_status = nullptr;           // device status words (see Status below)
   int* h_status = nullptr;           // pinned mirror
   unsigned long long launches = 0;   // kernels launched by this library
+  bool solve_pending = false;        // a solve's error word (ST_SOLVE) is still to be read
 };
 
 Context& ctx();
@@ -35,8 +36,10 @@ Context& ctx();
 //   [ST_ERROR] nonzero when a kernel's bounded wait expired (code of the wait)
 //   [ST_INFO]  numerical info: zero-based index of the first failing column,
 //              INT_MAX when none; kernels atomicMin into it
+//   [ST_SOLVE] nonzero when a wait of a one-launch triangular solve expired;
+//              read by sync_all() (a solve has no status_read() of its own)
 //   [ST_BAR..] counters of the grid barriers of cooperative kernels
-enum : int { ST_ERROR = 0, ST_INFO = 1, ST_BAR = 2, ST_WORDS = 64 };
+enum : int { ST_ERROR = 0, ST_INFO = 1, ST_BAR = 2, ST_SOLVE = 63, ST_WORDS = 64 };
 
 // Record one kernel launch issued by this library (for the launch count
 // reported by FLA_B200_kernel_launches()).
@@ -231,6 +234,7 @@ int laswp_dev(double* A, long ld, int row0, const int* d_piv, int npiv, int c0, 
 int trsm_left_dev(DMat T, DMat B, bool lower, bool trans, bool unit, cudaStream_t st);
 int trsm_block(const double* T, long ldt, double* B, long ldb, int b, long n, bool lower,
                bool trans, bool unit, cudaStream_t st);
+int trsm_sweep(DMat T, DMat B, bool lower, bool trans, bool unit, cudaStream_t st);
 // X := inv(L), L b x b lower triangular (unit diagonal if unit), X ld ldx.
 int tri_inverse_lower(const double* L, long ldl, int b, bool unit, double* X, long ldx, cudaStream_t st);
 // Inverses of the 128 x 128 diagonal blocks of an n x n triangle, one

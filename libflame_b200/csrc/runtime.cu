@@ -177,9 +177,20 @@ void prof_end(int slot, cudaStream_t st, int cls, double flops) {
 }
 
 int sync_all() {
-  FB_CK(cudaStreamSynchronize(ctx().side));
-  FB_CK(cudaStreamSynchronize(ctx().stream));
+  Context& c = ctx();
+  const bool solve = c.solve_pending;
+  if (solve) {
+    c.solve_pending = false;
+    FB_CK(cudaMemcpyAsync(c.h_status + ST_SOLVE, c.d_status + ST_SOLVE, sizeof(int), cudaMemcpyDeviceToHost, c.stream));
+  }
+  FB_CK(cudaStreamSynchronize(c.side));
+  FB_CK(cudaStreamSynchronize(c.stream));
   prof_collect();
+  if (solve && c.h_status[ST_SOLVE] != 0) {
+    FB_CK(cudaMemset(c.d_status + ST_SOLVE, 0, sizeof(int)));
+    set_last_error("a wait of the triangular solve exceeded its limit");
+    return FLA_FAILURE;
+  }
   return FLA_SUCCESS;
 }
 
