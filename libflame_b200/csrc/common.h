@@ -207,6 +207,10 @@ int gemm_f64(cudaStream_t st, bool ta, bool tb, long m, long n, long k, double a
 // kmax > 0 (full mode only): split k so that no CTA runs more than about
 // kmax of it, for GEMMs whose long-running tiles would keep SMs from a
 // cluster kernel waiting on the other stream.
+// Partial products of A^T B for m, n <= 64 (A k x m, B k x n, any alignment):
+// *S contiguous m x n blocks at *P, in the stream's split-K workspace.
+int gemm_tn_partials(cudaStream_t st, long m, long n, long k, const double* A, long lda, const double* B, long ldb,
+                     double** P, long* S);
 // The guard pointer is the status block's info word (INT_MAX, or the first
 // failing column): the kernel returns at once when it holds a column below
 // guard_limit, i.e. when a factorization step this update follows has failed.

@@ -587,55 +587,92 @@ __global__ void splitk_reduce_kernel(const double* __restrict__ P, long ldp, lon
   }
 }
 
-// Partial products of C = A^T B for small outputs (m, n <= 64) with a long
-// k (the W = U1^T B and T12 = U1^T U2 products of the QR panel recursion):
-// CTA z multiplies rows [z kc, (z+1) kc) of A (k x m) and B (k x n) with
-// FP64 FMAs, 32 rows at a time through shared memory, each of the 256
-// threads owning a TB x TB block of the output (16 TB >= m, n), and writes
-// its m x n partial to P + z m n; splitk_reduce_warp_kernel adds the
-// partials.  A 128 x 64 DMMA tile would spend most of its work on padding
-// for these shapes.
-constexpr int SK_ROWS = 32;
-template <int TB>
+// Partial products of C = A^T B for small outputs (m, n <= D, D = 16, 32 or
+// 64) with a long k (the W = U1^T B and T12 = U1^T U2 products of the QR
+// panel recursion): CTA z multiplies rows [z KC, (z+1) KC) of A (k x m) and B
+// (k x n) and writes its m x n partial to P + z m n; the partials are added
+// by splitk_reduce_warp_kernel or by the kernel that uses them.  Latency
+// bound (the whole product is a few MFLOP and each CTA one slab), so the slab
+// is brought in by one batch of asynchronous copies and the warps split its
+// rows as well as the output: warp (strip, group) forms 16 rows of the output
+// from every NG-th group of four slab rows, and the groups are added through
+// shared memory in order.  A slab of 128 rows (64 for D = 64) keeps about one
+// CTA per SM at 12288 rows.  Measured at k = 12288: 16 x 16 16.6 -> 3.7 us,
+// 64 x 64 21.4 -> 9.5 us against 32-row passes of FP64 FMAs, each pass
+// exposing its loads.
+template <int D>
+struct TnSmall {
+  static constexpr int KC = D == 64 ? 64 : 128;
+  static constexpr int LD = KC + 4;      // = 4 mod 16: conflict-free fragments
+  static constexpr int STRIPS = D / 16;  // 16-row strips of the output
+  static constexpr int NG = 8 / STRIPS;  // row groups
+  static constexpr size_t STAGE = (size_t)2 * D * LD, RED = (size_t)NG * D * (D + 1);
+  static constexpr size_t SMEM = sizeof(double) * (STAGE > RED ? STAGE : RED);
+};
+template <int D>
 __global__ void __launch_bounds__(256) gemm_tn_small_kernel(const double* __restrict__ A, long lda,
                                                             const double* __restrict__ B, long ldb, int m, int n,
-                                                            long k, long kc, double* __restrict__ P) {
-  constexpr int D = 16 * TB;  // output block covered by the CTA
-  __shared__ double As[SK_ROWS][D + 1], Bs[SK_ROWS][D + 1];
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-  const long k0 = blockIdx.x * kc, k1 = min(k, k0 + kc);
-  double acc[TB][TB] = {};
-  for (long kb = k0; kb < k1; kb += SK_ROWS) {
-    const int rows = (int)(k1 - kb < SK_ROWS ? k1 - kb : SK_ROWS);
-    for (int e = tid; e < SK_ROWS * D; e += 256) {
-      const int r = e % SK_ROWS, c = e / SK_ROWS;
-      As[r][c] = (r < rows && c < m) ? A[(kb + r) + (long)c * lda] : 0.0;
-      Bs[r][c] = (r < rows && c < n) ? B[(kb + r) + (long)c * ldb] : 0.0;
-    }
-    __syncthreads();
+                                                            long k, double* __restrict__ P) {
+  using T = TnSmall<D>;
+  constexpr int KC = T::KC, LD = T::LD, NG = T::NG;
+  extern __shared__ __align__(16) double tn_sm[];
+  double *sA = tn_sm, *sB = tn_sm + D * LD;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  auto load = [&](const double* X, long ldx, int cols, double* S, long k0, int rows) {
 #pragma unroll 8
-    for (int r = 0; r < SK_ROWS; ++r) {
-      double av[TB], bv[TB];
+    for (int e = tid; e < KC * D; e += 256) {
+      const int r = e % KC, c = e / KC;
+      if (r < rows && c < cols)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(S + r + c * LD)),
+                     "l"(X + (k0 + r) + (long)c * ldx)
+                     : "memory");
+      else
+        S[r + c * LD] = 0.0;
+    }
+  };
+  const int strip = warp / NG, grp = warp % NG, g = lane >> 2, t = lane & 3;
+  double acc[2][D / 8][2];
 #pragma unroll
-      for (int t = 0; t < TB; ++t) {
-        av[t] = As[r][tx + 16 * t];
-        bv[t] = Bs[r][ty + 16 * t];
+  for (int h = 0; h < 2; ++h)
+#pragma unroll
+    for (int c = 0; c < D / 8; ++c) acc[h][c][0] = acc[h][c][1] = 0.0;
+  const double* pa = sA + (strip * 16 + g) * LD + t;
+  const double* pb = sB + g * LD + t;
+  for (long k0 = (long)blockIdx.x * KC; k0 < k; k0 += (long)gridDim.x * KC) {
+    const int rows = (int)(k - k0 < KC ? k - k0 : KC);
+    load(A, lda, m, sA, k0, rows);
+    load(B, ldb, n, sB, k0, rows);
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+#pragma unroll 2
+    for (int kk = 4 * grp; kk < KC; kk += 4 * NG) {
+      const double a0 = pa[kk], a1 = pa[kk + 8 * LD];
+#pragma unroll
+      for (int c = 0; c < D / 8; ++c) {
+        const double b = pb[kk + 8 * c * LD];
+        dmma_884(acc[0][c][0], acc[0][c][1], a0, b);
+        dmma_884(acc[1][c][0], acc[1][c][1], a1, b);
       }
-#pragma unroll
-      for (int t = 0; t < TB; ++t)
-#pragma unroll
-        for (int u = 0; u < TB; ++u) acc[t][u] = fma(av[t], bv[u], acc[t][u]);
     }
     __syncthreads();
   }
+  // group sums: entry (i, j) of group grp at tn_sm[(grp D + j) (D + 1) + i]
+#pragma unroll
+  for (int h = 0; h < 2; ++h)
+#pragma unroll
+    for (int c = 0; c < D / 8; ++c)
+#pragma unroll
+      for (int e = 0; e < 2; ++e)
+        tn_sm[(grp * D + 8 * c + 2 * t + e) * (D + 1) + strip * 16 + 8 * h + g] = acc[h][c][e];
+  __syncthreads();
   double* Pz = P + (long)blockIdx.x * m * n;
+  for (int e = tid; e < m * n; e += 256) {
+    const int i = e % m, j = e / m;
+    double s = tn_sm[j * (D + 1) + i];
 #pragma unroll
-  for (int t = 0; t < TB; ++t)
-#pragma unroll
-    for (int u = 0; u < TB; ++u) {
-      const int i = tx + 16 * t, j = ty + 16 * u;
-      if (i < m && j < n) Pz[i + (long)j * m] = acc[t][u];
-    }
+    for (int q = 1; q < NG; ++q) s += tn_sm[(q * D + j) * (D + 1) + i];
+    Pz[e] = s;
+  }
 }
 
 // C := alpha sum_z P_z + beta C for S partials of m x n (contiguous, m x n
@@ -681,6 +718,36 @@ long small_tiles() {
 
 }  // namespace
 
+// Partial products of A^T B (A k x m, B k x n, m, n <= 64) in the stream's
+// split-K workspace: *S of them, m x n each, one after another at *P.
+int gemm_tn_partials(cudaStream_t st, long m, long n, long k, const double* A, long lda, const double* B, long ldb,
+                     double** P, long* S) {
+  const int D = m <= 16 && n <= 16 ? 16 : m <= 32 && n <= 32 ? 32 : 64;
+  const long kc = D == 64 ? TnSmall<64>::KC : TnSmall<16>::KC;
+  *S = std::min<long>(2L * ctx().num_sms, (k + kc - 1) / kc);
+  *P = (double*)ws_get(st == ctx().side ? WS_SPLITK_SIDE : WS_SPLITK, sizeof(double) * (size_t)(*S * m * n));
+  if (!*P) return FLA_FAILURE;
+  static bool attr = false;
+  if (!attr) {
+    FB_CK(cudaFuncSetAttribute(gemm_tn_small_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)TnSmall<32>::SMEM));
+    FB_CK(cudaFuncSetAttribute(gemm_tn_small_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)TnSmall<64>::SMEM));
+    attr = true;
+  }
+  const int ps = prof_begin(st);
+  if (D == 16)
+    gemm_tn_small_kernel<16><<<(unsigned)*S, 256, TnSmall<16>::SMEM, st>>>(A, lda, B, ldb, (int)m, (int)n, k, *P);
+  else if (D == 32)
+    gemm_tn_small_kernel<32><<<(unsigned)*S, 256, TnSmall<32>::SMEM, st>>>(A, lda, B, ldb, (int)m, (int)n, k, *P);
+  else
+    gemm_tn_small_kernel<64><<<(unsigned)*S, 256, TnSmall<64>::SMEM, st>>>(A, lda, B, ldb, (int)m, (int)n, k, *P);
+  prof_end(ps, st, PROF_GEMM, 2.0 * (double)m * (double)n * (double)k);
+  count_launch();
+  FB_CK(cudaGetLastError());
+  return FLA_SUCCESS;
+}
+
 int gemm_f64(cudaStream_t st, bool ta, bool tb, long m, long n, long k, double alpha,
              const double* A, long lda, const double* B, long ldb, double beta, double* C,
              long ldc, GemmMode mode, long diag_off, const int* guard, int guard_limit, long kmax,
@@ -692,23 +759,12 @@ int gemm_f64(cudaStream_t st, bool ta, bool tb, long m, long n, long k, double a
     if (beta == 1.0) return FLA_SUCCESS;
   }
   if (ta && !tb && mode == GEMM_FULL && !guard && m <= 64 && n <= 64 && k >= 1024) {
-    // slices of 128 rows, at most two per SM
-    const int sms = ctx().num_sms;
-    long S = std::max<long>(1, std::min<long>(2L * sms, k / 128));
-    const long kc = ((k + S - 1) / S + SK_ROWS - 1) / SK_ROWS * SK_ROWS;
-    S = (k + kc - 1) / kc;
-    double* Pz = (double*)ws_get(st == ctx().side ? WS_SPLITK_SIDE : WS_SPLITK, sizeof(double) * (size_t)(S * m * n));
-    if (!Pz) return FLA_FAILURE;
-    const int ps = prof_begin(st);
-    if (m <= 32 && n <= 32)
-      gemm_tn_small_kernel<2><<<(unsigned)S, 256, 0, st>>>(A, lda, B, ldb, (int)m, (int)n, k, kc, Pz);
-    else
-      gemm_tn_small_kernel<4><<<(unsigned)S, 256, 0, st>>>(A, lda, B, ldb, (int)m, (int)n, k, kc, Pz);
-    count_launch();
+    double* Pz = nullptr;
+    long S = 0;
+    if (gemm_tn_partials(st, m, n, k, A, lda, B, ldb, &Pz, &S) != FLA_SUCCESS) return FLA_FAILURE;
     splitk_reduce_warp_kernel<<<(unsigned)((m * n * 32 + 255) / 256), 256, 0, st>>>(Pz, (int)S, (int)m, (int)n,
                                                                                    alpha, beta, C, ldc);
     count_launch();
-    prof_end(ps, st, PROF_GEMM, 2.0 * (double)m * (double)n * (double)k);
     FB_CK(cudaGetLastError());
     return FLA_SUCCESS;
   }

@@ -25,15 +25,17 @@
 //   2. one CTA barrier; the CTA's partial vector is the fixed-order sum of
 //      the 16 warp slots (its entry q = j is ||x2||^2);
 //   3. (clusters only) warp 0 bulk-copies the CTA's partial vector, and
-//      CTA 0 row j, into every other CTA's shared memory, waits for the
-//      column's bytes on its mbarrier, and a second CTA barrier releases
-//      the CTA; every lane sums the C partial vectors in CTA order, so every
-//      CTA holds the same bits;
+//      CTA 0 row j, into every other CTA's shared memory; every warp waits
+//      for the column's bytes on the CTA's mbarrier; every lane sums the C
+//      partial vectors in the same order, so every CTA holds the same bits;
 //   4. every lane forms alpha, tau and the scale 1 / (chi1 - alpha); since
 //      u2 = x2 * scale, u2^T a_q = scale * (x^T a_q), so one exchange per
 //      column gives both ||x2|| and the update row w; the column-j lanes
-//      scale their column into u2 and broadcast u (with u_j = 1), and the
-//      lanes q > j apply a_q -= u w_q.  CTA 0 writes column j of T.
+//      scale their column into u2, and the lanes q > j apply
+//      a_q -= x (scale w_q) (row j: a_q -= w_q).  CTA 0 writes column j of T.
+// Bound by the latency of that chain: an 8192 x 32 leaf 151 us with two CTA
+// barriers per column, serial sums and two square roots and two divisions in
+// a row, 120 us in this form (a 12288 x 16 one 86 -> 68 us).
 // One exchange per column where the reference's order needs two reductions
 // (the norm, then the dot products): the sums are the same up to the
 // rounding of scaling before or after the summation.
@@ -133,55 +135,70 @@ __global__ void __launch_bounds__(QL_THREADS, 1) qr_leaf_kernel(QrLeafArgs a) {
 
   const int gfirst = r0 + wrow0 + g * 32;  // global row of v[0]
   const int ncols = min(a.w, a.M);
+  bool dead = false;                   // a wait of this warp ran out
+  const bool idle = wrow0 >= rows;     // this warp holds no rows: zero partial sums, no update
+  if (idle && g == 0) wpart[warp * W + q] = wpart[(QL_NW + warp) * W + q] = 0.0;
 #pragma unroll 1
   for (int j = 0; j < ncols; ++j) {
     const int par = j & 1;
     // ---- 1. broadcast column j; row j; partial dot products
     const bool low = r0 + wrow0 <= j;  // this warp holds rows <= j (CTA 0, warp 0)
-    if (q == j) {
-      if (low) {
+    if (!idle) {
+      if (q == j) {
+        if (low) {
 #pragma unroll
-        for (int i = 0; i < 32; i += 2)
-          *reinterpret_cast<double2*>(xs + g * 32 + i) =
-              make_double2(gfirst + i > j ? v[i] : 0.0, gfirst + i + 1 > j ? v[i + 1] : 0.0);
-      } else {
+          for (int i = 0; i < 32; i += 2)
+            *reinterpret_cast<double2*>(xs + g * 32 + i) =
+                make_double2(gfirst + i > j ? v[i] : 0.0, gfirst + i + 1 > j ? v[i + 1] : 0.0);
+        } else {
 #pragma unroll
-        for (int i = 0; i < 32; i += 2) *reinterpret_cast<double2*>(xs + g * 32 + i) = make_double2(v[i], v[i + 1]);
+          for (int i = 0; i < 32; i += 2) *reinterpret_cast<double2*>(xs + g * 32 + i) = make_double2(v[i], v[i + 1]);
+        }
       }
-    }
-    if (low && j >= gfirst && j < gfirst + 32) {
-      // row j lives in this lane group: publish it
-      const int ij = j - gfirst;
-      double r = v[0];
+      if (low && j >= gfirst && j < gfirst + 32) {
+        // row j lives in this lane group: publish it
+        const int ij = j - gfirst;
+        double r = v[0];
 #pragma unroll
-      for (int i = 1; i < 32; ++i)
-        if (i == ij) r = v[i];
-      rowj[par * W + q] = r;
-      if (C > 1) fence_proxy_async_smem();
-    }
-    __syncwarp();
-    double d = 0.0;
+        for (int i = 1; i < 32; ++i)
+          if (i == ij) r = v[i];
+        rowj[par * W + q] = r;
+        if (C > 1) fence_proxy_async_smem();
+      }
+      __syncwarp();
+      double d0 = 0.0, d1 = 0.0, d2 = 0.0, d3 = 0.0;  // four chains: FP64 FMA latency
 #pragma unroll
-    for (int i = 0; i < 32; i += 2) {
-      const double2 x = *reinterpret_cast<const double2*>(xs + g * 32 + i);
-      d = fma(x.x, v[i], d);
-      d = fma(x.y, v[i + 1], d);
-    }
+      for (int i = 0; i < 32; i += 4) {
+        const double2 x = *reinterpret_cast<const double2*>(xs + g * 32 + i);
+        const double2 y = *reinterpret_cast<const double2*>(xs + g * 32 + i + 2);
+        d0 = fma(x.x, v[i], d0);
+        d1 = fma(x.y, v[i + 1], d1);
+        d2 = fma(y.x, v[i + 2], d2);
+        d3 = fma(y.y, v[i + 3], d3);
+      }
+      double d = (d0 + d1) + (d2 + d3);
 #pragma unroll
-    for (int off = W; off < 32; off <<= 1) d += __shfl_xor_sync(0xffffffffu, d, off);
-    if (g == 0) wpart[(par * QL_NW + warp) * W + q] = d;
+      for (int off = W; off < 32; off <<= 1) d += __shfl_xor_sync(0xffffffffu, d, off);
+      if (g == 0) wpart[(par * QL_NW + warp) * W + q] = d;
+    }
     __syncthreads();
-    // ---- 2. the CTA's partial vector (fixed warp order)
+    // ---- 2. the CTA's partial vector (fixed warp order); in a cluster only
+    // warp 0 needs it (sixteen warps reading sixteen slots each would keep the
+    // shared memory busy for a quarter of the column)
+    const bool active_sum = C == 1 || warp == 0;
     double cs = 0.0;
+    if (active_sum) {
+      double s4[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll
-    for (int ww = 0; ww < QL_NW; ++ww) cs += wpart[(par * QL_NW + ww) * W + q];
+      for (int ww = 0; ww < QL_NW; ++ww) s4[ww & 3] += wpart[(par * QL_NW + ww) * W + q];
+      cs = (s4[0] + s4[1]) + (s4[2] + s4[3]);
+    }
     // ---- 3. the cluster's sum
     double dq = cs;
     if (C > 1) {
       const uint32_t fullp = full0 + 8 * par;
       const uint32_t ph = (uint32_t)((j >> 1) & 1);
       double* own = cslot + ((size_t)par * C + c) * W;
-      bool ok = true;
       if (warp == 0) {
         if (g == 0) own[q] = cs;
         fence_proxy_async_smem();
@@ -193,37 +210,45 @@ __global__ void __launch_bounds__(QL_THREADS, 1) qr_leaf_kernel(QrLeafArgs a) {
             bulk_copy_to_peer(mapa_shared(smem_u32(rowj + par * W), (uint32_t)lane), smem_u32(rowj + par * W),
                               (uint32_t)(8 * W), rbar);
         }
+        // the arrive also publishes this CTA's own slot to its other warps
         if (lane == 0) mbar_arrive_expect_tx(fullp, (uint32_t)((C - 1) * 8 * W + (c == 0 ? 0 : 8 * W)));
-        ok = mbar_wait_cluster(fullp, ph, a.err, 33);
       }
-      // the CTA leaves the loop together if the (bounded) wait ran out
-      if (__syncthreads_or(ok ? 0 : 1)) break;
-      if (warp != 0) (void)mbar_try_wait_cluster(fullp, ph);  // acquire of the completed phase
-      dq = 0.0;
+      // every warp waits for the column's bytes itself (no second CTA
+      // barrier); after a wait that ran out (bounded, reported) the later
+      // ones are skipped, so the barrier counts stay the same everywhere
+      if (!dead && !mbar_wait_cluster(fullp, ph, a.err, 33)) dead = true;
+      double c4[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll
       for (int cc = 0; cc < QL_MAXC; ++cc)
-        if (cc < C) dq += (cc == c) ? cs : cslot[((size_t)par * C + cc) * W + q];
+        if (cc < C) c4[cc & 3] += cslot[((size_t)par * C + cc) * W + q];
+      dq = (c4[0] + c4[1]) + (c4[2] + c4[3]);
     }
+    if (idle) continue;  // nothing to update
     // ---- 4. Householder vector, w, T column; the update
     const double ss = __shfl_sync(0xffffffffu, dq, j);  // ||x2||^2 (lane j of group 0)
     const double chi1 = rowj[par * W + j];
-    const double nx2 = sqrt(ss);
-    double scale, alpha, tau;
-    const bool trivial = nx2 == 0.0;
-    if (trivial) {
-      scale = 1.0;
-      alpha = -chi1;
-      tau = 0.5;
-    } else {
-      const double nx = sqrt(fma(chi1, chi1, ss));  // ||[chi1; x2]||
-      alpha = -((chi1 < 0.0) ? -1.0 : 1.0) * nx;
-      const double cma = chi1 - alpha;
-      scale = 1.0 / cma;
-      const double qq = nx2 * fabs(scale);  // ||x2|| / |chi1 - alpha|
-      tau = 0.5 + 0.5 * (qq * qq);
+    // With t = chi1^2 + ss, r = 1 / sqrt(t), sg = sign(chi1):
+    //   alpha = -sg sqrt(t),  scale = 1 / (chi1 - alpha) = sg / (|chi1| + sqrt(t)),
+    //   tau = 1/2 + 1/2 ss scale^2 = sqrt(t) |scale|,  1 / tau = 1 + |chi1| r,
+    //   w_q = (a1(q) + scale x^T a_q) / tau = a1(q) / tau + sg r x^T a_q
+    // (scale / tau = sg r): the update row waits for one reciprocal square
+    // root only; the division by |chi1| + sqrt(t) runs beside it.
+    const bool trivial = ss == 0.0;
+    double scale = 1.0, alpha = -chi1, tau = 0.5, rtau = 2.0, rs = 2.0;
+    if (!trivial) {
+      const double t = fma(chi1, chi1, ss), r = rsqrt(t), ac = fabs(chi1);
+      double nx = t * r;
+      nx = fma(0.5 * r, fma(-nx, nx, t), nx);  // sqrt(t), rounded like sqrt()
+      scale = copysign(1.0 / (ac + nx), chi1 < 0.0 ? -1.0 : 1.0);
+      alpha = chi1 < 0.0 ? nx : -nx;
+      tau = nx * fabs(scale);
+      rtau = fma(ac, r, 1.0);
+      rs = chi1 < 0.0 ? -r : r;
     }
-    const double rtau = 1.0 / tau;
-    const double tq = rowj[par * W + q] + scale * dq;  // a1(q) + u2^T a2(q)
+    const double a1q = rowj[par * W + q];
+    const double tq = fma(scale, dq, a1q);  // a1(q) + u2^T a2(q)
+    const double wq = fma(rs, dq, a1q * rtau);
+    const double sw = scale * wq;
     if (c == 0 && warp == 0 && g == 0 && q < a.w) {
       if (q < j) a.T[q + (long)j * a.ldt] = tq;
       else if (q == j) a.T[j + (long)j * a.ldt] = tau;
@@ -244,12 +269,11 @@ __global__ void __launch_bounds__(QL_THREADS, 1) qr_leaf_kernel(QrLeafArgs a) {
         for (int i = 0; i < 32; ++i) v[i] *= scale;
       }
     } else if (q > j) {
-      const double wq = tq * rtau;
 #pragma unroll
       for (int i = 0; i < 32; i += 2) {
         const double2 x = *reinterpret_cast<const double2*>(xs + g * 32 + i);
-        v[i] = fma(-(trivial ? x.x : x.x * scale), wq, v[i]);
-        v[i + 1] = fma(-(trivial ? x.y : x.y * scale), wq, v[i + 1]);
+        v[i] = fma(-x.x, sw, v[i]);
+        v[i + 1] = fma(-x.y, sw, v[i + 1]);
       }
       if (low && j >= gfirst && j < gfirst + 32) {
         const int ij = j - gfirst;
@@ -337,6 +361,8 @@ int qleaf_width(long M, int w) {
 
 int qleaf_launch(double* P, long ld, long M, int w, int W, double* T, long ldt, double* U, long ldu,
                  cudaStream_t st) {
+  // as few CTAs as hold the rows: a column's exchange costs more with each
+  // (M = 12288, W = 16: FLA_QR_UT 12288 x 6144 2 ms faster with 12 than 16)
   const long per = (long)QL_THREADS * (32 / W);
   const int C = (int)((M + per - 1) / per);
   QrLeafArgs la;
@@ -381,6 +407,66 @@ __global__ void qr_unit_lower_kernel(const double* __restrict__ P, long ldp, dou
   U[row + (long)col * ldu] = row > col ? P[row + (long)col * ldp] : (row == col ? 1.0 : 0.0);
 }
 
+// W := T^-T (sum_z P_z) for the joins of the panel recursion: S partial
+// products P_z (w1 x w2, contiguous, one after another) added in z order, then
+// forward substitution with the transposed upper triangle T (w1 <= 64).  One
+// CTA per four columns, one warp per column in the substitution (lane l:
+// rows l and l + 32, the solved entry broadcast); several threads share an
+// element's partials when there are threads to spare.  Latency bound; it takes
+// the place of a reduction, a 128-row triangular solve or an inverse with its
+// product (9 to 20 us) and takes about 10 us.
+constexpr int RS_THREADS = 512, RS_COLS = 4;
+__global__ void __launch_bounds__(RS_THREADS) qr_reduce_solve_kernel(const double* __restrict__ P, int S, int w1,
+                                                                     int w2, const double* __restrict__ T, long ldt,
+                                                                     double* __restrict__ W, long ldw) {
+  __shared__ double sT[64 * 65];            // sT[j + i * 65] = T(j, i), j <= i
+  __shared__ double sW[RS_THREADS];
+  __shared__ double sr[64];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int c0 = blockIdx.x * RS_COLS, nc = min(RS_COLS, w2 - c0);
+  for (int e = tid; e < w1 * w1; e += RS_THREADS) {
+    const int j = e % w1, i = e / w1;
+    const double v = j <= i ? T[j + (long)i * ldt] : 0.0;
+    sT[j + i * 65] = v;
+    if (i == j) sr[j] = 1.0 / v;
+  }
+  const int ne = w1 * nc;                   // <= 512 elements, contiguous in each partial
+  const int tpe = max(1, RS_THREADS / (w1 * RS_COLS));  // threads per element
+  const int e = tid / tpe, h = tid % tpe;
+  double s = 0.0;
+  if (e < ne) {
+    const double* p = P + (long)c0 * w1 + e;
+    const long step = (long)w1 * w2;
+#pragma unroll 8
+    for (int z = h; z < S; z += tpe) s += p[(long)z * step];
+  }
+  sW[tid] = s;
+  __syncthreads();
+  if (warp < nc) {
+    double r[2] = {0.0, 0.0};
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int i = lane + 32 * u;
+      if (i < w1)
+        for (int q = 0; q < tpe; ++q) r[u] += sW[(warp * w1 + i) * tpe + q];
+    }
+    for (int j = 0; j < w1; ++j) {
+      const double x = __shfl_sync(0xffffffffu, j < 32 ? r[0] : r[1], j & 31) * sr[j];
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int i = lane + 32 * u;
+        if (i == j) r[u] = x;
+        else if (i > j && i < w1) r[u] = fma(-sT[j + i * 65], x, r[u]);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int i = lane + 32 * u;
+      if (i < w1) W[i + (long)(c0 + warp) * ldw] = r[u];
+    }
+  }
+}
+
 // Factor the M x w piece P (ld) in place; Tb (ld ldtb) receives its w x w
 // T and U (ld ldu, aligned with P: U[i + q ldu] is element (i, q) of the
 // piece) its unit lower trapezoid, rows 0 .. M - 1.  Wk (w x w, ld ldw) is
@@ -399,19 +485,34 @@ int panel_rec(double* P, long ld, long M, int w, double* Tb, long ldtb, double* 
   const int w2 = w - w1;
   if (panel_rec(P, ld, M, w1, Tb, ldtb, U, ldu, Wk, ldw, st) != FLA_SUCCESS) return FLA_FAILURE;
   // B := (I - U1 T11^-T U1^T) B on the right half: W := U1^T B,
-  // W := T11^-T W (through T11^-1 for the wider halves), B -= U1 W
+  // W := T11^-T W, B -= U1 W
   double* B = P + (long)w1 * ld;
   double* W1 = Wk;
-  if (gemm_f64(st, true, false, w1, w2, M, 1.0, U, ldu, B, ld, 0.0, W1, ldw) != FLA_SUCCESS) return FLA_FAILURE;
-  if (w1 >= 32) {
+  if (w1 <= 64 && w2 <= 64) {
+    // the reduction of a long product goes with the solve while it has few
+    // elements per CTA; a 64-wide one is reduced by the whole GPU first
+    double* Pz = W1;
+    long S = 1;
+    if (w1 <= 32 && w2 <= 32 && M >= 1024) {
+      if (gemm_tn_partials(st, w1, w2, M, U, ldu, B, ld, &Pz, &S) != FLA_SUCCESS) return FLA_FAILURE;
+    } else {
+      Pz = Wk + (long)ldw * w2;  // w1 x w2, contiguous for the solve
+      if (gemm_f64(st, true, false, w1, w2, M, 1.0, U, ldu, B, ld, 0.0, Pz, w1) != FLA_SUCCESS) return FLA_FAILURE;
+    }
+    const int ps = prof_begin(st);
+    qr_reduce_solve_kernel<<<(unsigned)((w2 + RS_COLS - 1) / RS_COLS), RS_THREADS, 0, st>>>(
+        Pz, (int)S, w1, w2, Tb, ldtb, W1, ldw);
+    prof_end(ps, st, PROF_TRSM, (double)w1 * w1 * w2);
+    count_launch();
+    FB_CK(cudaGetLastError());
+  } else {
     double* Ti = Wk + (long)ldw * w2;          // w1 x w1
     double* W2 = Ti + (long)ldw * w1;          // w1 x w2
+    if (gemm_f64(st, true, false, w1, w2, M, 1.0, U, ldu, B, ld, 0.0, W1, ldw) != FLA_SUCCESS) return FLA_FAILURE;
     if (tri_inverse(Tb, ldtb, w1, false, false, Ti, ldw, st) != FLA_SUCCESS) return FLA_FAILURE;
     if (gemm_f64(st, true, false, w1, w2, w1, 1.0, Ti, ldw, W1, ldw, 0.0, W2, ldw) != FLA_SUCCESS)
       return FLA_FAILURE;
     W1 = W2;
-  } else if (trsm_block(Tb, ldtb, W1, ldw, w1, w2, false, true, false, st) != FLA_SUCCESS) {
-    return FLA_FAILURE;
   }
   if (gemm_f64(st, false, false, M, w2, w1, -1.0, U, ldu, W1, ldw, 1.0, B, ld) != FLA_SUCCESS) return FLA_FAILURE;
   if (M <= w1) return FLA_SUCCESS;
