@@ -195,6 +195,9 @@ int status_read(int* info);
 struct GemmSplit {
   double* p = nullptr;
   size_t elems = 0;
+  long max_slices = 0;     // 0: no limit of its own
+  long* slices = nullptr;  // if set: the slices (m x n, ld m rounded up to even, one after another) stay at p
+                           // for the caller to add, *slices of them; C is not used
 };
 enum GemmMode : int { GEMM_FULL = 0, GEMM_LOWER = 1 };
 int gemm_f64(cudaStream_t st, bool ta, bool tb, long m, long n, long k, double alpha,
@@ -230,6 +233,10 @@ inline bool tma_ok(const void* p, long ld) {
 int chol_lower_dev(DMat A, int* info);
 int chol_upper_dev(DMat A, int* info);
 int chol_lower_enqueue(DMat A, cudaStream_t st);
+// B := Q^T B or Q B by super-blocks of S = apply_q_width(b_alg) columns
+// (qr_apply.cu); U, B 16-byte aligned with even leading dimensions.
+int apply_q_width(int b_alg);
+int apply_q_blocks(DMat U, long k, DMat T, int b_alg, int S, DMat B, bool transpose_q, cudaStream_t st);
 int lu_piv_dev(DMat A, int* d_piv, int* info);       // d_piv: device, relative
 int apply_pivots_dev(DMat A, const int* d_piv, int k1, int k2, bool reverse, cudaStream_t st);
 int laswp_dev(double* A, long ld, int row0, const int* d_piv, int npiv, int c0, int n0, int c1,

@@ -753,12 +753,19 @@ int gemm_f64(cudaStream_t st, bool ta, bool tb, long m, long n, long k, double a
              long ldc, GemmMode mode, long diag_off, const int* guard, int guard_limit, long kmax,
              const GemmSplit* split) {
   if (m <= 0 || n <= 0) return FLA_SUCCESS;
+  const bool keep = split && split->slices;  // leave the partial products
+  if (keep) {  // one slice unless k is split below
+    *split->slices = 1;
+    C = split->p;
+    ldc = (m + 1) & ~1L;
+    beta = 0.0;
+  }
   if (k <= 0 || alpha == 0.0) {
     // C := beta*C only; k == 0 never occurs on the factorization path with
     // beta != 1, so only the trivial case is supported here.
     if (beta == 1.0) return FLA_SUCCESS;
   }
-  if (ta && !tb && mode == GEMM_FULL && !guard && m <= 64 && n <= 64 && k >= 1024) {
+  if (ta && !tb && mode == GEMM_FULL && !guard && !keep && m <= 64 && n <= 64 && k >= 1024) {
     double* Pz = nullptr;
     long S = 0;
     if (gemm_tn_partials(st, m, n, k, A, lda, B, ldb, &Pz, &S) != FLA_SUCCESS) return FLA_FAILURE;
@@ -785,7 +792,7 @@ int gemm_f64(cudaStream_t st, bool ta, bool tb, long m, long n, long k, double a
   CUtensorMap mA, mB;
   // products with at most 32 columns and a long k (the refinement residual
   // R = B - A X): 128 x 32 tiles, k split to fill the GPU
-  const bool narrow = (n <= 32 && mode == GEMM_FULL && !guard && k >= 2048);
+  const bool narrow = (n <= 32 && mode == GEMM_FULL && !guard && !split && k >= 2048);
   // Split K when the output has too few tiles to occupy the GPU and K is
   // long (the W = U^T B products of the QR updates and of FLA_Apply_Q_UT):
   // slices of K go to blockIdx.z, each into its own partial product, and one
@@ -801,6 +808,7 @@ int gemm_f64(cudaStream_t st, bool ta, bool tb, long m, long n, long k, double a
     // a tile's prologue and epilogue outweigh its products), as many as fill
     // the four CTAs an SM holds.
     S = std::min<long>(std::min<long>(4L * sms / tiles, k / 128), (long)(split->elems / (size_t)zs));
+    if (split->max_slices > 0) S = std::min<long>(S, split->max_slices);
   } else if (mode == GEMM_FULL && !guard && (((tiles * 2 <= sms || narrow) && k >= 2048) || capped)) {
     S = std::min<long>(std::min<long>(((narrow ? 4L : 2L) * sms + tiles - 1) / tiles, k / 512), 64);
     if (capped) S = std::min<long>(std::max<long>(S, (k + kmax - 1) / kmax), 64);
@@ -831,7 +839,7 @@ int gemm_f64(cudaStream_t st, bool ta, bool tb, long m, long n, long k, double a
   int* err = ctx().d_status + ST_ERROR;
   double* Cl = S > 1 ? Pz : C;
   const long ldcl = S > 1 ? ldp : ldc;
-  const double al = S > 1 ? 1.0 : alpha, be = S > 1 ? 0.0 : beta;
+  const double al = S > 1 && !keep ? 1.0 : alpha, be = S > 1 ? 0.0 : beta;
   const int pslot = prof_begin(st);
 #define FB_GEMM_LAUNCH(AK, BK_)                                                                                  \
   (small ? launch_small<AK, BK_>(grid, st, mA, mB, Cl, ldcl, m, n, k, al, be, mode, diag_off, err, guard,         \
@@ -847,7 +855,8 @@ int gemm_f64(cudaStream_t st, bool ta, bool tb, long m, long n, long k, double a
   else if (!ta && !tb) FB_GEMM_LAUNCH(false, true);
   else FB_GEMM_LAUNCH(false, false);
 #undef FB_GEMM_LAUNCH
-  if (S > 1) {
+  if (keep) *split->slices = S;
+  if (S > 1 && !keep) {
     const long total = m * n;
     splitk_reduce_kernel<<<(unsigned)std::min<long>(4L * sms, (total + 255) / 256), 256, 0, st>>>(
         Pz, ldp, zs, (int)S, (int)m, (int)n, alpha, beta, C, ldc);

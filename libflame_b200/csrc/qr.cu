@@ -397,6 +397,23 @@ int apply_q_dev(DMat U, DMat T, int b_alg, DMat B, bool transpose_q) {
   cudaStream_t st = cx.stream;
   const long m = U.m, k = std::min(U.m, U.n), nr = B.n;
   if (k == 0 || nr == 0) return FLA_SUCCESS;
+  if (const int Sq = b_alg <= QR_NB ? apply_q_width(b_alg) : 0; Sq > 0 && tma_ok(B.p, B.ld)) {
+    op_begin(st);
+    if (!tma_ok(U.p, U.ld)) {
+      // reflectors off the 16-byte grid: one aligned copy
+      const long ldu = even_up(m);
+      double* Uc = (double*)ws_get(WS_QR_U, sizeof(double) * (size_t)ldu * (size_t)k);
+      if (!Uc) return FLA_FAILURE;
+      FB_CK(cudaMemcpy2DAsync(Uc, sizeof(double) * ldu, U.p, sizeof(double) * U.ld, sizeof(double) * m, k,
+                              cudaMemcpyDeviceToDevice, st));
+      U.p = Uc;
+      U.ld = ldu;
+    }
+    if (apply_q_blocks(U, k, T, b_alg, Sq, B, transpose_q, st) != FLA_SUCCESS) return FLA_FAILURE;
+    op_end(st);
+    return FLA_SUCCESS;
+  }
+  // T blocks wider than 128, or odd ones wider than 64
   const int S = std::max(1, QR_NB / b_alg) * b_alg;
   const long ldy = even_up(m), ldg = even_up(S);
   double* Y = (double*)ws_get(WS_QR_U, sizeof(double) * (size_t)ldy * (size_t)(S + nr));  // [U | B]
