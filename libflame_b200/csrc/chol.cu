@@ -3,7 +3,7 @@
 // Right-looking blocked algorithm with the reference's structure
 // (src/lapack/dec/chol/l/flamec/FLA_Chol_l_blk_var3.c:13-66):
 //   for each 128-column block:  A11 := chol(A11)        [potrf_diag_kernel]
-//                               A21 := A21 inv(A11)^T   [DMMA GEMM with inv(L11)]
+//                               A21 := A21 inv(A11)^T   [rlt_kernel, rlt.cu]
 //                               A22 -= A21 A21^T (lower) [DMMA GEMM engine]
 // with the next block column factored on a second stream while the rest of
 // the trailing update runs (chol_lower_enqueue).
@@ -19,6 +19,7 @@
 #include <climits>
 #include <cstdlib>
 
+#include "chol_leaf.cuh"
 #include "common.h"
 #include "dev_util.cuh"
 
@@ -27,22 +28,10 @@ namespace fb {
 namespace {
 
 constexpr int NB = 128;        // outer block
-constexpr int IB = 32;         // inner block
+constexpr int IB = CHOL_IB;    // inner block
 constexpr int LDS = NB + 4;    // SMEM leading dimension (= 4 mod 16: conflict-free DMMA fragments)
 constexpr int POTRF_THREADS = 256;
 constexpr int POTRF_SMEM = NB * LDS * 8;
-// Block columns of at most this many rows below the diagonal block are
-// solved by substitution; taller ones through inv(L11) and a DMMA GEMM.
-// FLA_B200_CHOL_SUBST_ROWS overrides it for tuning.
-long chol_subst_rows() {
-  static long v = -1;
-  if (v < 0) {
-    v = 4096;
-    if (const char* e = std::getenv("FLA_B200_CHOL_SUBST_ROWS")) v = std::max(0L, std::atol(e));
-  }
-  return v;
-}
-
 __device__ __forceinline__ bool guard_failed(const int* info) {
   return *((volatile const int*)info) != INT_MAX;
 }
@@ -94,76 +83,6 @@ __device__ __forceinline__ void syrk_tiles(double* S, int jb, int r_lo, int nti,
   }
 }
 
-__device__ __forceinline__ void publish(int* cnt, int v) {
-  asm volatile("st.release.cta.shared.b32 [%0], %1;" ::"r"(smem_u32(cnt)), "r"(v) : "memory");
-}
-__device__ __forceinline__ int published(const int* cnt) {
-  int v;
-  asm volatile("ld.acquire.cta.shared.b32 %0, [%1];" : "=r"(v) : "r"(smem_u32(cnt)) : "memory");
-  return v;
-}
-
-// (a): warp 0 factors the w x w diagonal block at (jb, jb).  Every update is
-// unconditional (no divergent branches in the chain): a lane only ever reads
-// a[c] of its own row for c <= lane, and entries above the diagonal or past
-// w never reach those.  After a failing pivot the rest of the block is not
-// meaningful; the failing column is what is reported.  Column j goes to S
-// (lanes below the diagonal and the pivot), its reciprocal pivot to s_rinv[j],
-// then *cnt := base + j + 1.  Columns are published for all of IB, so the
-// readers' waits always end.
-__device__ __forceinline__ void potrf_diag32(double* S, int jb, int w, int lane, double* s_rinv, int* cnt, int base,
-                                             int* s_fail) {
-  double a[IB];
-#pragma unroll
-  for (int c = 0; c < IB; ++c)  // rows past w: unit pivots
-    a[c] = (c <= lane && lane < w) ? S[(jb + lane) + (jb + c) * LDS] : (c == lane ? 1.0 : 0.0);
-  int fail = -1;
-  double d = __shfl_sync(0xffffffffu, a[0], 0);
-#pragma unroll
-  for (int j = 0; j < IB; ++j) {
-    if (!(d > 0.0) && fail < 0 && j < w) fail = j;  // <= 0 or NaN
-    const double rinv = rsqrt(d), sd = d * rinv;
-    a[j] = lane == j ? sd : (lane > j ? a[j] * rinv : a[j]);
-    const double lj = a[j];
-    double* col = S + jb + (jb + j) * LDS;
-    if (lane >= j) col[lane] = lj;
-    if (lane == 0) s_rinv[j] = rinv;
-    if (j + 1 < IB) {
-      // lane j + 1's next pivot from its own multiplier, then the broadcast
-      const double dn = fma(-lj, lj, a[j + 1]);
-      d = __shfl_sync(0xffffffffu, dn, j + 1);
-    }
-    __syncwarp();
-    if (lane == 0) publish(cnt, base + j + 1);
-#pragma unroll
-    for (int c = j + 1; c < IB; ++c) a[c] = fma(-lj, col[c], a[c]);
-  }
-  if (lane == 0 && fail >= 0) *s_fail = jb + fail;
-}
-
-// (a): row r below the diagonal block at (jb, jb), in step with warp 0.
-// The wait is for another warp of this CTA, which needs nothing from the
-// waiting one; it is bounded all the same (*err set when it runs out).
-__device__ __forceinline__ void potrf_row(double* S, int jb, int r, const double* s_rinv, const int* cnt, int base,
-                                          int* err) {
-  double x[IB];
-#pragma unroll
-  for (int c = 0; c < IB; ++c) x[c] = S[r + (jb + c) * LDS];
-  int seen = base;
-#pragma unroll
-  for (int j = 0; j < IB; ++j) {
-    for (int spin = 0; seen < base + j + 1; seen = published(cnt))
-      if (++spin > (1 << 20)) {
-        atomicExch(err, 61);
-        return;
-      }
-    x[j] *= s_rinv[j];
-    S[r + (jb + j) * LDS] = x[j];
-#pragma unroll
-    for (int c = j + 1; c < IB; ++c) x[c] = fma(-x[j], S[(jb + c) + (jb + j) * LDS], x[c]);
-  }
-}
-
 __global__ void __launch_bounds__(POTRF_THREADS, 1) potrf_diag_kernel(double* A, long ld, int b, int gcol,
                                                                    int* info, int* err) {
   extern __shared__ __align__(16) double S[];  // S[r + c*LDS]
@@ -187,10 +106,10 @@ __global__ void __launch_bounds__(POTRF_THREADS, 1) potrf_diag_kernel(double* A,
     // (a); the counter runs on over the chunks (base jb), s_rinv alternates
     double* rinv = s_rinv[(jb / IB) & 1];
     if (warp == 0) {
-      potrf_diag32(S, jb, w, lane, rinv, &s_cnt, jb, &s_fail);
+      potrf_diag32<LDS>(S, jb, w, lane, rinv, &s_cnt, jb, &s_fail);
     } else if (warp < 4) {
       const int r = r0 + (warp - 1) * 32 + lane;
-      if (r < b) potrf_row(S, jb, r, rinv, &s_cnt, jb, err);
+      if (r < b) potrf_row<LDS>(S, jb, r, rinv, &s_cnt, jb, err);
     } else if (jb > 0 && r0 < b) {
       syrk_tiles(S, jb - IB, r0, (b8 - r0) / 8, r0, (b8 - r0) / 8, warp - 4, 4, lane);
     }
@@ -233,8 +152,8 @@ int chol_blocksize() {
 // Enqueue the blocked factorization of the lower triangle of A on `st`.
 // Outer blocks of NBO = 128 or 256 columns; each outer panel is factored as
 // 128-column sub-panels:
-//   sub-panel j:   A11 := chol(A11); inv(L11) formed next to it;
-//                  A21 := A21 inv(L11)^T as a DMMA GEMM;
+//   sub-panel j:   A11 := chol(A11);
+//                  A21 := A21 inv(L11)^T in one launch;
 //                  the panel's later columns -= A21 A21^T
 //   then the panel's rows below its diagonal block are copied transposed,
 //   and step k updates A22(:, next panel) -= A21 A21(next rows)^T, factors
@@ -259,21 +178,19 @@ int chol_lower_enqueue(DMat A, cudaStream_t st) {
   }();
   cudaStream_t sd = (look && st == cx.stream) ? cx.side : st;
   const long NBO = chol_blocksize();
-  double* Linv = (double*)ws_get(WS_MISC, sizeof(double) * NB * NB);
-  double* W = (double*)ws_get(WS_MISC2, sizeof(double) * NB * (size_t)(std::max<long>(0, n - NB) + 2));
   // Transposed copy of each factored outer panel's rows below its diagonal
   // block (NBO x rows, k contiguous), two buffers used in turn: the
   // lookahead and trailing updates take their second operand from it
   // k-contiguous (one 16 x 64 TMA box per stage, the LU's operand shape).
   const long ldpt = NBO;
   double* PT = (double*)ws_get(WS_PANEL_T, sizeof(double) * 2 * (size_t)ldpt * (size_t)std::max<long>(n, 1));
-  if (!Linv || !W || !PT) return FLA_FAILURE;
+  if (!PT) return FLA_FAILURE;
   auto pt_of = [&](long k) { return PT + ((k / NBO) & 1) * (size_t)ldpt * (size_t)n; };
   cudaEvent_t ev_look = cx.ev[2], ev_panel = cx.ev[3];
   auto at = [&](long i, long j) { return A.p + i + j * ld; };
 
-  // 128-column sub-panel at column k: diagonal block, its inverse, and the
-  // block column below it.
+  // 128-column sub-panel at column k: diagonal block and the block column
+  // below it.
   auto sub = [&](long k, cudaStream_t s) -> int {
     const int b = (int)std::min<long>(NB, n - k);
     int ps = prof_begin(s);
@@ -283,16 +200,7 @@ int chol_lower_enqueue(DMat A, cudaStream_t st) {
     FB_CK(cudaGetLastError());
     const long m2 = n - k - b;
     if (m2 <= 0) return FLA_SUCCESS;
-    // a short block column: forward substitution in one launch (the latency
-    // of the inverse, the copy and the product would dominate it)
-    if (m2 <= chol_subst_rows()) return trsm_rlt_subst(at(k, k), at(k + b, k), ld, b, m2, info, (int)(k + b), s);
-    const long ldl = (b + 1) & ~1L;  // TMA: 16-byte leading dimensions
-    if (tri_inverse_lower(at(k, k), ld, b, false, Linv, ldl, s) != FLA_SUCCESS) return FLA_FAILURE;
-    const long ldw = (m2 + 1) & ~1L;
-    FB_CK(cudaMemcpy2DAsync(W, sizeof(double) * ldw, at(k + b, k), sizeof(double) * ld, sizeof(double) * m2, b,
-                            cudaMemcpyDeviceToDevice, s));
-    return gemm_f64(s, false, true, m2, b, b, 1.0, W, ldw, Linv, ldl, 0.0, at(k + b, k), ld, GEMM_FULL, 0, info,
-                    (int)(k + b));
+    return trsm_rlt_subst(at(k, k), at(k + b, k), ld, b, m2, info, (int)(k + b), s);
   };
   // Outer panel at column k: its sub-panels left to right, each followed by
   // the update of the panel's remaining columns; then the transposed copy of

@@ -8,7 +8,7 @@
 //     [A11;A21], p1 := LU_piv([A11;A21])   lu_panel_factor (lu_panel.cu)
 //     pivot [A10;A20] and [A12;A22]         laswp_compose/apply kernels
 //     A12 := inv(tril_unit(A11)) A12         forward substitution, one launch
-//                                            (u12_subst_kernel)
+//                                            (rlt_kernel, rlt.cu)
 //     A22 -= A21 A12                         DMMA GEMM engine
 // run on the transposed matrix, with the next panel factored on a second
 // stream while the trailing update runs (lu_piv_dev below).  Pivot choice is the reference's: the entry of
@@ -585,213 +585,6 @@ int lu_blocksize() {
 // Only three launches stand between the end of one panel and the start of
 // the next.  The side stream has the higher priority, so the panel's CTAs
 // are placed as soon as trailing-update CTAs retire.
-// U12 := inv(L11) A12 on the transposed storage by forward substitution,
-// the order of dtrsm's left, lower, no-transpose, unit case
-// (src/flablas/f2c/dtrsm.c): for j = 0..b-1, rows i > j of every column c
-// lose L11(i, j) U12(j, c).  L11(i, j) is at Ls[j + i ld] (row i of L11 is
-// a contiguous column of A^T), A12(i, c) at X[c + i ld], overwritten.
-// The triangle (b <= 128) sits in shared memory; one warp per RV columns c
-// keeps rows lane, lane+32, lane+64, lane+96 of them in registers, and at
-// step j the owner lane broadcasts U12(j, c): no block barrier inside the
-// sweep, so a step costs one shuffle and a few FMAs of latency.
-constexpr int U12_WARPS = 16;
-constexpr int U12_LDS = NBMAX + 1;  // odd stride: a half-warp reads 16 banks
-// shared memory for a triangle of order b: whole 32-row groups (the sweep
-// reads the rows of every group it touches)
-// (and, after it, the reciprocals of the diagonal for the non-unit form)
-inline size_t u12_smem(int b) { return sizeof(double) * ((size_t)((b + 31) & ~31) * U12_LDS + NBMAX); }
-
-// NU = false: unit lower L11 with L11(i, j) at Ls[j + i ld] (the LU on A^T).
-// NU = true:  non-unit lower L11 with L11(i, j) at Ls[i + j ld] (column-
-//             major, the Cholesky's A21 := A21 inv(L11)^T, rows of A21 as
-//             the right-hand sides); each solved entry is first multiplied
-//             by the reciprocal of its pivot (dtrsm's R,L,T,N case).
-// Returns at once when *guard holds a failing column below guard_limit.
-// TX: the element type of X (float for the low-precision Cholesky's
-// factors: loaded into FP64, solved in FP64, rounded back); X has its own
-// leading dimension ldx.
-template <int RV, bool NU, typename TX = double>
-__global__ void __launch_bounds__(U12_WARPS * 32) u12_subst_kernel(const double* __restrict__ Ls,
-                                                                    TX* __restrict__ X, long ld, int b,
-                                                                    int ncols, const int* guard, int guard_limit,
-                                                                    long ldx) {
-  extern __shared__ double sL[];  // sL[i * U12_LDS + j] = L11(i, j), rows i < 32 ceil(b / 32)
-  double* sR = sL + ((b + 31) & ~31) * U12_LDS;
-  if (guard && *((volatile const int*)guard) < guard_limit) return;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  // The triangle: lanes run along its contiguous index e (a column of L11
-  // for NU, a row for the transposed storage), each warp takes every
-  // sixteenth line o; sixteen loads per lane are in flight before they are
-  // stored (one memory round trip per batch, not per entry).
-  for (int o0 = warp; o0 < b; o0 += U12_WARPS * 4) {
-    double v[4][4];
-#pragma unroll
-    for (int a = 0; a < 4; ++a)
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const int o = o0 + a * U12_WARPS, e = lane + 32 * q;
-        v[a][q] = (o < b && e < b) ? Ls[e + (long)o * ld] : 0.0;
-      }
-#pragma unroll
-    for (int a = 0; a < 4; ++a)
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const int o = o0 + a * U12_WARPS, e = lane + 32 * q;
-        if (o < b && e < b) {
-          if (NU) {
-            sL[e * U12_LDS + o] = v[a][q];  // L11(e, o)
-            if (e == o) sR[o] = 1.0 / v[a][q];
-          } else {
-            sL[o * U12_LDS + e] = v[a][q];  // L11(o, e)
-          }
-        }
-      }
-  }
-  __syncthreads();
-  const int c0 = (blockIdx.x * U12_WARPS + warp) * RV;
-  if (c0 >= ncols) return;
-  double r[4][RV];
-#pragma unroll
-  for (int m = 0; m < 4; ++m)
-#pragma unroll
-    for (int v = 0; v < RV; ++v) {
-      const int i = lane + 32 * m, c = c0 + v;
-      r[m][v] = (i < b && c < ncols) ? (double)X[c + (long)i * ldx] : 0.0;
-    }
-  // rows at or beyond b hold zeros and read unset shared memory of their
-  // group: they are never written back; groups at or beyond b are skipped
-  const int groups = (b + 31) >> 5;
-#pragma unroll
-  for (int slot = 0; slot < 4; ++slot) {
-    if (slot >= groups) break;
-    const int jend = min(32, b - 32 * slot);
-    for (int jj = 0; jj < jend; ++jj) {
-      const int j = 32 * slot + jj;
-      double y[RV];
-#pragma unroll
-      for (int v = 0; v < RV; ++v) y[v] = __shfl_sync(0xffffffffu, r[slot][v], jj);
-      if (NU) {
-        const double rc = sR[j];
-#pragma unroll
-        for (int v = 0; v < RV; ++v) {
-          y[v] *= rc;
-          if (lane == jj) r[slot][v] = y[v];
-        }
-      }
-      const double l0 = sL[(lane + 32 * slot) * U12_LDS + j];
-      if (lane > jj) {
-#pragma unroll
-        for (int v = 0; v < RV; ++v) r[slot][v] = fma(-l0, y[v], r[slot][v]);
-      }
-#pragma unroll
-      for (int m = slot + 1; m < 4; ++m) {
-        if (m < groups) {
-          const double l = sL[(lane + 32 * m) * U12_LDS + j];
-#pragma unroll
-          for (int v = 0; v < RV; ++v) r[m][v] = fma(-l, y[v], r[m][v]);
-        }
-      }
-    }
-  }
-#pragma unroll
-  for (int m = 0; m < 4; ++m)
-#pragma unroll
-    for (int v = 0; v < RV; ++v) {
-      const int i = lane + 32 * m, c = c0 + v;
-      if (i < b && c < ncols) X[c + (long)i * ldx] = (TX)r[m][v];
-    }
-}
-
-template <int RV, bool NU = false, typename TX = double>
-void u12_subst_launch(const double* Ls, TX* X, long ld, int b, int ncols, cudaStream_t st,
-                      const int* guard = nullptr, int guard_limit = 0, long ldx = -1) {
-  static bool attr = false;
-  if (!attr) {
-    cudaFuncSetAttribute(u12_subst_kernel<RV, NU, TX>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)u12_smem(NBMAX));
-    attr = true;
-  }
-  const unsigned grid = (unsigned)((ncols + U12_WARPS * RV - 1) / (U12_WARPS * RV));
-  u12_subst_kernel<RV, NU, TX><<<grid, U12_WARPS * 32, u12_smem(b), st>>>(Ls, X, ld, b, ncols, guard, guard_limit,
-                                                                         ldx < 0 ? ld : ldx);
-}
-
-// X := X inv(L)^T for an ncols x b block X (column-major, ld ld) and a
-// non-unit lower L of order b <= 128 (column-major, same ld): the
-// Cholesky's A21 := A21 inv(L11)^T by forward substitution in one launch.
-int trsm_rlt_subst(const double* L, double* X, long ld, int b, long ncols, const int* guard, int guard_limit,
-                   cudaStream_t st) {
-  if (ncols <= 0 || b <= 0) return FLA_SUCCESS;
-  if (b > NBMAX) {
-    set_last_error("trsm_rlt_subst: triangle wider than 128");
-    return FLA_FAILURE;
-  }
-  const int sms = ctx().num_sms;
-  const int ps = prof_begin(st);
-  if (ncols <= (long)sms * U12_WARPS) u12_subst_launch<1, true>(L, X, ld, b, (int)ncols, st, guard, guard_limit);
-  else if (ncols <= (long)sms * U12_WARPS * 2) u12_subst_launch<2, true>(L, X, ld, b, (int)ncols, st, guard, guard_limit);
-  else if (ncols <= (long)sms * U12_WARPS * 4) u12_subst_launch<4, true>(L, X, ld, b, (int)ncols, st, guard, guard_limit);
-  else u12_subst_launch<8, true>(L, X, ld, b, (int)ncols, st, guard, guard_limit);
-  prof_end(ps, st, PROF_TRSM, (double)ncols * b * b);
-  count_launch();
-  FB_CK(cudaGetLastError());
-  return FLA_SUCCESS;
-}
-
-// The same for an FP32 X (ld ldx) against an FP64 L (ld ldl): the
-// low-precision Cholesky's A21 := A21 inv(L11)^T with L11 its FP64
-// diagonal factor, solved in FP64 and rounded to FP32.
-int trsm_rlt_subst_f32(const double* L, long ldl, float* X, long ldx, int b, long ncols, const int* guard,
-                       int guard_limit, cudaStream_t st) {
-  if (ncols <= 0 || b <= 0) return FLA_SUCCESS;
-  if (b > NBMAX) {
-    set_last_error("trsm_rlt_subst_f32: triangle wider than 128");
-    return FLA_FAILURE;
-  }
-  const int sms = ctx().num_sms;
-  const int ps = prof_begin(st);
-  if (ncols <= (long)sms * U12_WARPS)
-    u12_subst_launch<1, true, float>(L, X, ldl, b, (int)ncols, st, guard, guard_limit, ldx);
-  else if (ncols <= (long)sms * U12_WARPS * 2)
-    u12_subst_launch<2, true, float>(L, X, ldl, b, (int)ncols, st, guard, guard_limit, ldx);
-  else if (ncols <= (long)sms * U12_WARPS * 4)
-    u12_subst_launch<4, true, float>(L, X, ldl, b, (int)ncols, st, guard, guard_limit, ldx);
-  else
-    u12_subst_launch<8, true, float>(L, X, ldl, b, (int)ncols, st, guard, guard_limit, ldx);
-  prof_end(ps, st, PROF_TRSM, (double)ncols * b * b);
-  count_launch();
-  FB_CK(cudaGetLastError());
-  return FLA_SUCCESS;
-}
-
-// U12 := inv(L11) A12 for ncols columns (layout above), any b: blocks of
-// 128 rows, each solved by the kernel, the rows below updated by a GEMM.
-// Columns per warp grow with ncols so that the grid stays about one wave
-// (a 128-row triangle's 132 KB of shared memory allow one CTA per SM).
-int u12_subst(const double* Ls, double* X, long ld, int b, long ncols, cudaStream_t st) {
-  if (ncols <= 0 || b <= 0) return FLA_SUCCESS;
-  const int sms = ctx().num_sms;
-  for (int r0 = 0; r0 < b; r0 += NBMAX) {
-    const int bb = std::min(NBMAX, b - r0);
-    const double* L = Ls + r0 + (long)r0 * ld;
-    double* Y = X + (long)r0 * ld;
-    const int ps = prof_begin(st);
-    if (ncols <= (long)sms * U12_WARPS) u12_subst_launch<1>(L, Y, ld, bb, (int)ncols, st);
-    else if (ncols <= (long)sms * U12_WARPS * 2) u12_subst_launch<2>(L, Y, ld, bb, (int)ncols, st);
-    else if (ncols <= (long)sms * U12_WARPS * 4) u12_subst_launch<4>(L, Y, ld, bb, (int)ncols, st);
-    else u12_subst_launch<8>(L, Y, ld, bb, (int)ncols, st);
-    prof_end(ps, st, PROF_TRSM, (double)ncols * bb * bb);
-    count_launch();
-    FB_CK(cudaGetLastError());
-    const int rest = b - r0 - bb;
-    // U12^T[:, r0+bb:] -= U12^T[:, r0:r0+bb] L11^T[r0:r0+bb, r0+bb:]
-    if (rest > 0 && gemm_f64(st, false, false, ncols, rest, bb, -1.0, Y, ld, Ls + r0 + (long)(r0 + bb) * ld, ld,
-                             1.0, X + (long)(r0 + bb) * ld, ld) != FLA_SUCCESS)
-      return FLA_FAILURE;
-  }
-  return FLA_SUCCESS;
-}
-
 int lu_piv_dev(DMat A, int* d_piv, int* info) {
   set_attrs();
   Context& cx = ctx();

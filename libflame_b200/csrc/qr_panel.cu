@@ -35,7 +35,7 @@
 //      a_q -= x (scale w_q) (row j: a_q -= w_q).  CTA 0 writes column j of T.
 // Bound by the latency of that chain: an 8192 x 32 leaf 151 us with two CTA
 // barriers per column, serial sums and two square roots and two divisions in
-// a row, 120 us in this form (a 12288 x 16 one 86 -> 68 us).
+// a row, 128 us in this form (a 12288 x 16 one 86 -> 70 us).
 // One exchange per column where the reference's order needs two reductions
 // (the norm, then the dot products): the sums are the same up to the
 // rounding of scaling before or after the summation.
@@ -361,8 +361,8 @@ int qleaf_width(long M, int w) {
 
 int qleaf_launch(double* P, long ld, long M, int w, int W, double* T, long ldt, double* U, long ldu,
                  cudaStream_t st) {
-  // as few CTAs as hold the rows: a column's exchange costs more with each
-  // (M = 12288, W = 16: FLA_QR_UT 12288 x 6144 2 ms faster with 12 than 16)
+  // as few CTAs as hold the rows (spreading 12288 x 16 over 16 CTAs instead of
+  // 12 changes nothing: 70 us)
   const long per = (long)QL_THREADS * (32 / W);
   const int C = (int)((M + per - 1) / per);
   QrLeafArgs la;
