@@ -96,7 +96,6 @@ enum WsSlot : int {
   WS_LP2,
   WS_LP3,           //   FP64 panel / inverses
   WS_LP4,           //   inverse blocks kept for the correction solves
-  WS_LP5,           //   coupling blocks of the correction sweeps
   WS_IR0,           //   refinement vectors (FP64 / FP32)
   WS_IR1,
   WS_IR2,
@@ -105,7 +104,7 @@ enum WsSlot : int {
   WS_PERM,          // composed row orders of long pivot sequences
   WS_PERM_T,        // gathered rows
   WS_TRINV,         // inverted diagonal blocks of the solves
-  WS_SOLVE_W,       // block of solved unknowns
+  WS_SOLVE_W,       // exchange buffer of the one-launch triangular solves
   WS_SPLITK,        // partial products of split-K GEMMs (main stream)
   WS_SPLITK_SIDE,   //   (side stream: the two streams' GEMMs may overlap)
   WS_QR_T,          // FLA_QR_UT: the T factors of two panels (ping-pong)
@@ -117,7 +116,6 @@ enum WsSlot : int {
   WS_FLASH2,
   WS_FLASH3,
   WS_PANEL_T,       // transposed copies of Cholesky panels (two, ping-pong)
-  WS_SWEEP,         // ready flags of the one-launch triangular sweeps
   WS_NSLOTS
 };
 void* ws_get(int slot, size_t bytes);  // nullptr on allocation failure
@@ -246,6 +244,8 @@ int trsm_left_dev(DMat T, DMat B, bool lower, bool trans, bool unit, cudaStream_
 int trsm_block(const double* T, long ldt, double* B, long ldb, int b, long n, bool lower,
                bool trans, bool unit, cudaStream_t st);
 int trsm_sweep(DMat T, DMat B, bool lower, bool trans, bool unit, cudaStream_t st);
+int trsm_sweep_f32(const float* F, long ldf, const float* Inv, const float* Y, float* X, long ldb, long n, long nr,
+                   bool trans, bool bwd, cudaStream_t st);
 // X := inv(L), L b x b lower triangular (unit diagonal if unit), X ld ldx.
 int tri_inverse_lower(const double* L, long ldl, int b, bool unit, double* X, long ldx, cudaStream_t st);
 // Inverses of the 128 x 128 diagonal blocks of an n x n triangle, one

@@ -19,8 +19,9 @@
 //   * optional power-of-two equilibration (rows and columns for LU, the
 //     symmetric diag(a_ii)^-1/2 for Cholesky) keeps the 16-bit operands in
 //     range (required for FP16);
-//   * the correction solves run in FP32 with the inverted diagonal blocks
-//     formed during the factorization (two GEMMs per block);
+//   * the correction solves take FP32 right-hand sides and factors, with the
+//     inverted diagonal blocks formed with the factorization, and run in one
+//     launch per triangle, in FP64 inside (trsm_sweep_f32);
 //   * FP64 is used only for r = b - A x (DMMA GEMM), the update of x and the
 //     norms;
 //   * GMRES-IR: the correction equation A d = r is solved by GMRES(m) left-
@@ -141,14 +142,27 @@ __global__ void diag_kernel(const double* __restrict__ A, long lda, int n, doubl
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) v[i] = fabs(A[i + (long)i * lda]);
 }
-// ||A||_inf = max_i sum_j |a_ij|, one thread per row; the maximum is taken
-// with an integer atomicMax on the (non-negative) double's bits
-__global__ void inf_norm_kernel(const double* __restrict__ A, long lda, int n, unsigned long long* out) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
+// ||A||_inf = max_i sum_j |a_ij|: 32 rows per CTA, lane = row, the eight
+// warps taking every eighth column (HBM bound: 256 CTAs with eight loads in
+// flight per thread at n = 8192; one thread per row took 856 us there).  The
+// maximum is taken with an integer atomicMax on the (non-negative) double's
+// bits.
+__global__ void __launch_bounds__(256) inf_norm_kernel(const double* __restrict__ A, long lda, int n,
+                                                       unsigned long long* out) {
+  __shared__ double part[8][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int i = blockIdx.x * 32 + lane;
   double s = 0.0;
-  for (int j = 0; j < n; ++j) s += fabs(A[i + (long)j * lda]);
-  atomicMax(out, (unsigned long long)__double_as_longlong(s));
+  if (i < n) {
+#pragma unroll 8
+    for (int j = warp; j < n; j += 8) s += fabs(A[i + (long)j * lda]);
+  }
+  part[warp][lane] = s;
+  __syncthreads();
+  if (warp == 0 && i < n) {
+    for (int w = 1; w < 8; ++w) s += part[w][lane];
+    atomicMax(out, (unsigned long long)__double_as_longlong(s));
+  }
 }
 // out[c] = max_i |X(i, c)|, one block per column
 __global__ void colmax_kernel(const double* __restrict__ X, long ldx, int n, double* __restrict__ out) {
@@ -255,259 +269,6 @@ __global__ void gather_rows_kernel(const double* __restrict__ R, long ldr, const
   }
 }
 
-// Building blocks of the blocked triangular sweeps (FP32, 128-row blocks,
-// nr <= 32 right-hand sides) of the correction solves.
-// 128 x 128 block of op(P) into registers, 16 float4 per thread, every load
-// in flight at once.  ROWMAJ: element (i, k) at P[k + i * ld], else
-// P[i + k * ld]; the contiguous index runs in float4 steps (the caller
-// guarantees 16-byte alignment and that the float4 holding the last valid
-// element lies inside the allocation).  Columns k >= mk are zero (padding
-// columns would otherwise multiply zeros of the right-hand block by
-// whatever the workspace holds); rows i >= mi are zero too.
-template <bool ROWMAJ>
-__device__ __forceinline__ void block_load(const float* __restrict__ P, long ld, int mi, int mk, float4 (&v)[16]) {
-#pragma unroll
-  for (int j = 0; j < 16; ++j) {
-    const int e4 = threadIdx.x + j * 256;
-    const int a = e4 >> 5, b4 = (e4 & 31) * 4;  // ROWMAJ: (row a, columns b4..); else (column a, rows b4..)
-    const int i = ROWMAJ ? a : b4, k = ROWMAJ ? b4 : a;
-    float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (ROWMAJ ? (i < mi && k < mk) : (k < mk && i < mi))
-      x = *reinterpret_cast<const float4*>(ROWMAJ ? P + k + (long)i * ld : P + i + (long)k * ld);
-    if (ROWMAJ) {
-      if (k + 1 >= mk) x.y = 0.f;
-      if (k + 2 >= mk) x.z = 0.f;
-      if (k + 3 >= mk) x.w = 0.f;
-    } else {
-      if (i + 1 >= mi) x.y = 0.f;
-      if (i + 2 >= mi) x.z = 0.f;
-      if (i + 3 >= mi) x.w = 0.f;
-    }
-    v[j] = x;
-  }
-}
-// ... and into shared memory as sF[i * 129 + k]
-template <bool ROWMAJ>
-__device__ __forceinline__ void block_store(float* sF, const float4 (&v)[16]) {
-#pragma unroll
-  for (int j = 0; j < 16; ++j) {
-    const int e4 = threadIdx.x + j * 256;
-    const int a = e4 >> 5, b4 = (e4 & 31) * 4;
-    if (ROWMAJ) {
-      float* d = sF + a * 129 + b4;
-      d[0] = v[j].x; d[1] = v[j].y; d[2] = v[j].z; d[3] = v[j].w;
-    } else {
-      float* d = sF + b4 * 129 + a;
-      d[0] = v[j].x; d[129] = v[j].y; d[258] = v[j].z; d[387] = v[j].w;
-    }
-  }
-}
-// acc(a, b) += sum_{k < kn} sF(rg + 32 a, k) sX(k, 4 cg + b): lane rg takes
-// rows rg, rg+32, rg+64, rg+96 (conflict-free scalar reads of sF, stride
-// 129), warp cg takes right-hand sides 4cg..4cg+3 (one broadcast float4 of
-// sX per k): 16 FMAs per 5 shared loads.
-__device__ __forceinline__ void block_fma(const float* sF, const float (*sX)[36], int kn, int rg, int cg,
-                                          float (&acc)[4][4]) {
-#pragma unroll 8
-  for (int k = 0; k < kn; ++k) {
-    const float4 x = *reinterpret_cast<const float4*>(&sX[k][4 * cg]);
-#pragma unroll
-    for (int a = 0; a < 4; ++a) {
-      const float f = sF[(rg + 32 * a) * 129 + k];
-      acc[a][0] = fmaf(f, x.x, acc[a][0]);
-      acc[a][1] = fmaf(f, x.y, acc[a][1]);
-      acc[a][2] = fmaf(f, x.z, acc[a][2]);
-      acc[a][3] = fmaf(f, x.w, acc[a][3]);
-    }
-  }
-}
-
-constexpr int SOLVE_SMEM = (128 * 36 + 128 * 129) * 4;
-
-__device__ __forceinline__ int ld_acquire_flag(const int* p) {
-  int v;
-  asm volatile("ld.acquire.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
-__device__ __forceinline__ void st_release_flag(int* p, int v) {
-  asm volatile("st.release.gpu.global.b32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
-
-// Whole blocked triangular sweep in one cooperative launch (FP32, nr <= 32
-// right-hand sides, 128-row blocks):
-//   X_i := op(Inv_i) (Y_i - sum_j op(F)(block i, block j) X_j)
-// over the blocks j solved before i (j < i forward, j > i backward).  CTA g
-// owns the blocks solved g-th, (g + G)-th, ... (G = gridDim.x).  For block i,
-// whose predecessor in solve order is p (i - 1 forward, i + 1 backward):
-//   Z_i := op(Inv_i) (Y_i - sum_{j before p} op(F)(i, j) X_j)
-// is formed while p is still being solved (the contributions are taken as
-// the blocks are published), and once p is published only
-//   X_i := Z_i - W_i X_p,   W_i = op(Inv_i) op(F)(i, p)
-// (W precomputed per factorization, sweep_couplings) remains on the critical
-// path: one block product per block of the chain.  A block is published by
-// its X stores, a fence, and flags[i] := epoch.  Every block depends only on
-// blocks solved earlier and every CTA takes its blocks in solve order, so
-// with all CTAs resident (cooperative launch) the sweep cannot deadlock; each
-// wait is bounded.  X blocks of other CTAs are read through L2
-// (ld.global.cg): they were written during this launch.
-// op(Inv)(i, k) = Inv[k + i * 128] when TI (else Inv[i + k * 128]);
-// op(F)(r, c) = F[c + r * ldf] when TF (else F[r + c * ldf]); W_i(r, c) at
-// W[i * 128 * 128 + r + c * 128].
-template <bool TI, bool TF, bool BWD>
-__global__ void __launch_bounds__(256) solve_sweep_kernel(const float* __restrict__ F, long ldf,
-                                                          const float* __restrict__ Inv,
-                                                          const float* __restrict__ W, float* X,
-                                                          const float* __restrict__ Y, long ldy, int n, int nr,
-                                                          int nblk, int* flags, int epoch, int* err) {
-  extern __shared__ __align__(16) float sm_solve[];
-  float (*sX)[36] = reinterpret_cast<float (*)[36]>(sm_solve);
-  float* sF = sm_solve + 128 * 36;
-  __shared__ int s_ok;
-  const int tid = threadIdx.x;
-  const int rg = tid & 31, cg = tid >> 5;
-  // wait (thread 0, bounded) until block bj is published; CTA-uniform result
-  auto wait_block = [&](int bj) -> bool {
-    if (tid == 0) {
-      int ok = 1;
-      if (ld_acquire_flag(flags + bj) < epoch) {
-        const unsigned long long t0 = globaltimer_ns();
-        while (ld_acquire_flag(flags + bj) < epoch) {
-          if (*((volatile int*)err) != 0 || globaltimer_ns() - t0 > kWaitLimitNs) {
-            atomicExch(err, 51);
-            ok = 0;
-            break;
-          }
-        }
-      }
-      s_ok = ok;
-    }
-    __syncthreads();
-    return s_ok != 0;
-  };
-  auto load_x = [&](int c0, int w) {
-#pragma unroll
-    for (int j = 0; j < 16; ++j) {
-      const int e = tid + j * 256;
-      const int k = e & 127, c = e >> 7;
-      sX[k][c] = (k < w && c < nr) ? __ldcg(X + (long)(c0 + k) + (long)c * ldy) : 0.f;
-    }
-  };
-  for (int q = blockIdx.x; q < nblk; q += gridDim.x) {
-    const int bi = BWD ? nblk - 1 - q : q;
-    const int r0 = bi * 128, wn = min(128, n - r0);
-    float acc[4][4];
-#pragma unroll
-    for (int a = 0; a < 4; ++a)
-#pragma unroll
-      for (int b = 0; b < 4; ++b) acc[a][b] = 0.f;
-    float4 v[16];
-    for (int t = 0; t + 1 < q; ++t) {
-      const int bj = BWD ? nblk - 1 - t : t;
-      const int c0 = bj * 128, w = min(128, n - c0);
-      block_load<TF>(TF ? F + c0 + (long)r0 * ldf : F + r0 + (long)c0 * ldf, ldf, wn, w, v);
-      if (!wait_block(bj)) return;
-      load_x(c0, w);
-      block_store<TF>(sF, v);
-      __syncthreads();
-      block_fma(sF, sX, w, rg, cg, acc);
-      __syncthreads();
-    }
-    // Z_i := op(Inv_i) (Y_i - acc)
-    block_load<TI>(Inv + (long)bi * 128 * 128, 128, wn, wn, v);
-#pragma unroll
-    for (int a = 0; a < 4; ++a) {
-      const int i = rg + 32 * a;
-#pragma unroll
-      for (int b = 0; b < 4; ++b) {
-        const int c = 4 * cg + b;
-        sX[i][c] = (i < wn && c < nr) ? Y[(long)(r0 + i) + (long)c * ldy] - acc[a][b] : 0.f;
-        acc[a][b] = 0.f;
-      }
-    }
-    block_store<TI>(sF, v);
-    __syncthreads();
-    block_fma(sF, sX, wn, rg, cg, acc);
-    if (q > 0) {
-      // X_i := Z_i - W_i X_p once the predecessor p is published
-      const int bp = BWD ? bi + 1 : bi - 1;
-      const int c0 = bp * 128, w = min(128, n - c0);
-      block_load<false>(W + (long)bi * 128 * 128, 128, wn, w, v);
-      __syncthreads();
-      if (!wait_block(bp)) return;
-      load_x(c0, w);
-      block_store<false>(sF, v);
-      __syncthreads();
-#pragma unroll
-      for (int a = 0; a < 4; ++a)
-#pragma unroll
-        for (int b = 0; b < 4; ++b) acc[a][b] = -acc[a][b];
-      block_fma(sF, sX, w, rg, cg, acc);  // acc = W X_p - Z
-#pragma unroll
-      for (int a = 0; a < 4; ++a)
-#pragma unroll
-        for (int b = 0; b < 4; ++b) acc[a][b] = -acc[a][b];
-    }
-#pragma unroll
-    for (int a = 0; a < 4; ++a) {
-      const int i = rg + 32 * a;
-      if (i < wn)
-#pragma unroll
-        for (int b = 0; b < 4; ++b)
-          if (4 * cg + b < nr) __stcg(X + (long)(r0 + i) + (long)(4 * cg + b) * ldy, acc[a][b]);
-    }
-    __threadfence();
-    __syncthreads();
-    if (tid == 0) st_release_flag(flags + bi, epoch);
-  }
-}
-
-// Coupling blocks of the sweeps: W_i = op(Inv_i) op(F)(block i, block p),
-// p the block solved just before i (i - 1 forward, i + 1 backward), one CTA
-// per block, four 32-column passes of the 128 x 128 x 128 product; W_i(r, c)
-// at W[i * 128 * 128 + r + c * 128].
-template <bool TI, bool TF, bool BWD>
-__global__ void __launch_bounds__(256) sweep_coupling_kernel(const float* __restrict__ F, long ldf,
-                                                             const float* __restrict__ Inv, float* __restrict__ W,
-                                                             int n, int nblk) {
-  extern __shared__ __align__(16) float sm_solve[];
-  float (*sX)[36] = reinterpret_cast<float (*)[36]>(sm_solve);
-  float* sF = sm_solve + 128 * 36;
-  const int bi = blockIdx.x;
-  const int bp = BWD ? bi + 1 : bi - 1;
-  if (bp < 0 || bp >= nblk) return;
-  const int tid = threadIdx.x, rg = tid & 31, cg = tid >> 5;
-  const int r0 = bi * 128, wn = min(128, n - r0), c0 = bp * 128, w = min(128, n - c0);
-  float4 v[16];
-  block_load<TI>(Inv + (long)bi * 128 * 128, 128, wn, wn, v);
-  block_store<TI>(sF, v);
-  for (int pc = 0; pc < 4; ++pc) {
-    // sX(k, c) = op(F)(r0 + k, c0 + 32 pc + c)
-    for (int e = tid; e < 128 * 32; e += 256) {
-      const int k = e & 127, c = e >> 7;
-      const int col = 32 * pc + c;
-      sX[k][c] = (k < wn && col < w) ? (TF ? F[(c0 + col) + (long)(r0 + k) * ldf] : F[(r0 + k) + (long)(c0 + col) * ldf])
-                                     : 0.f;
-    }
-    __syncthreads();
-    float acc[4][4];
-#pragma unroll
-    for (int a = 0; a < 4; ++a)
-#pragma unroll
-      for (int b = 0; b < 4; ++b) acc[a][b] = 0.f;
-    block_fma(sF, sX, wn, rg, cg, acc);
-#pragma unroll
-    for (int a = 0; a < 4; ++a) {
-      const int i = rg + 32 * a;
-#pragma unroll
-      for (int b = 0; b < 4; ++b) {
-        const int c = 32 * pc + 4 * cg + b;
-        W[(long)bi * 128 * 128 + i + c * 128] = (i < wn && c < w) ? acc[a][b] : 0.f;
-      }
-    }
-    __syncthreads();
-  }
-}
-
 inline int grid_for(long total) { return (int)std::min<long>(8192, (total + 255) / 256); }
 
 }  // namespace
@@ -569,39 +330,6 @@ int lp_workspace(long n, LpFactor* f, LpWork* w) {
 }
 
 }  // namespace
-
-// Coupling blocks of both correction sweeps for the current factors (see
-// solve_sweep_kernel), one launch per direction.
-int lp_couplings(LpFactor* f, cudaStream_t st) {
-  const long n = f->n;
-  const long nblk = (n + MB - 1) / MB;
-  float* w = (float*)ws_get(WS_LP5, sizeof(float) * 2 * (size_t)std::max<long>(nblk, 1) * MB * MB);
-  if (!w) return FLA_FAILURE;
-  f->wf = w;
-  f->wb = w + (size_t)nblk * MB * MB;
-  static bool attr = false;
-  if (!attr) {
-    FB_CK(cudaFuncSetAttribute(sweep_coupling_kernel<false, false, false>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize, SOLVE_SMEM));
-    FB_CK(cudaFuncSetAttribute(sweep_coupling_kernel<true, true, false>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize, SOLVE_SMEM));
-    FB_CK(cudaFuncSetAttribute(sweep_coupling_kernel<true, true, true>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize, SOLVE_SMEM));
-    attr = true;
-  }
-  if (f->chol)
-    sweep_coupling_kernel<false, false, false><<<(unsigned)nblk, 256, SOLVE_SMEM, st>>>(f->F, f->ldf, f->inv1,
-                                                                                        f->wf, (int)n, (int)nblk);
-  else
-    sweep_coupling_kernel<true, true, false><<<(unsigned)nblk, 256, SOLVE_SMEM, st>>>(f->F, f->ldf, f->inv1, f->wf,
-                                                                                      (int)n, (int)nblk);
-  sweep_coupling_kernel<true, true, true><<<(unsigned)nblk, 256, SOLVE_SMEM, st>>>(
-      f->F, f->ldf, f->chol ? f->inv1 : f->inv2, f->wb, (int)n, (int)nblk);
-  count_launch(2);
-  FB_CK(cudaGetLastError());
-  f->coupled = true;
-  return FLA_SUCCESS;
-}
 
 // LU with partial pivoting of (diag(sr) A diag(sc)) in low precision, on the
 // transposed FP32 copy F = (scaled A)^T (n x n, ld ldf): the layout and the
@@ -695,7 +423,6 @@ int lp_lu_factor(DMat A, LowPrec prec, bool scale, LpFactor* f) {
     count_launch();
     FB_CK(cudaGetLastError());
   }
-  if (lp_couplings(f, st) != FLA_SUCCESS) return FLA_FAILURE;
   int info = -1;
   if (status_read(&info) != FLA_SUCCESS) return FLA_FAILURE;
   f->info = info;
@@ -799,7 +526,6 @@ int lp_chol_factor_shift(DMat A, bool upper, LowPrec prec, bool scale, double si
   const long nblk = (n + MB - 1) / MB;
   if (tri_inverse_blocks(w.P64, MB, n, true, false, w.Xall, st) != FLA_SUCCESS) return FLA_FAILURE;
   if (convert2d<float, double>(st, w.Xall, MB, f->inv1, MB, MB, nblk * MB) != FLA_SUCCESS) return FLA_FAILURE;
-  if (lp_couplings(f, st) != FLA_SUCCESS) return FLA_FAILURE;
   int inf = -1;
   if (status_read(&inf) != FLA_SUCCESS) return FLA_FAILURE;
   f->info = inf;
@@ -823,58 +549,6 @@ int lp_chol_factor(DMat A, bool upper, LowPrec prec, bool scale, LpFactor* f) {
   return FLA_SUCCESS;
 }
 
-// One triangular sweep of the correction solve in a single cooperative
-// launch (solve_sweep_kernel): forward (L y = rhs) or backward (L^T x = y,
-// U x = y).  The ready flags live in a workspace slot that is zeroed when it
-// is (re)allocated; each sweep publishes a new epoch, so no reset is needed
-// between sweeps.
-int sweep(const LpFactor& f, const float* Yin, float* Xout, long n, long nrhs, bool backward, cudaStream_t st) {
-  static void* last_flags = nullptr;
-  static int epoch = 0;
-  static int max_ctas = 0;
-  const long nblk = (n + MB - 1) / MB;
-  int* flags = (int*)ws_get(WS_SWEEP, sizeof(int) * (size_t)std::max<long>(nblk, 1024));
-  if (!flags) return FLA_FAILURE;
-  if (flags != last_flags) {
-    FB_CK(cudaMemsetAsync(flags, 0, sizeof(int) * (size_t)std::max<long>(nblk, 1024), st));
-    last_flags = flags;
-    epoch = 0;
-  }
-  ++epoch;
-  if (max_ctas == 0) {
-    FB_CK(cudaFuncSetAttribute(solve_sweep_kernel<true, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               SOLVE_SMEM));
-    FB_CK(cudaFuncSetAttribute(solve_sweep_kernel<false, false, false>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize, SOLVE_SMEM));
-    FB_CK(cudaFuncSetAttribute(solve_sweep_kernel<true, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               SOLVE_SMEM));
-    int per_sm = 0;
-    FB_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, solve_sweep_kernel<true, true, true>, 256,
-                                                        SOLVE_SMEM));
-    max_ctas = std::max(1, per_sm) * ctx().num_sms;
-  }
-  const int G = (int)std::min<long>(nblk, max_ctas);
-  const float* F = f.F;
-  long ldf = f.ldf;
-  const float* inv = backward ? (f.chol ? f.inv1 : f.inv2) : f.inv1;
-  const float* Wc = backward ? f.wb : f.wf;
-  float* X = Xout;
-  const float* Y = Yin;
-  long ldy = n;
-  int ni = (int)n, nr = (int)nrhs, nb = (int)nblk, ep = epoch;
-  int* err = ctx().d_status + ST_ERROR;
-  void* args[] = {(void*)&F, (void*)&ldf, (void*)&inv, (void*)&Wc, (void*)&X, (void*)&Y, (void*)&ldy,
-                  (void*)&ni, (void*)&nr, (void*)&nb, (void*)&flags, (void*)&ep, (void*)&err};
-  void* fn;
-  if (backward) fn = (void*)solve_sweep_kernel<true, true, true>;
-  else fn = f.chol ? (void*)solve_sweep_kernel<false, false, false> : (void*)solve_sweep_kernel<true, true, false>;
-  const int ps = prof_begin(st);
-  FB_CK(cudaLaunchCooperativeKernel(fn, dim3(G), dim3(256), args, SOLVE_SMEM, st));
-  prof_end(ps, st, PROF_TRSM, (double)n * (double)n * (double)nrhs);
-  count_launch();
-  return FLA_SUCCESS;
-}
-
 // ===========================================================================
 // Correction solve with the low-precision factors: D := M^-1 R (FP64 in and
 // out, FP32 inside).  T is an FP32 n x nrhs workspace, ld n.
@@ -895,10 +569,13 @@ int lp_solve(const LpFactor& f, const double* R, long ldr, double* D, long ldd, 
   }
   count_launch();
   // Forward sweep L y = T (T -> Tb), backward sweep U x = y or L^T x = y
-  // (Tb -> T): one cooperative launch each while nrhs <= 32.
-  if (nrhs <= 32) {
-    if (sweep(f, T, Tb, n, nrhs, false, st) != FLA_SUCCESS) return FLA_FAILURE;
-    if (sweep(f, Tb, T, n, nrhs, true, st) != FLA_SUCCESS) return FLA_FAILURE;
+  // (Tb -> T): one cooperative launch each (trsm.cu) up to 256 columns.
+  // Cholesky: F = L, forward L, backward L^T; LU: F = (L U)^T, both
+  // transposed.
+  if (nrhs <= 256) {
+    if (trsm_sweep_f32(F, ldf, f.inv1, T, Tb, n, n, nrhs, !f.chol, false, st) != FLA_SUCCESS) return FLA_FAILURE;
+    if (trsm_sweep_f32(F, ldf, f.chol ? f.inv1 : f.inv2, Tb, T, n, n, nrhs, true, true, st) != FLA_SUCCESS)
+      return FLA_FAILURE;
   } else {
     // wide right-hand sides: sgemm per block
     for (long kb = 0; kb < nblk; ++kb) {
@@ -1114,7 +791,7 @@ int ir_refine(const DMat& A, const DMat& B, double* X, long ldx, const LpFactor&
   // cte = ||A||_inf * eps * sqrt(n)  (dsgesv.c:287-289)
   unsigned long long* dn = (unsigned long long*)b.small;
   FB_CK(cudaMemsetAsync(dn, 0, sizeof(unsigned long long), st));
-  inf_norm_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(A.p, A.ld, (int)n, dn);
+  inf_norm_kernel<<<(unsigned)((n + 31) / 32), 256, 0, st>>>(A.p, A.ld, (int)n, dn);
   count_launch();
   unsigned long long bits = 0;
   FB_CK(cudaMemcpyAsync(&bits, dn, sizeof(bits), cudaMemcpyDeviceToHost, st));

@@ -181,60 +181,90 @@ __global__ void __launch_bounds__(INV_WARPS * 32) tri_inv_kernel(const double* _
 // start as all-ones (a NaN no arithmetic produces): a reader polls the data
 // itself, one trip through L2 per step instead of store, fence, flag, poll
 // and load.  Per step of the chain: that trip and two 64 x 64 x 16 DMMA
-// products.  n = 8192, 32 columns: 444 us, 3.5 us per
-// block.
+// products.  n = 8192, 32 columns: 3.0 us per block (FP64 factors), 2.6 us
+// (FP32).
 // ---------------------------------------------------------------------------
 constexpr int SB = 64;                  // block rows
 constexpr int SC = 16;                  // right-hand sides per task
 constexpr int SH = SB / 2;              // k-width of a half tile
-constexpr int SLD = SB + 4;             // = 4 mod 16: conflict-free fragments
-constexpr int SLDH = SH + 4;
-constexpr int S_HALF = SB * SLDH;       // doubles of a half tile (either layout)
-constexpr size_t SWEEP_SMEM = sizeof(double) * (2 * S_HALF + SB * SLD + 2 * SC * SLD);
-static_assert(SH * SLD <= S_HALF, "half tile");
+constexpr int SLD = SB + 4;             // X, Z: = 4 mod 16, conflict-free fragments
+// Tiles of op(T) and the inverse in the factor's type TF, in either storage:
+// row index contiguous (ld RI) or k contiguous (ld KH for a half tile, KF for
+// the inverse).  A fragment load touches rows g = 0..7 and k = t = 0..3 (half
+// of them at a time for doubles): conflict-free with RI = 4 mod 16 doubles or 8
+// mod 32 floats, KH, KF = 4 mod 16 doubles or 4 mod 32 floats.
+template <typename TF>
+struct SweepTile {
+  static constexpr int RI = sizeof(TF) == 8 ? SB + 4 : SB + 8;
+  static constexpr int KH = SH + 4, KF = SB + 4;
+  static constexpr int HALF = SB * KH > SH * RI ? SB * KH : SH * RI;
+  static constexpr int FULL = SB * (RI > KF ? RI : KF);
+  static constexpr size_t SMEM = sizeof(TF) * (2 * HALF + FULL) + sizeof(double) * 2 * SC * SLD;
+};
 
-__device__ __forceinline__ void cp_async16(double* dst, const double* src, int bytes) {
+// 16 bytes, the first `bytes` of them from src, the rest zero
+__device__ __forceinline__ void cp_async16(void* dst, const void* src, int bytes) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(bytes) : "memory");
 }
 
-// TRANS: op(T)(r, c) = T(c, r).  BWD: blocks solved last to first.
-template <bool TRANS, bool BWD>
-__global__ void __launch_bounds__(256, 2) trsm_sweep_kernel(const double* __restrict__ T, long ldt,
-                                                            const double* __restrict__ Inv, double* B, long ldb,
-                                                            double* XB, int n, int nr, int nblk, int* err) {
-  extern __shared__ __align__(16) double sw_sm[];
-  double* sT = sw_sm;                   // two half tiles
-  double* sI = sT + 2 * S_HALF;         // op(Inv_q)
-  double* sX = sI + SB * SLD;           // X_j: sX[k + c * SLD]
-  double* sZ = sX + SC * SLD;           // Y_q - sum
+template <typename TF, typename TV>
+struct SweepArgs {
+  const TF* T;     // n x n triangle, ld ldt
+  long ldt;
+  const TF* Inv;   // inverse of block q at Inv + (q / per) * istride + (q % per) * SB * (1 + ldi), ld ldi
+  long ldi, istride;
+  int per;
+  const TV* Y;     // right-hand sides (ld ldb); may be X
+  TV* X;           // solutions (ld ldb)
+  long ldb;
+  double* XB;      // exchange buffer, nblk * SB x nr, all ones
+  int n, nr, nblk;
+  int* err;
+};
+
+// TRANS: op(T)(r, c) = T(c, r), op(Inv) alike.  BWD: blocks solved last to
+// first.  Products and sums in FP64 for either type of factor.
+template <bool TRANS, bool BWD, typename TF, typename TV>
+__global__ void __launch_bounds__(256, 2) trsm_sweep_kernel(SweepArgs<TF, TV> a) {
+  using ST = SweepTile<TF>;
+  constexpr int V = 16 / sizeof(TF);    // elements per copy
+  extern __shared__ __align__(16) unsigned char sw_sm[];
+  double* sX = reinterpret_cast<double*>(sw_sm);  // X_j: sX[k + c * SLD]
+  double* sZ = sX + SC * SLD;                     // Y_q - sum
+  TF* sT = reinterpret_cast<TF*>(sZ + SC * SLD);  // two half tiles
+  TF* sI = sT + 2 * ST::HALF;                     // op(Inv_q)
   __shared__ int s_dead;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int g = lane >> 2, t = lane & 3;
   const int i0 = warp * 8 + g;          // this lane's row of the block
+  const int n = a.n, nr = a.nr, nblk = a.nblk;
   const int ngrp = (nr + SC - 1) / SC;
   const long ldx = (long)nblk * SB;     // exchange buffer: padded rows x columns
   if (tid == 0) s_dead = 0;
   __syncthreads();
-  // half tile h of op(T)(block bi, block bj) into buffer buf; entries past n
-  // read as zero.  Stored as it lies in memory: row index contiguous
-  // (sT[i + k * SLD]) or, transposed, k contiguous (sT[k + i * SLDH]).
-  auto load_half = [&](int bi, int bj, int h, double* buf) {
-    const int r0 = bi * SB, c0 = bj * SB + h * SH;
+  // an mr x mk block stored row index contiguous (TRANS: k contiguous) at
+  // src, ld lds, into dst; rows past vr and columns past vk read as zero
+  auto load_tile = [&](const TF* src, long lds, int mk, int vr, int vk, TF* dst, int ldk) {
     if (TRANS) {
-      for (int e = tid; e < SB * (SH / 2); e += 256) {
-        const int k = (e % (SH / 2)) * 2, i = e / (SH / 2);
-        const int left = r0 + i < n ? n - (c0 + k) : 0;
-        cp_async16(buf + k + i * SLDH, left > 0 ? T + (c0 + k) + (long)(r0 + i) * ldt : T,
-                   left >= 2 ? 16 : left == 1 ? 8 : 0);
+      for (int e = tid; e < SB * (mk / V); e += 256) {
+        const int k = (e % (mk / V)) * V, i = e / (mk / V);
+        const int left = i < vr ? min(V, max(0, vk - k)) : 0;
+        cp_async16(dst + k + i * ldk, left > 0 ? src + k + (long)i * lds : src, left * (int)sizeof(TF));
       }
     } else {
-      for (int e = tid; e < (SB / 2) * SH; e += 256) {
-        const int i = (e % (SB / 2)) * 2, k = e / (SB / 2);
-        const int left = c0 + k < n ? n - (r0 + i) : 0;
-        cp_async16(buf + i + k * SLD, left > 0 ? T + (r0 + i) + (long)(c0 + k) * ldt : T,
-                   left >= 2 ? 16 : left == 1 ? 8 : 0);
+      for (int e = tid; e < (SB / V) * mk; e += 256) {
+        const int i = (e % (SB / V)) * V, k = e / (SB / V);
+        const int left = k < vk ? min(V, max(0, vr - i)) : 0;
+        cp_async16(dst + i + k * ST::RI, left > 0 ? src + i + (long)k * lds : src, left * (int)sizeof(TF));
       }
     }
+  };
+  // half tile h of op(T)(block bi, block bj)
+  auto load_half = [&](int bi, int bj, int h, TF* buf) {
+    const int r0 = bi * SB, c0 = bj * SB + h * SH;
+    const TF* src = a.T + (TRANS ? c0 + (long)r0 * a.ldt : r0 + (long)c0 * a.ldt);
+    if (c0 < n) load_tile(src, a.ldt, SH, n - r0, n - c0, buf, ST::KH);
+    else load_tile(a.T, a.ldt, SH, 0, 0, buf, ST::KH);
   };
   auto commit = [] { asm volatile("cp.async.commit_group;" ::: "memory"); };
   // the 64 x 16 block X_bj of this group from the exchange buffer, as soon as
@@ -243,7 +273,7 @@ __global__ void __launch_bounds__(256, 2) trsm_sweep_kernel(const double* __rest
     const int c = tid >> 4, k0 = (tid & 15) * 4;  // column, four consecutive rows
     double v[4] = {0.0, 0.0, 0.0, 0.0};
     if (c < nc) {
-      const double* p = XB + (long)bj * SB + k0 + (long)(col0 + c) * ldx;
+      const double* p = a.XB + (long)bj * SB + k0 + (long)(col0 + c) * ldx;
       unsigned long long start = 0;
       int spins = 0;
       for (;;) {
@@ -259,7 +289,7 @@ __global__ void __launch_bounds__(256, 2) trsm_sweep_kernel(const double* __rest
           const unsigned long long now = globaltimer_ns();
           if (start == 0) start = now;
           if (*((volatile int*)&s_dead) || now - start > kWaitLimitNs) {
-            atomicExch(err, 52);
+            atomicExch(a.err, 52);
             *((volatile int*)&s_dead) = 1;
             break;
           }
@@ -275,32 +305,36 @@ __global__ void __launch_bounds__(256, 2) trsm_sweep_kernel(const double* __rest
     const int bi = BWD ? nblk - 1 - q : q, r0 = bi * SB;
     auto blk = [&](int j) { return BWD ? nblk - 1 - j : j; };
     __syncthreads();  // the buffers of the previous task are free
-    // group 0: the inverse, in the layout of the full tile; group 1: the
-    // first half tile
-    for (int e = tid; e < SB * SB / 2; e += 256) {
-      const int a = (e % (SB / 2)) * 2, b = e / (SB / 2);
-      cp_async16(sI + a + b * SLD, Inv + (long)bi * SB * SB + a + b * SB, 16);
-    }
+    load_tile(a.Inv + (bi / a.per) * a.istride + (long)(bi % a.per) * SB * (1 + a.ldi), a.ldi, SB, n - r0, n - r0, sI,
+              ST::KF);
     commit();
     if (q > 0) load_half(bi, blk(0), 0, sT);
     commit();
+    double y[2][2];  // the right-hand sides: read before any solution of this block is stored
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int c = 8 * h + 2 * t + e;
+        y[h][e] = (r0 + i0 < n && c < nc) ? (double)a.Y[(long)(r0 + i0) + (long)(col0 + c) * a.ldb] : 0.0;
+      }
     // acc[n-tile][parity of the k-step]: four chains of DMMAs
     double acc[2][2][2] = {};
     for (int u = 0; u < 2 * q; ++u) {
-      if (u + 1 < 2 * q) load_half(bi, blk((u + 1) >> 1), (u + 1) & 1, sT + ((u + 1) & 1) * S_HALF);
+      if (u + 1 < 2 * q) load_half(bi, blk((u + 1) >> 1), (u + 1) & 1, sT + ((u + 1) & 1) * ST::HALF);
       commit();
       if ((u & 1) == 0) poll_x(blk(u >> 1), col0, nc);
       asm volatile("cp.async.wait_group 1;" ::: "memory");
       __syncthreads();
-      const double* buf = sT + (u & 1) * S_HALF;
-      const double* pa = TRANS ? buf + t + i0 * SLDH : buf + i0 + t * SLD;
+      const TF* buf = sT + (u & 1) * ST::HALF;
+      const TF* pa = TRANS ? buf + t + i0 * ST::KH : buf + i0 + t * ST::RI;
       const double* pb = sX + (u & 1) * SH + t + g * SLD;
 #pragma unroll
       for (int k = 0; k < SH; k += 4) {
-        const double a = TRANS ? pa[k] : pa[k * SLD];
+        const double x = (double)(TRANS ? pa[k] : pa[k * ST::RI]);
         const double b0 = pb[k], b1 = pb[k + 8 * SLD];
-        dmma_884(acc[0][(k >> 2) & 1][0], acc[0][(k >> 2) & 1][1], a, b0);
-        dmma_884(acc[1][(k >> 2) & 1][0], acc[1][(k >> 2) & 1][1], a, b1);
+        dmma_884(acc[0][(k >> 2) & 1][0], acc[0][(k >> 2) & 1][1], x, b0);
+        dmma_884(acc[1][(k >> 2) & 1][0], acc[1][(k >> 2) & 1][1], x, b1);
       }
       __syncthreads();
     }
@@ -309,21 +343,19 @@ __global__ void __launch_bounds__(256, 2) trsm_sweep_kernel(const double* __rest
     for (int h = 0; h < 2; ++h)
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
-        const int c = 8 * h + 2 * t + e;
-        const double y = (r0 + i0 < n && c < nc) ? B[(long)(r0 + i0) + (long)(col0 + c) * ldb] : 0.0;
-        sZ[i0 + c * SLD] = y - (acc[h][0][e] + acc[h][1][e]);
+        sZ[i0 + (8 * h + 2 * t + e) * SLD] = y[h][e] - (acc[h][0][e] + acc[h][1][e]);
         acc[h][0][e] = acc[h][1][e] = 0.0;
       }
     __syncthreads();
     // op(Inv)(i, k): Inv(i, k), or Inv(k, i) when transposed
-    const double* pa = TRANS ? sI + t + i0 * SLD : sI + i0 + t * SLD;
+    const TF* pa = TRANS ? sI + t + i0 * ST::KF : sI + i0 + t * ST::RI;
     const double* pb = sZ + t + g * SLD;
 #pragma unroll
     for (int k = 0; k < SB; k += 4) {
-      const double a = TRANS ? pa[k] : pa[k * SLD];
+      const double x = (double)(TRANS ? pa[k] : pa[k * ST::RI]);
       const double b0 = pb[k], b1 = pb[k + 8 * SLD];
-      dmma_884(acc[0][(k >> 2) & 1][0], acc[0][(k >> 2) & 1][1], a, b0);
-      dmma_884(acc[1][(k >> 2) & 1][0], acc[1][(k >> 2) & 1][1], a, b1);
+      dmma_884(acc[0][(k >> 2) & 1][0], acc[0][(k >> 2) & 1][1], x, b0);
+      dmma_884(acc[1][(k >> 2) & 1][0], acc[1][(k >> 2) & 1][1], x, b1);
     }
 #pragma unroll
     for (int h = 0; h < 2; ++h)
@@ -333,9 +365,10 @@ __global__ void __launch_bounds__(256, 2) trsm_sweep_kernel(const double* __rest
         double x = acc[h][0][e] + acc[h][1][e];
         if (__double_as_longlong(x) == -1ll) x = __longlong_as_double(0x7ff8000000000000ll);  // another NaN
         if (c < nc) {
-          asm volatile("st.relaxed.gpu.global.f64 [%0], %1;" ::"l"(XB + (long)r0 + i0 + (long)(col0 + c) * ldx), "d"(x)
+          asm volatile("st.relaxed.gpu.global.f64 [%0], %1;" ::"l"(a.XB + (long)r0 + i0 + (long)(col0 + c) * ldx),
+                       "d"(x)
                        : "memory");
-          if (r0 + i0 < n) B[(long)(r0 + i0) + (long)(col0 + c) * ldb] = x;
+          if (r0 + i0 < n) a.X[(long)(r0 + i0) + (long)(col0 + c) * a.ldb] = (TV)x;
         }
       }
   }
@@ -374,47 +407,81 @@ void set_attrs() {
 
 }  // namespace
 
-// B := inv(op(T)) B by trsm_sweep_kernel: T n x n, B n x nr, 16-byte aligned
-// with even leading dimensions.
-int trsm_sweep(DMat T, DMat B, bool lower, bool trans, bool unit, cudaStream_t st) {
-  set_attrs();
-  const long n = T.m, nr = B.n, nblk = (n + SB - 1) / SB, ngrp = (nr + SC - 1) / SC;
-  void* const kern = lower ? (trans ? (void*)trsm_sweep_kernel<true, true> : (void*)trsm_sweep_kernel<false, false>)
-                           : (trans ? (void*)trsm_sweep_kernel<true, false> : (void*)trsm_sweep_kernel<false, true>);
+template <typename TF, typename TV>
+int sweep_launch(SweepArgs<TF, TV> a, bool trans, bool bwd, cudaStream_t st) {
+  void* const kern = bwd ? (trans ? (void*)trsm_sweep_kernel<true, true, TF, TV> : (void*)trsm_sweep_kernel<false, true, TF, TV>)
+                         : (trans ? (void*)trsm_sweep_kernel<true, false, TF, TV> : (void*)trsm_sweep_kernel<false, false, TF, TV>);
+  constexpr size_t smem = SweepTile<TF>::SMEM;
   static int resident = 0;
   if (resident == 0) {
     int per = 0;
-    for (void* f : {(void*)trsm_sweep_kernel<true, true>, (void*)trsm_sweep_kernel<false, false>,
-                    (void*)trsm_sweep_kernel<true, false>, (void*)trsm_sweep_kernel<false, true>}) {
-      FB_CK(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SWEEP_SMEM));
+    for (void* f : {(void*)trsm_sweep_kernel<true, true, TF, TV>, (void*)trsm_sweep_kernel<false, true, TF, TV>,
+                    (void*)trsm_sweep_kernel<true, false, TF, TV>, (void*)trsm_sweep_kernel<false, false, TF, TV>}) {
+      FB_CK(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
       int p = 0;
-      FB_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&p, f, 256, SWEEP_SMEM));
+      FB_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&p, f, 256, smem));
       per = per == 0 ? p : std::min(per, p);
     }
     resident = std::max(1, per) * ctx().num_sms;
   }
-  double* Inv = (double*)ws_get(WS_TRINV, sizeof(double) * (size_t)nblk * SB * SB);
-  const size_t xbytes = sizeof(double) * (size_t)nblk * SB * (size_t)nr;
-  double* XB = (double*)ws_get(WS_SOLVE_W, xbytes);
-  if (!Inv || !XB) return FLA_FAILURE;
-  FB_CK(cudaMemsetAsync(XB, 0xff, xbytes, st));
-  // the last block's inverse is smaller than its 64 x 64 slot
-  if (n % SB) FB_CK(cudaMemsetAsync(Inv + (nblk - 1) * SB * SB, 0, sizeof(double) * SB * SB, st));
-  if (tri_inverse_blocks_bs(T.p, T.ld, n, SB, lower, unit, Inv, st) != FLA_SUCCESS) return FLA_FAILURE;
-  const double *tp = T.p, *ip = Inv;
-  double* bp = B.p;
-  long ldt = T.ld, ldb = B.ld;
-  int ni = (int)n, nri = (int)nr, nb = (int)nblk;
-  int* err = ctx().d_status + ST_SOLVE;
+  a.nblk = (a.n + SB - 1) / SB;
+  const long tasks = (long)a.nblk * ((a.nr + SC - 1) / SC);
+  const size_t xbytes = sizeof(double) * (size_t)a.nblk * SB * (size_t)a.nr;
+  a.XB = (double*)ws_get(WS_SOLVE_W, xbytes);
+  if (!a.XB) return FLA_FAILURE;
+  FB_CK(cudaMemsetAsync(a.XB, 0xff, xbytes, st));
+  a.err = ctx().d_status + ST_SOLVE;
   ctx().solve_pending = true;
-  void* args[] = {(void*)&tp, (void*)&ldt, (void*)&ip, (void*)&bp, (void*)&ldb, (void*)&XB,
-                  (void*)&ni, (void*)&nri, (void*)&nb, (void*)&err};
-  const unsigned G = (unsigned)std::min<long>(nblk * ngrp, resident);
+  void* args[] = {(void*)&a};
   const int ps = prof_begin(st);
-  FB_CK(cudaLaunchCooperativeKernel(kern, dim3(G), dim3(256), args, SWEEP_SMEM, st));
-  prof_end(ps, st, PROF_TRSM, (double)n * n * nr);
+  FB_CK(cudaLaunchCooperativeKernel(kern, dim3((unsigned)std::min<long>(tasks, resident)), dim3(256), args, smem, st));
+  prof_end(ps, st, PROF_TRSM, (double)a.n * a.n * a.nr);
   count_launch();
   return FLA_SUCCESS;
+}
+
+// B := inv(op(T)) B by trsm_sweep_kernel: T n x n, B n x nr, T 16-byte
+// aligned with an even leading dimension.
+int trsm_sweep(DMat T, DMat B, bool lower, bool trans, bool unit, cudaStream_t st) {
+  const long n = T.m, nblk = (n + SB - 1) / SB;
+  double* Inv = (double*)ws_get(WS_TRINV, sizeof(double) * (size_t)nblk * SB * SB);
+  if (!Inv) return FLA_FAILURE;
+  if (tri_inverse_blocks_bs(T.p, T.ld, n, SB, lower, unit, Inv, st) != FLA_SUCCESS) return FLA_FAILURE;
+  SweepArgs<double, double> a = {};
+  a.T = T.p;
+  a.ldt = T.ld;
+  a.Inv = Inv;
+  a.ldi = SB;
+  a.istride = SB * SB;
+  a.per = 1;
+  a.Y = B.p;
+  a.X = B.p;
+  a.ldb = B.ld;
+  a.n = (int)n;
+  a.nr = (int)B.n;
+  return sweep_launch(a, trans, lower == trans, st);
+}
+
+// X := inv(op(F)) Y for the FP32 factors of the mixed-precision solvers, in
+// FP64 inside: F n x n (ld ldf a multiple of 4), Inv the FP32 inverses of its
+// 128 x 128 diagonal blocks (128 * 128 apart, ld 128; the diagonal halves of
+// a triangle's inverse are the inverses of its diagonal halves), X, Y n x nr
+// with leading dimension ldb.
+int trsm_sweep_f32(const float* F, long ldf, const float* Inv, const float* Y, float* X, long ldb, long n, long nr,
+                   bool trans, bool bwd, cudaStream_t st) {
+  SweepArgs<float, float> a = {};
+  a.T = F;
+  a.ldt = ldf;
+  a.Inv = Inv;
+  a.ldi = 2 * SB;
+  a.istride = 4 * SB * SB;
+  a.per = 2;
+  a.Y = Y;
+  a.X = X;
+  a.ldb = ldb;
+  a.n = (int)n;
+  a.nr = (int)nr;
+  return sweep_launch(a, trans, bwd, st);
 }
 
 // B := inv(op(T)) B for a b x n block B, T b x b (b <= 128) triangular.
