@@ -656,43 +656,42 @@ __global__ void __launch_bounds__(BT, 1) lu_batched_kernel(BatchArgs<T> a) {
 
 template <typename T>
 int launch_batched(bool lu, BatchArgs<T> args, cudaStream_t st) {
-  if constexpr (sizeof(T) == 8) {
-    if (!lu) {
-      // FP64 Cholesky: the DMMA kernel (orders up to 1024)
-      static bool dattr = false;
-      if (!dattr) {
-        FB_CK(cudaFuncSetAttribute(chol_batched_dmma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)DSMEM_BYTES));
-        dattr = true;
-      }
-      const int grid = std::min(ctx().num_sms, std::max(1, args.count));
-      const int ps = prof_begin(st);
-      chol_batched_dmma_kernel<<<grid, DT, DSMEM_BYTES, st>>>(args);
-      prof_end(ps, st, PROF_OTHER, 0.0);
-      count_launch();
-      FB_CK(cudaGetLastError());
-      return FLA_SUCCESS;
-    }
-  }
-  static bool attr[2] = {false, false};
-  const size_t smem = BSmem<T>::BYTES;
-  if (!attr[lu ? 1 : 0]) {
-    if (lu)
-      FB_CK(cudaFuncSetAttribute(lu_batched_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    else
-      FB_CK(cudaFuncSetAttribute(chol_batched_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    attr[lu ? 1 : 0] = true;
-  }
   const int grid = std::min(ctx().num_sms, std::max(1, args.count));
-  const int ps = prof_begin(st);
-  if (lu)
-    lu_batched_kernel<T><<<grid, BT, smem, st>>>(args);
-  else
-    chol_batched_kernel<T><<<grid, BT, smem, st>>>(args);
-  prof_end(ps, st, PROF_OTHER, 0.0);
-  count_launch();
-  FB_CK(cudaGetLastError());
-  return FLA_SUCCESS;
+  if constexpr (sizeof(T) == 8) {
+    // FP64 Cholesky: the DMMA kernel (orders up to 1024); the FP64 LU is
+    // batched_lu_f64
+    static bool dattr = false;
+    if (!dattr) {
+      FB_CK(cudaFuncSetAttribute(chol_batched_dmma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)DSMEM_BYTES));
+      dattr = true;
+    }
+    const int ps = prof_begin(st);
+    chol_batched_dmma_kernel<<<grid, DT, DSMEM_BYTES, st>>>(args);
+    prof_end(ps, st, PROF_OTHER, 0.0);
+    count_launch();
+    FB_CK(cudaGetLastError());
+    return FLA_SUCCESS;
+  } else {
+    static bool attr[2] = {false, false};
+    const size_t smem = BSmem<T>::BYTES;
+    if (!attr[lu ? 1 : 0]) {
+      if (lu)
+        FB_CK(cudaFuncSetAttribute(lu_batched_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      else
+        FB_CK(cudaFuncSetAttribute(chol_batched_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      attr[lu ? 1 : 0] = true;
+    }
+    const int ps = prof_begin(st);
+    if (lu)
+      lu_batched_kernel<T><<<grid, BT, smem, st>>>(args);
+    else
+      chol_batched_kernel<T><<<grid, BT, smem, st>>>(args);
+    prof_end(ps, st, PROF_OTHER, 0.0);
+    count_launch();
+    FB_CK(cudaGetLastError());
+    return FLA_SUCCESS;
+  }
 }
 
 // per-device panel width by matrix order (autotuned), index 0..BMAXN
@@ -730,7 +729,7 @@ int batched_factor(bool lu, int count, const int* h_n, T** d_A, const long* d_ld
   std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return h_n[x] > h_n[y]; });
   int* dwork = (int*)ws_get(WS_MISC, sizeof(int) * ((size_t)count + 64));
   if (!dwork) return FLA_FAILURE;
-  FB_CK(cudaMemsetAsync(dwork, 0, sizeof(int), st));
+  FB_CK(cudaMemsetAsync(dwork, 0, 4 * sizeof(int), st));
   FB_CK(cudaMemcpyAsync(dwork + 32, order.data(), sizeof(int) * count, cudaMemcpyHostToDevice, st));
   BatchArgs<T> a;
   a.count = count;
@@ -750,6 +749,13 @@ int batched_factor(bool lu, int count, const int* h_n, T** d_A, const long* d_ld
   if (!a.nb_of_size) return FLA_FAILURE;
   // the host order must stay valid until the copy is done
   FB_CK(cudaStreamSynchronize(st));
+  if constexpr (sizeof(T) == 8) {
+    // matrices above order 512 (Cholesky only) and above 256 in the schedule
+    int top = 0, mid = 0;
+    while (top < count && h_n[order[top]] > BMAXN) ++top;
+    while (top + mid < count && h_n[order[top + mid]] > 256) ++mid;
+    if (lu) return batched_lu_f64(a, mid, h_n[order[0]], st);
+  }
   return launch_batched<T>(lu, a, st);
 }
 template int batched_factor<double>(bool, int, const int*, double**, const long*, const int*, int**, int, double**,

@@ -36,6 +36,7 @@
 
 #include "common.h"
 #include "dev_util.cuh"
+#include "lu_leaf.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -321,7 +322,6 @@ __global__ void __launch_bounds__(LEAF_THREADS, 1) lu_leaf_cluster_kernel(LeafAr
 // CTA has finished reading column j's (it must first have passed column
 // j + 1's exchange, which needs this CTA's column j + 1 copies, issued
 // after its column j work).
-constexpr int RLEAF_THREADS = 512;
 constexpr int RLEAF_NW = RLEAF_THREADS / 32;
 
 // One exchange slot: 16-byte header and the W entries of the row.
@@ -331,13 +331,6 @@ struct RSlot {
   int row;                 // global row of the candidate (INT_MAX: none)
   int pad;
   double v[W];
-};
-
-// A warp's candidate: ordering key and row.
-struct RHdr {
-  unsigned long long key;
-  int row;
-  int pad;
 };
 
 // Layout: hdr [2][16] (the warps' candidates), cslot [2][C] (the CTAs'
@@ -352,42 +345,6 @@ __host__ __device__ inline size_t rleaf_smem_bytes(int w, int C) {
   return rleaf_tile_offset(w, C) + sizeof(double) * RLEAF_NW * 32 * ((size_t)w + 1) + 128;
 }
 
-// Non-negative magnitudes order like their bit patterns, so the key orders
-// candidates by magnitude; no candidate orders below every magnitude (and
-// NaN never becomes a candidate: `t > best` is false for it).
-__device__ __forceinline__ unsigned long long rleaf_key(double bv, int bi) {
-  return bi == INT_MAX ? 0ull : (unsigned long long)__double_as_longlong(bv) + 1ull;
-}
-
-// Warp argmax of (key, row): the largest key, the smallest row among equal
-// keys; every lane receives the result.  Rows are distinct, INT_MAX marks
-// no candidate (key 0).
-__device__ __forceinline__ void rleaf_argmax_warp(unsigned long long& key, int& row) {
-  const unsigned hi = (unsigned)(key >> 32), lo = (unsigned)key;
-  const unsigned mhi = __reduce_max_sync(0xffffffffu, hi);
-  const unsigned mlo = __reduce_max_sync(0xffffffffu, hi == mhi ? lo : 0u);
-  const bool top = hi == mhi && lo == mlo;
-  row = (int)__reduce_min_sync(0xffffffffu, top ? (unsigned)row : 0xffffffffu);
-  key = ((unsigned long long)mhi << 32) | mlo;
-}
-
-template <int W, int RPT>
-__device__ __forceinline__ double rleaf_pick(const double (&rv)[RPT][W], int k, int q) {
-  double v = rv[0][q];
-#pragma unroll
-  for (int kk = 1; kk < RPT; ++kk)
-    if (kk == k) v = rv[kk][q];
-  return v;
-}
-
-// Row slot k of the calling thread into shared memory (16-byte aligned).
-template <int W, int RPT>
-__device__ __forceinline__ void rleaf_store_row(const double (&rv)[RPT][W], int k, double* dst) {
-#pragma unroll
-  for (int q = 0; q < W; q += 2)
-    *reinterpret_cast<double2*>(dst + q) = make_double2(rleaf_pick<W, RPT>(rv, k, q), rleaf_pick<W, RPT>(rv, k, q + 1));
-}
-
 // The warp's 32 rows of slot k (slab rows base .. base + 31) pass through
 // its 32 x (W + 1) shared tile, so every global access of the warp reads or
 // writes whole rows (W contiguous doubles) instead of one entry of 32 rows.
@@ -397,7 +354,7 @@ __device__ __forceinline__ void rleaf_load(double (&rv)[RPT][W], const LeafArgs&
 #pragma unroll
   for (int k = 0; k < RPT; ++k) {
     const int base = warp * 32 + k * RLEAF_THREADS;
-#pragma unroll 8
+#pragma unroll 16
     for (int e = lane; e < 32 * W; e += 32) {
       const int rr = e / W, q = e % W;
       tile[rr * (W + 1) + q] = (base + rr < rows) ? a.P[(long)(r0 + base + rr) * a.ld + q] : 0.0;
@@ -424,72 +381,6 @@ __device__ __forceinline__ void rleaf_store(const double (&rv)[RPT][W], const Le
       if (base + rr < rows) a.P[(long)(r0 + base + rr) * a.ld + q] = tile[rr * (W + 1) + q];
     }
     __syncwarp();
-  }
-}
-
-// Entry j (run-time) of a register row: a select chain over compile-time
-// indices, so the row stays in registers.
-template <int W>
-__device__ __forceinline__ double rleaf_pick_col(const double (&row)[W], int j) {
-  double v = row[0];
-#pragma unroll
-  for (int q = 1; q < W; ++q)
-    if (q == j) v = row[q];
-  return v;
-}
-
-// Column J of the leaf for the calling thread's rows, J a compile-time
-// constant so every register of a row is addressed directly: exchange
-// rows j and r, scale column J below the pivot (reciprocal multiply, as
-// bl1_dinvscalv), rank-1 update, and the candidate for column J + 1.
-template <int W, int RPT, int J>
-__device__ __forceinline__ void rleaf_column(double (&rv)[RPT][W], int tid, int r0, int rows, int r,
-                                             const double* u, const double* oldj, double rinv, double& bv,
-                                             int& bi, int& bk) {
-#pragma unroll
-  for (int k = 0; k < RPT; ++k) {
-    const int i = tid + k * RLEAF_THREADS, gi = r0 + i;
-    if (i >= rows || gi < J) continue;
-    if (gi == J) {
-      if (r != J)
-#pragma unroll
-        for (int q = 0; q < W; ++q) rv[k][q] = u[q];
-      continue;
-    }
-    if (gi == r)
-#pragma unroll
-      for (int q = 0; q < W; ++q) rv[k][q] = oldj[q];
-    const double l = rv[k][J] * rinv;
-    rv[k][J] = l;
-#pragma unroll
-    for (int q = J + 1; q < W; ++q) rv[k][q] = fma(-l, u[q], rv[k][q]);
-    if constexpr (J + 1 < W) {
-      const double t = fabs(rv[k][J + 1]);
-      if (t > bv) { bv = t; bi = gi; bk = k; }
-    }
-  }
-}
-
-// Run-time column j to its compile-time body through one jump table.
-template <int W, int RPT>
-__device__ __forceinline__ void rleaf_column_at(int j, double (&rv)[RPT][W], int tid, int r0, int rows, int r,
-                                                const double* u, const double* oldj, double rinv, double& bv,
-                                                int& bi, int& bk) {
-  static_assert(W <= 32, "leaf width");
-  switch (j) {
-#define FB_RLEAF_CASE(J)                                                              \
-  case J:                                                                             \
-    if constexpr (J < W) rleaf_column<W, RPT, J>(rv, tid, r0, rows, r, u, oldj, rinv, bv, bi, bk); \
-    break;
-    FB_RLEAF_CASE(0) FB_RLEAF_CASE(1) FB_RLEAF_CASE(2) FB_RLEAF_CASE(3) FB_RLEAF_CASE(4) FB_RLEAF_CASE(5)
-    FB_RLEAF_CASE(6) FB_RLEAF_CASE(7) FB_RLEAF_CASE(8) FB_RLEAF_CASE(9) FB_RLEAF_CASE(10) FB_RLEAF_CASE(11)
-    FB_RLEAF_CASE(12) FB_RLEAF_CASE(13) FB_RLEAF_CASE(14) FB_RLEAF_CASE(15) FB_RLEAF_CASE(16)
-    FB_RLEAF_CASE(17) FB_RLEAF_CASE(18) FB_RLEAF_CASE(19) FB_RLEAF_CASE(20) FB_RLEAF_CASE(21)
-    FB_RLEAF_CASE(22) FB_RLEAF_CASE(23) FB_RLEAF_CASE(24) FB_RLEAF_CASE(25) FB_RLEAF_CASE(26)
-    FB_RLEAF_CASE(27) FB_RLEAF_CASE(28) FB_RLEAF_CASE(29) FB_RLEAF_CASE(30) FB_RLEAF_CASE(31)
-#undef FB_RLEAF_CASE
-    default:
-      break;
   }
 }
 
