@@ -755,6 +755,23 @@ int batched_factor(bool lu, int count, const int* h_n, T** d_A, const long* d_ld
     while (top < count && h_n[order[top]] > BMAXN) ++top;
     while (top + mid < count && h_n[order[top + mid]] > 256) ++mid;
     if (lu) return batched_lu_f64(a, mid, h_n[order[0]], st);
+    BatchArgs<T> rest = a;
+    rest.count = count - top;
+    rest.order = a.order + top;
+    rest.counter = a.counter + 1;
+    if (top == 0) return batched_chol_f64(rest, mid, st);
+    // the large ones first, the others beside them on the second stream as
+    // SMs become free
+    Context& cx = ctx();
+    a.count = top;
+    if (rest.count == 0) return launch_batched<T>(lu, a, st);
+    FB_CK(cudaEventRecord(cx.ev[0], st));
+    FB_CK(cudaStreamWaitEvent(cx.side, cx.ev[0], 0));
+    if (launch_batched<T>(lu, a, st) != FLA_SUCCESS || batched_chol_f64(rest, mid, cx.side) != FLA_SUCCESS)
+      return FLA_FAILURE;
+    FB_CK(cudaEventRecord(cx.ev[1], cx.side));
+    FB_CK(cudaStreamWaitEvent(st, cx.ev[1], 0));
+    return FLA_SUCCESS;
   }
   return launch_batched<T>(lu, a, st);
 }
