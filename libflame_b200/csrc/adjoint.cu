@@ -108,7 +108,30 @@ __global__ void __cluster_dims__(ADJ_CL, 1, 1) __launch_bounds__(ADJ_THREADS)
       }
     }
   };
-  load_x([&](int i, int j) { return L[i + (long)j * ld]; });
+  // triangles that are only copied: asynchronous copies, all in flight, in
+  // pairs of rows where the source allows it
+  auto copy_x = [&](const double* __restrict__ src, long lds) {
+    const bool vec = ((reinterpret_cast<uintptr_t>(src) | (uintptr_t)(lds * 8)) & 15u) == 0;
+    for (int e = tid; e < AB * AB / 2; e += ADJ_THREADS) {
+      const int i = (e & (AB / 2 - 1)) * 2, j = e >> 6;
+      double* d = sX + i + j * ADJ_LD;
+      if (vec && i > j && i + 1 < w) {
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(d)), "l"(src + i + (long)j * lds)
+                     : "memory");
+      } else {
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          if (in(i + u, j))
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(d + u)),
+                         "l"(src + i + u + (long)j * lds)
+                         : "memory");
+          else d[u] = 0.0;
+        }
+      }
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+  };
+  copy_x(L, ld);
   {
     double v[8];
 #pragma unroll
@@ -134,7 +157,7 @@ __global__ void __cluster_dims__(ADJ_CL, 1, 1) __launch_bounds__(ADJ_THREADS)
   __syncthreads();
   adj_xtz(sX, sD, warp, lane, v2);  // Dbar^T D(:, J)
   __syncthreads();
-  load_x([&](int i, int j) { return Dinv[i + j * AB]; });
+  copy_x(Dinv, AB);
   const int g = lane >> 2, t = lane & 3;
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
@@ -211,18 +234,27 @@ bool g_adj_attr = false;
 }  // namespace
 
 // Scratch of chol_adjoint_dev for order n, in doubles: the inverses of all
-// diagonal blocks, W (ldw x AB: S over Cbar), the product Cbar^T C, and the
-// partial products of `splits` slices of an AB-row GEMM.
+// diagonal blocks, two W (ldw x AB each: S over Cbar, of two consecutive
+// blocks), the product Cbar^T C, and the partial products of `splits` slices
+// of an AB-row GEMM for either stream.
 static long adj_ldw(long n) { return (n + AB + 1) & ~1L; }
 size_t chol_adjoint_scratch(long n, int splits) {
   const size_t nblk = (size_t)((n + AB - 1) / AB);
-  return nblk * AB * AB + (size_t)adj_ldw(n) * AB + (size_t)AB * AB + (size_t)splits * AB * (size_t)(n + AB);
+  return nblk * AB * AB + 2 * (size_t)adj_ldw(n) * AB + (size_t)AB * AB + 2 * (size_t)splits * AB * (size_t)(n + AB);
 }
 
 // In place over Lb (lower triangle); L lower Cholesky factor; n x n, ld.
 // scratch: chol_adjoint_scratch(n, splits) doubles of device memory, used by
-// this call alone until its work on st is done.
-int chol_adjoint_dev(const double* L, double* Lb, long ld, long n, cudaStream_t st, double* scratch, int splits) {
+// this call alone until its work is done.
+//
+// The chain from block to block (Cbar inv(D), Cbar^T C, the diagonal block,
+// and the updates of the next block's columns) runs on `sd`; the updates of
+// the columns left of the next block run on `st`, one block behind, beside the
+// next block's chain.  sd == st: in stream order (the batched form, whose
+// matrices overlap one another).  n = 4096: 4.46 ms in stream order, 3.81
+// ms so.
+int chol_adjoint_dev(const double* L, double* Lb, long ld, long n, cudaStream_t st, cudaStream_t sd, double* scratch,
+                     int splits) {
   if (n <= 0) return FLA_SUCCESS;
   if (!g_adj_attr) {
     FB_CK(cudaFuncSetAttribute(chol_adj_diag_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ADJ_SMEM));
@@ -231,48 +263,75 @@ int chol_adjoint_dev(const double* L, double* Lb, long ld, long n, cudaStream_t 
   const long nblk = (n + AB - 1) / AB;
   const long ldw = adj_ldw(n);
   double* Dinv = scratch;
-  double* W = Dinv + (size_t)nblk * AB * AB;
-  double* G = W + (size_t)ldw * AB;
-  GemmSplit sp;
-  sp.p = G + (size_t)AB * AB;
-  sp.elems = (size_t)splits * AB * (size_t)(n + AB);
+  double* W2 = Dinv + (size_t)nblk * AB * AB;
+  double* G = W2 + 2 * (size_t)ldw * AB;
+  GemmSplit sp_chain, sp_rest;
+  sp_chain.p = G + (size_t)AB * AB;
+  sp_chain.elems = sp_rest.elems = (size_t)splits * AB * (size_t)(n + AB);
+  sp_rest.p = sp_chain.p + sp_chain.elems;
   auto Lat = [&](long i, long j) { return L + i + j * ld; };
   auto Bat = [&](long i, long j) { return Lb + i + j * ld; };
+  const bool two = sd != st;
+  cudaEvent_t ev_chain = ctx().ev[0], ev_rest = ctx().ev[1];
   if (tri_inverse_blocks(L, ld, n, true, false, Dinv, st) != FLA_SUCCESS) return FLA_FAILURE;
+  if (two) {
+    FB_CK(cudaEventRecord(ev_rest, st));
+    FB_CK(cudaStreamWaitEvent(sd, ev_rest, 0));
+  }
+  // columns [c0, c1) left of block q lose its contribution (rows j0 .. n - 1):
+  //   Rbar := Rbar - (Dbar + Dbar^T) R - Cbar^T B: S over Cbar in W against R
+  //   over B, one product of depth w + m;  Bbar := Bbar - Cbar R
+  auto update = [&](const double* W, long j0, int w, long m, long c0, long c1, cudaStream_t s,
+                    const GemmSplit* sp) -> int {
+    if (c1 <= c0) return FLA_SUCCESS;
+    if (gemm_f64(s, true, false, w, c1 - c0, w + m, -1.0, W, ldw, Lat(j0, c0), ld, 1.0, Bat(j0, c0), ld, GEMM_FULL, 0,
+                 nullptr, 0, 0, sp) != FLA_SUCCESS)
+      return FLA_FAILURE;
+    if (m > 0 && gemm_f64(s, false, false, m, c1 - c0, w, -1.0, W + w, ldw, Lat(j0, c0), ld, 1.0, Bat(j0 + w, c0), ld) !=
+                     FLA_SUCCESS)
+      return FLA_FAILURE;
+    return FLA_SUCCESS;
+  };
   for (long q = nblk - 1; q >= 0; --q) {
     const long j0 = q * AB;
     const int w = (int)std::min<long>(AB, n - j0);
     const long m = n - j0 - w;  // rows below the block (w = AB when there are any)
+    const long jn = std::max<long>(0, j0 - AB);  // the next block's first column
     const double* Dq = Dinv + (size_t)q * AB * AB;
+    double* W = W2 + (size_t)(q & 1) * ldw * AB;
     double* Cb = W + w;  // Cbar, below the block's S in W
     if (m > 0) {
       // Cbar := Cbar inv(D)
-      if (gemm_f64(st, false, false, m, w, w, 1.0, Bat(j0 + w, j0), ld, Dq, AB, 0.0, Cb, ldw) != FLA_SUCCESS)
+      if (gemm_f64(sd, false, false, m, w, w, 1.0, Bat(j0 + w, j0), ld, Dq, AB, 0.0, Cb, ldw) != FLA_SUCCESS)
         return FLA_FAILURE;
       // G := Cbar^T C, which Dbar loses in the diagonal kernel
-      if (gemm_f64(st, true, false, w, w, m, 1.0, Cb, ldw, Lat(j0 + w, j0), ld, 0.0, G, AB, GEMM_FULL, 0, nullptr, 0,
-                   0, &sp) != FLA_SUCCESS)
+      if (gemm_f64(sd, true, false, w, w, m, 1.0, Cb, ldw, Lat(j0 + w, j0), ld, 0.0, G, AB, GEMM_FULL, 0, nullptr, 0,
+                   0, &sp_chain) != FLA_SUCCESS)
         return FLA_FAILURE;
     }
-    const int ps = prof_begin(st);
-    chol_adj_diag_kernel<<<ADJ_CL, ADJ_THREADS, ADJ_SMEM, st>>>(Lat(j0, j0), Dq, Bat(j0, j0), ld, w,
+    const int ps = prof_begin(sd);
+    chol_adj_diag_kernel<<<ADJ_CL, ADJ_THREADS, ADJ_SMEM, sd>>>(Lat(j0, j0), Dq, Bat(j0, j0), ld, w,
                                                                m > 0 ? G : nullptr, W, ldw);
-    prof_end(ps, st, PROF_DIAG, 2.0 * w * (double)w * w / 3.0);
+    prof_end(ps, sd, PROF_DIAG, 2.0 * w * (double)w * w / 3.0);
     count_launch();
     FB_CK(cudaGetLastError());
-    // Rbar := Rbar - (Dbar + Dbar^T) R - Cbar^T B: S over Cbar in W against
-    // R over B, one product of depth w + m
-    if (j0 > 0 && gemm_f64(st, true, false, w, j0, w + m, -1.0, W, ldw, Lat(j0, 0), ld, 1.0, Bat(j0, 0), ld, GEMM_FULL,
-                           0, nullptr, 0, 0, &sp) != FLA_SUCCESS)
+    if (two) {
+      // the next block's columns have the other blocks' contributions once the
+      // updates of the block before this one are done
+      FB_CK(cudaEventRecord(ev_chain, sd));
+      FB_CK(cudaStreamWaitEvent(sd, ev_rest, 0));
+      FB_CK(cudaStreamWaitEvent(st, ev_chain, 0));
+    }
+    if (update(W, j0, w, m, jn, j0, sd, &sp_chain) != FLA_SUCCESS || update(W, j0, w, m, 0, jn, st, &sp_rest) != FLA_SUCCESS)
       return FLA_FAILURE;
-    if (m > 0) {
-      // Bbar := Bbar - Cbar R
-      if (j0 > 0 && gemm_f64(st, false, false, m, j0, w, -1.0, Cb, ldw, Lat(j0, 0), ld, 1.0, Bat(j0 + w, 0), ld) !=
-                        FLA_SUCCESS)
-        return FLA_FAILURE;
+    if (m > 0)
       FB_CK(cudaMemcpy2DAsync(Bat(j0 + w, j0), sizeof(double) * ld, Cb, sizeof(double) * ldw, sizeof(double) * m, w,
                               cudaMemcpyDeviceToDevice, st));
-    }
+    if (two) FB_CK(cudaEventRecord(ev_rest, st));
+  }
+  if (two) {
+    FB_CK(cudaEventRecord(ev_chain, sd));
+    FB_CK(cudaStreamWaitEvent(st, ev_chain, 0));
   }
   FB_CK(cudaGetLastError());
   return FLA_SUCCESS;
@@ -334,7 +393,8 @@ FLA_Error FLA_Chol_adjoint(FLA_Uplo uplo, FLA_Obj L, FLA_Obj Lbar) {
   op_begin(st);
   double* scr = (double*)ws_get(WS_ADJ, sizeof(double) * chol_adjoint_scratch((long)L.m, 16));
   if (!scr) return FLA_FAILURE;
-  if (chol_adjoint_dev((const double*)sl.dev, (double*)sb.dev, sl.ld, (long)L.m, st, scr, 16) != FLA_SUCCESS)
+  if (chol_adjoint_dev((const double*)sl.dev, (double*)sb.dev, sl.ld, (long)L.m, st, ctx().side, scr, 16) !=
+      FLA_SUCCESS)
     return FLA_FAILURE;
   op_end(st);
   if (unstage(sb) != FLA_SUCCESS || sync_all() != FLA_SUCCESS) return FLA_FAILURE;
@@ -438,7 +498,7 @@ FLA_Error FLA_Chol_adjoint_batched(int count, const int* n, double** L, const in
     if (n[i] == 0) continue;
     if (logdet_scale != 0.0 && logdet_adjoint_dev(L[i], Lbar[i], ld[i], n[i], logdet_scale, pool[q]) != FLA_SUCCESS)
       return FLA_FAILURE;
-    if (chol_adjoint_dev(L[i], Lbar[i], ld[i], n[i], pool[q], scr + per * q, 4) != FLA_SUCCESS) return FLA_FAILURE;
+    if (chol_adjoint_dev(L[i], Lbar[i], ld[i], n[i], pool[q], pool[q], scr + per * q, 4) != FLA_SUCCESS) return FLA_FAILURE;
   }
   for (int q = 0; q < NS; ++q) {
     FB_CK(cudaEventRecord(ev[q], pool[q]));
