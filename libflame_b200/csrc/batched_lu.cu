@@ -24,7 +24,9 @@
 // matrix's panel overlaps the other's updates; larger ones in CTAs of 512.
 // Measured: 2500 matrices, n uniform in 8..512, 4 right-hand sides: 47.4 ms
 // with a left-looking panel in shared memory on FP64 FMAs (ten barriers and a
-// serial exchange loop per column), 16.1 ms in this form.
+// serial exchange loop per column), 15.0 ms in this form.  (Registers that
+// rotate so that one loop body serves every column of the panel were slower:
+// 1.1 against 0.96 us a column.)
 #include <algorithm>
 
 #include "batched.h"
@@ -62,18 +64,23 @@ __device__ void lub_transpose(double* W, int ldw, double* G, long ldg, int nr, i
   const int tr = (nr + 31) / 32, tc = (nc + 31) / 32;
   for (int e = warp; e < tr * tc; e += NT / 32) {
     const int r0 = (e % tr) * 32, c0 = (e / tr) * 32;
+    double v[32];  // the whole tile in flight
     if (IN) {
-#pragma unroll 16
+#pragma unroll
       for (int q = 0; q < 32; ++q)
-        tile[lane * 33 + q] = (r0 + lane < nr && c0 + q < nc) ? G[(long)(r0 + lane) + (long)(c0 + q) * ldg] : 0.0;
+        v[q] = (r0 + lane < nr && c0 + q < nc) ? G[(long)(r0 + lane) + (long)(c0 + q) * ldg] : 0.0;
+#pragma unroll
+      for (int q = 0; q < 32; ++q) tile[lane * 33 + q] = v[q];
       __syncwarp();
 #pragma unroll 16
       for (int q = 0; q < 32; ++q)
         if (r0 + q < nr && c0 + lane < nc) W[(long)(r0 + q) * ldw + c0 + lane] = tile[q * 33 + lane];
     } else {
-#pragma unroll 16
+#pragma unroll
       for (int q = 0; q < 32; ++q)
-        tile[q * 33 + lane] = (r0 + q < nr && c0 + lane < nc) ? W[(long)(r0 + q) * ldw + c0 + lane] : 0.0;
+        v[q] = (r0 + q < nr && c0 + lane < nc) ? W[(long)(r0 + q) * ldw + c0 + lane] : 0.0;
+#pragma unroll
+      for (int q = 0; q < 32; ++q) tile[q * 33 + lane] = v[q];
       __syncwarp();
 #pragma unroll 16
       for (int q = 0; q < 32; ++q)
@@ -96,7 +103,8 @@ __global__ void __launch_bounds__(NT, LuB<NT>::MINB) lu_batched_f64_kernel(Batch
   double* rowj = srow + 2 * LW;            // [2][LW] row j
   double* sx = rowj + 2 * LW;              // [LMAXRHS][LW]
   RHdr* hdr = reinterpret_cast<RHdr*>(sx + LMAXRHS * LW);  // [2][NW]
-  __shared__ int s_next, s_r[LW], s_tgt[LW], s_row[2 * LW], s_src[2 * LW], s_list[2 * LW], s_nlist;
+  __shared__ int s_next, s_r[LW], s_nlist;
+  __shared__ int2 s_list[2 * LW];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   double* W = ws + (size_t)blockIdx.x * ws_stride;
   for (;;) {
@@ -190,59 +198,71 @@ __global__ void __launch_bounds__(NT, LuB<NT>::MINB) lu_batched_f64_kernel(Batch
         }
         rleaf_column_at<LW, 1>(j, rv, tid, 0, rows, r, u, oldj, 1.0 / piv, bv, bi, bk);
       }
-      if (tid < rows) {
-        double* p = W + (long)(j0 + tid) * ldw + j0;
 #pragma unroll
-        for (int q = 0; q < LW; q += 2) *reinterpret_cast<double2*>(p + q) = make_double2(rv[0][q], rv[0][q + 1]);
+      for (int q = 0; q < LW; q += 2)
+        *reinterpret_cast<double2*>(sL + tid * LSL + q) = make_double2(rv[0][q], rv[0][q + 1]);
+      __syncthreads();
+      // the panel's rows (multipliers and U) back to the copy, whole rows at a
+      // time
+      for (int e = tid; e < rows * (LW / 2); e += NT) {
+        const int r = e / (LW / 2), q = 2 * (e % (LW / 2));
+        *reinterpret_cast<double2*>(W + (long)(j0 + r) * ldw + j0 + q) = *reinterpret_cast<const double2*>(sL + r * LSL + q);
       }
-      // ---- the interchanges on the other columns: composition of the w
-      // swaps over the w panel rows (slots 0..) and the far targets (slots
-      // LW + first swap with it)
-      __syncthreads();
-      for (int q = tid; q < 2 * LW; q += NT) s_row[q] = q < w ? q : -1;
-      __syncthreads();
-      if (tid < w) {
-        const int t = s_r[tid];
-        int slot = t;
-        if (t >= w) {
-          int first = tid;
-          for (int i2 = tid - 1; i2 >= 0; --i2) first = s_r[i2] == t ? i2 : first;
-          slot = LW + first;
-          if (first == tid) s_row[slot] = t;
-        }
-        s_tgt[tid] = slot;
-      }
-      __syncthreads();
-      if (tid == 0) {
-        for (int q = 0; q < 2 * LW; ++q) s_src[q] = q;
+      // ---- the interchanges on the other columns.  Warp 0 composes the w swaps
+      // over 2 LW slots: the panel's first rows (slot = row) and the far rows
+      // (slot LW + first swap with it); lane l holds the labels of slots l and
+      // LW + l, and the slots whose row changes form the list (row, source).
+      if (warp == 0) {
+        const int t = lane < w ? s_r[lane] : lane;
+        const unsigned same = __match_any_sync(0xffffffffu, t);
+        const int first = __ffs(same) - 1;
+        const int tgt = t < LW ? t : LW + first;         // slot of row t (rows w.. of a short panel: themselves)
+        const int row1 = t >= LW && first == lane ? t : -1;  // row of slot LW + lane
+        int d0 = lane, d1 = LW + lane;
         for (int i = 0; i < w; ++i) {
-          const int b = s_tgt[i], x = s_src[i];
-          s_src[i] = s_src[b];
-          s_src[b] = x;
+          const int b = __shfl_sync(0xffffffffu, tgt, i);
+          const int x = __shfl_sync(0xffffffffu, d0, i);
+          const int y0 = __shfl_sync(0xffffffffu, d0, b & 31), y1 = __shfl_sync(0xffffffffu, d1, b & 31);
+          const int y = b < LW ? y0 : y1;
+          if (lane == i) d0 = y;
+          if (lane == (b & 31)) { if (b < LW) d0 = x; else d1 = x; }
         }
-        int m = 0;
-        for (int q = 0; q < 2 * LW; ++q)
-          if (s_row[q] >= 0 && s_src[q] != q) s_list[m++] = q;
-        s_nlist = m;
+        // labels are slots: the row that a slot's content comes from
+        auto row_of = [&](int slot) {
+          const int far = __shfl_sync(0xffffffffu, row1, slot & 31);
+          return slot < LW ? slot : far;
+        };
+        const int src0 = row_of(d0), src1 = row_of(d1);
+        const unsigned m0 = __ballot_sync(0xffffffffu, d0 != lane);
+        const unsigned m1 = __ballot_sync(0xffffffffu, row1 >= 0 && d1 != LW + lane);
+        const unsigned below = (1u << lane) - 1u;
+        if (d0 != lane) s_list[__popc(m0 & below)] = make_int2(lane, src0);
+        if (row1 >= 0 && d1 != LW + lane) s_list[__popc(m0) + __popc(m1 & below)] = make_int2(row1, src1);
+        if (lane == 0) s_nlist = __popc(m0) + __popc(m1);
       }
       __syncthreads();
-      const int m = s_nlist, tot2 = (ncol - LW) / 2;  // other columns, in pairs
+      const int m = s_nlist, tot2 = (ncol - LW) / 2;  // changed rows; other columns, in pairs
       if (m > 0) {
-        const int cap2 = S::BIG / 2 / m;  // column pairs per pass
+        // whole rows through the (free) U12 buffer, one warp per row
+        const int cap2 = LW * LDU / 2 / m;  // column pairs per pass
         for (int c2 = 0; c2 < tot2; c2 += cap2) {
           const int k2 = min(cap2, tot2 - c2);
-          for (int e = tid; e < m * k2; e += NT) {
-            const int l = e / k2, c = 2 * (c2 + e % k2);
-            const int src = s_row[s_src[s_list[l]]];
-            reinterpret_cast<double2*>(big)[e] =
-                *reinterpret_cast<const double2*>(W + (long)(j0 + src) * ldw + (c < j0 ? c : c + LW));
+          for (int l = warp; l < m; l += NW) {
+            const double* p = W + (long)(j0 + s_list[l].y) * ldw;
+#pragma unroll 4
+            for (int k = lane; k < k2; k += 32) {
+              const int c = 2 * (c2 + k);
+              reinterpret_cast<double2*>(sU)[l * k2 + k] = *reinterpret_cast<const double2*>(p + (c < j0 ? c : c + LW));
+            }
           }
           __syncthreads();
-          for (int e = tid; e < m * k2; e += NT) {
-            const int l = e / k2, c = 2 * (c2 + e % k2);
-            const int dst = s_row[s_list[l]];
-            *reinterpret_cast<double2*>(W + (long)(j0 + dst) * ldw + (c < j0 ? c : c + LW)) =
-                reinterpret_cast<double2*>(big)[e];
+          for (int l = warp; l < m; l += NW) {
+            double* p = W + (long)(j0 + s_list[l].x) * ldw;
+#pragma unroll 4
+            for (int k = lane; k < k2; k += 32) {
+              const int c = 2 * (c2 + k);
+              *reinterpret_cast<double2*>(p + (c < j0 ? c : c + LW)) = reinterpret_cast<double2*>(sU)[l * k2 + k];
+            }
           }
           __syncthreads();
         }
@@ -250,10 +270,6 @@ __global__ void __launch_bounds__(NT, LuB<NT>::MINB) lu_batched_f64_kernel(Batch
       const int ct = ncol - j0 - LW;  // trailing columns (a multiple of 8)
       if (ct <= 0) continue;
       // ---- U12: one thread per column
-#pragma unroll
-      for (int q = 0; q < LW; q += 2)
-        *reinterpret_cast<double2*>(sL + tid * LSL + q) = make_double2(rv[0][q], rv[0][q + 1]);
-      __syncthreads();
       if (tid < ct) {
         double* p = W + (long)j0 * ldw + j0 + LW + tid;
         double x[LW];
@@ -340,6 +356,18 @@ __global__ void __launch_bounds__(NT, LuB<NT>::MINB) lu_batched_f64_kernel(Batch
       for (int b0 = (n - 1) / LW * LW; b0 >= 0; b0 -= LW) {
         const int w = min(LW, n - b0);
         __syncthreads();
+        // this thread's row above the block (b0 <= NT): in flight during the
+        // block's own solve
+        double u[LW];
+        {
+          const double* p = W + (long)tid * ldw + b0;
+#pragma unroll
+          for (int s = 0; s < LW; s += 2) {
+            const double2 x = tid < b0 ? *reinterpret_cast<const double2*>(p + s) : make_double2(0.0, 0.0);
+            u[s] = x.x;
+            u[s + 1] = x.y;
+          }
+        }
         for (int e = tid; e < LW * LW; e += NT) {
           const int r = e / LW, c = e % LW;
           sD[r * 33 + c] = r < w && c < w ? W[(long)(b0 + r) * ldw + b0 + c] : (r == c ? 1.0 : 0.0);
@@ -357,23 +385,15 @@ __global__ void __launch_bounds__(NT, LuB<NT>::MINB) lu_batched_f64_kernel(Batch
           if (lane < w) a.B[mi][(long)(b0 + lane) + (long)q * a.ldb[mi]] = y;
         }
         __syncthreads();
-        for (int r = tid; r < b0; r += NT) {
-          const double* p = W + (long)r * ldw + b0;
-          double u[LW];
-#pragma unroll
-          for (int s = 0; s < LW; s += 2) {
-            const double2 v = *reinterpret_cast<const double2*>(p + s);
-            u[s] = v.x;
-            u[s + 1] = v.y;
-          }
+        if (tid < b0) {
           for (int q = 0; q < nrhs; ++q) {
-            double y0 = W[(long)r * ldw + n32 + q], y1 = 0.0;
+            double y0 = W[(long)tid * ldw + n32 + q], y1 = 0.0;
 #pragma unroll
             for (int s = 0; s < LW; s += 2) {  // entries past w meet zeros of the copy
               y0 = fma(-u[s], sx[q * LW + s], y0);
               y1 = fma(-u[s + 1], sx[q * LW + s + 1], y1);
             }
-            W[(long)r * ldw + n32 + q] = y0 + y1;
+            W[(long)tid * ldw + n32 + q] = y0 + y1;
           }
         }
       }
