@@ -167,15 +167,11 @@ __device__ __forceinline__ uint32_t mapa_shared(uint32_t addr, uint32_t rank) {
   return r;
 }
 
-__device__ __forceinline__ void st_async_f64(uint32_t raddr, double v, uint32_t rbar) {
-  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(raddr),
-               "l"(__double_as_longlong(v)), "r"(rbar)
-               : "memory");
-}
-
-__device__ __forceinline__ void st_async_b32(uint32_t raddr, uint32_t v, uint32_t rbar) {
-  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(raddr), "r"(v),
-               "r"(rbar)
+// 16 bytes (16-byte aligned) into a cluster peer's shared memory, completing
+// them on the peer's mbarrier rbar (both addresses from mapa).
+__device__ __forceinline__ void st_async16(uint32_t raddr, uint4 v, uint32_t rbar) {
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(raddr),
+               "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w), "r"(rbar)
                : "memory");
 }
 
@@ -185,22 +181,6 @@ __device__ __forceinline__ void st_async_b32(uint32_t raddr, uint32_t v, uint32_
 __device__ __forceinline__ void bulk_copy_g2s(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
                "l"(src), "r"(bytes), "r"(bar)
-               : "memory");
-}
-
-// Orders this thread's generic-proxy writes to shared memory before later
-// async-proxy reads of them (a bulk copy issued after a CTA barrier).
-__device__ __forceinline__ void fence_proxy_async_smem() {
-  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-}
-
-// Bulk copy of `bytes` (a multiple of 16; both addresses 16-byte aligned)
-// from this CTA's shared memory to a cluster peer's (rdst, from mapa),
-// completing the bytes on the peer's mbarrier rbar.  No multicast.
-__device__ __forceinline__ void bulk_copy_to_peer(uint32_t rdst, uint32_t src, uint32_t bytes, uint32_t rbar) {
-  asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                   rdst),
-               "r"(src), "r"(bytes), "r"(rbar)
                : "memory");
 }
 

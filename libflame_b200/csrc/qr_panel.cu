@@ -24,8 +24,8 @@
 //      the owner of row j publishes row j;
 //   2. one CTA barrier; the CTA's partial vector is the fixed-order sum of
 //      the 16 warp slots (its entry q = j is ||x2||^2);
-//   3. (clusters only) warp 0 bulk-copies the CTA's partial vector, and
-//      CTA 0 row j, into every other CTA's shared memory; every warp waits
+//   3. (clusters only) warp 0 stores the CTA's partial vector, and CTA 0 row j,
+//      into every other CTA's shared memory (st.async); every warp waits
 //      for the column's bytes on the CTA's mbarrier; every lane sums the C
 //      partial vectors in the same order, so every CTA holds the same bits;
 //   4. every lane forms alpha, tau and the scale 1 / (chi1 - alpha); since
@@ -35,7 +35,8 @@
 //      a_q -= x (scale w_q) (row j: a_q -= w_q).  CTA 0 writes column j of T.
 // Bound by the latency of that chain: an 8192 x 32 leaf 151 us with two CTA
 // barriers per column, serial sums and two square roots and two divisions in
-// a row, 128 us in this form (a 12288 x 16 one 86 -> 70 us).
+// a row, 119 us in this form (a 12288 x 16 one 86 -> 67 us; with bulk copies
+// instead of st.async 128 and 70).
 // One exchange per column where the reference's order needs two reductions
 // (the norm, then the dot products): the sums are the same up to the
 // rounding of scaling before or after the summation.
@@ -163,7 +164,6 @@ __global__ void __launch_bounds__(QL_THREADS, 1) qr_leaf_kernel(QrLeafArgs a) {
         for (int i = 1; i < 32; ++i)
           if (i == ij) r = v[i];
         rowj[par * W + q] = r;
-        if (C > 1) fence_proxy_async_smem();
       }
       __syncwarp();
       double d0 = 0.0, d1 = 0.0, d2 = 0.0, d3 = 0.0;  // four chains: FP64 FMA latency
@@ -201,14 +201,17 @@ __global__ void __launch_bounds__(QL_THREADS, 1) qr_leaf_kernel(QrLeafArgs a) {
       double* own = cslot + ((size_t)par * C + c) * W;
       if (warp == 0) {
         if (g == 0) own[q] = cs;
-        fence_proxy_async_smem();
         __syncwarp();
-        if (lane < C && lane != c) {
-          const uint32_t rbar = mapa_shared(fullp, (uint32_t)lane);
-          bulk_copy_to_peer(mapa_shared(smem_u32(own), (uint32_t)lane), smem_u32(own), (uint32_t)(8 * W), rbar);
-          if (c == 0)
-            bulk_copy_to_peer(mapa_shared(smem_u32(rowj + par * W), (uint32_t)lane), smem_u32(rowj + par * W),
-                              (uint32_t)(8 * W), rbar);
+        // 16 bytes per lane, W / 2 lanes per peer
+        constexpr int LP = W / 2, PP = 32 / LP;
+        const int ch = lane % LP;
+        const uint4 mine = reinterpret_cast<const uint4*>(own)[ch];
+        const uint4 row = reinterpret_cast<const uint4*>(rowj + par * W)[ch];
+        for (int p = lane / LP; p < C; p += PP) {
+          if (p == c) continue;
+          const uint32_t rbar = mapa_shared(fullp, (uint32_t)p);
+          st_async16(mapa_shared(smem_u32(own), (uint32_t)p) + 16 * ch, mine, rbar);
+          if (c == 0) st_async16(mapa_shared(smem_u32(rowj + par * W), (uint32_t)p) + 16 * ch, row, rbar);
         }
         // the arrive also publishes this CTA's own slot to its other warps
         if (lane == 0) mbar_arrive_expect_tx(fullp, (uint32_t)((C - 1) * 8 * W + (c == 0 ? 0 : 8 * W)));
