@@ -82,6 +82,7 @@ __device__ __forceinline__ void adj_xtz(const double* __restrict__ sX, const dou
 __global__ void __cluster_dims__(ADJ_CL, 1, 1) __launch_bounds__(ADJ_THREADS)
     chol_adj_diag_kernel(const double* __restrict__ L, const double* __restrict__ Dinv, double* Lb, long ld, int w,
                          const double* __restrict__ G, double* __restrict__ Sout, long lds) {
+  chain_begin();
   extern __shared__ double asm_[];
   double* sX = asm_;                        // lower triangular operand, zero above
   double* sD = sX + AB * ADJ_LD;            // 16 columns of D, later of M
@@ -190,6 +191,7 @@ __global__ void __cluster_dims__(ADJ_CL, 1, 1) __launch_bounds__(ADJ_THREADS)
   // release / acquire at cluster scope: Y is complete; it is also the last
   // access to a peer's shared memory, so a CTA may exit on its own after it
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  chain_next();
   adj_xtz(sX, sY, warp, lane, v1);  // S(:, J) = inv(D)^T Y(J, :)^T
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
@@ -252,7 +254,7 @@ size_t chol_adjoint_scratch(long n, int splits) {
 // the columns left of the next block run on `st`, one block behind, beside the
 // next block's chain.  sd == st: in stream order (the batched form, whose
 // matrices overlap one another).  n = 4096: 4.46 ms in stream order, 3.81
-// ms so.
+// ms so (3.41 with launch_chain).
 int chol_adjoint_dev(const double* L, double* Lb, long ld, long n, cudaStream_t st, cudaStream_t sd, double* scratch,
                      int splits) {
   if (n <= 0) return FLA_SUCCESS;
@@ -310,8 +312,9 @@ int chol_adjoint_dev(const double* L, double* Lb, long ld, long n, cudaStream_t 
         return FLA_FAILURE;
     }
     const int ps = prof_begin(sd);
-    chol_adj_diag_kernel<<<ADJ_CL, ADJ_THREADS, ADJ_SMEM, sd>>>(Lat(j0, j0), Dq, Bat(j0, j0), ld, w,
-                                                               m > 0 ? G : nullptr, W, ldw);
+    FB_LAUNCH(launch_chain(chol_adj_diag_kernel, dim3(ADJ_CL), dim3(ADJ_THREADS), ADJ_SMEM, sd,
+        Lat(j0, j0), Dq, Bat(j0, j0), ld, w,
+                                                               m > 0 ? G : nullptr, W, ldw));
     prof_end(ps, sd, PROF_DIAG, 2.0 * w * (double)w * w / 3.0);
     count_launch();
     FB_CK(cudaGetLastError());

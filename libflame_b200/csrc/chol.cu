@@ -85,6 +85,7 @@ __device__ __forceinline__ void syrk_tiles(double* S, int jb, int r_lo, int nti,
 
 __global__ void __launch_bounds__(POTRF_THREADS, 1) potrf_diag_kernel(double* A, long ld, int b, int gcol,
                                                                    int* info, int* err) {
+  chain_begin();
   extern __shared__ __align__(16) double S[];  // S[r + c*LDS]
   __shared__ int s_fail, s_cnt;
   __shared__ double s_rinv[2][IB];
@@ -119,6 +120,7 @@ __global__ void __launch_bounds__(POTRF_THREADS, 1) potrf_diag_kernel(double* A,
     if (r0 < b) syrk_tiles(S, jb, r0, (b8 - r0) / 8, r0, min(IB, b8 - r0) / 8, warp, POTRF_THREADS / 32, lane);
     __syncthreads();
   }
+  chain_next();
   // write back the lower triangle (the strictly upper part of A is untouched)
   for (int c = warp; c < b; c += POTRF_THREADS / 32)
     for (int r = c + lane; r < b; r += 32) A[r + (long)c * ld] = S[r + c * LDS];
@@ -194,7 +196,8 @@ int chol_lower_enqueue(DMat A, cudaStream_t st) {
   auto sub = [&](long k, cudaStream_t s) -> int {
     const int b = (int)std::min<long>(NB, n - k);
     int ps = prof_begin(s);
-    potrf_diag_kernel<<<1, POTRF_THREADS, POTRF_SMEM, s>>>(at(k, k), ld, b, (int)k, info, cx.d_status + ST_ERROR);
+    FB_LAUNCH(launch_chain(potrf_diag_kernel, dim3(1), dim3(POTRF_THREADS), POTRF_SMEM, s,
+        at(k, k), ld, b, (int)k, info, cx.d_status + ST_ERROR));
     prof_end(ps, s, PROF_DIAG, (double)b * b * b / 3.0);
     count_launch();
     FB_CK(cudaGetLastError());
@@ -252,8 +255,9 @@ int chol_lower_enqueue(DMat A, cudaStream_t st) {
 int potrf_diag_dev(double* A, long ld, int b, int gcol, cudaStream_t st) {
   set_attrs();
   int ps = prof_begin(st);
-  potrf_diag_kernel<<<1, POTRF_THREADS, POTRF_SMEM, st>>>(A, ld, b, gcol, ctx().d_status + ST_INFO,
-                                                            ctx().d_status + ST_ERROR);
+  FB_LAUNCH(launch_chain(potrf_diag_kernel, dim3(1), dim3(POTRF_THREADS), POTRF_SMEM, st,
+        A, ld, b, gcol, ctx().d_status + ST_INFO,
+                                                            ctx().d_status + ST_ERROR));
   prof_end(ps, st, PROF_DIAG, (double)b * b * b / 3.0);
   count_launch();
   FB_CK(cudaGetLastError());

@@ -64,6 +64,15 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int* er
   }
 }
 
+// Kernels launched by launch_chain: chain_begin() before anything of memory is
+// touched, in every block, also one with nothing to do (it waits until the
+// stream's previous kernel has completed and its writes are visible; the next
+// kernel relies on it for the kernels before this one); chain_next() once the
+// bulk of the work is done, which lets the next such kernel be placed: not
+// earlier, since its waiting blocks would keep SMs from the other stream.
+__device__ __forceinline__ void chain_begin() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // 2D tiled TMA load into shared memory, completion on an mbarrier.
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int x, int y,
                                             uint32_t bar) {

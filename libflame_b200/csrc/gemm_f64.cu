@@ -323,9 +323,7 @@ __global__ void __launch_bounds__(128) dgemm_small_kernel(const __grid_constant_
                                                           const int* guard, int guard_limit, int k_chunk,
                                                           long c_zstride) {
   extern __shared__ unsigned char smem_raw[];
-  if (guard && *((volatile const int*)guard) < guard_limit) return;
   const int tile_m = blockIdx.x * SM_T, tile_n = blockIdx.y * SM_T;
-  if (mode == GEMM_LOWER && (long)tile_m + SM_T - 1 - tile_n < diag_off) return;
   const uintptr_t base = (reinterpret_cast<uintptr_t>(smem_raw) + 2047) & ~uintptr_t(2047);
   unsigned char* sm = reinterpret_cast<unsigned char*>(base);
   const uint32_t sm_base = smem_u32(sm);
@@ -341,7 +339,12 @@ __global__ void __launch_bounds__(128) dgemm_small_kernel(const __grid_constant_
       mbar_init(empty0 + 8 * s, 4);
     }
     fence_barrier_init();
+    prefetch_tmap(&mapA);
+    prefetch_tmap(&mapB);
   }
+  chain_begin();  // nothing of memory is read before this
+  if (guard && *((volatile const int*)guard) < guard_limit) return;
+  if (mode == GEMM_LOWER && (long)tile_m + SM_T - 1 - tile_n < diag_off) return;
   __syncthreads();
   // stage: two 16-wide k halves, each A (32 x 16) then B; a half past the end
   // of k reads zeros (the map's fill), one inside another slice its values,
@@ -435,6 +438,7 @@ __global__ void __launch_bounds__(128) dgemm_small_kernel(const __grid_constant_
         mbar_wait(full0 + 8 * (kt % SM_STAGES), (kt / SM_STAGES) & 1, nullptr, 0);
     return;
   }
+  chain_next();
   // partial tiles through shared memory (every stage has been read): warp w's
   // at sC + w * 32 * LDC
   constexpr int LDC = SM_T + 2;
@@ -568,14 +572,16 @@ void launch_small(dim3 grid, cudaStream_t st, const CUtensorMap& mA, const CUten
     cudaFuncSetAttribute(dgemm_small_kernel<A_K, B_K>, cudaFuncAttributeMaxDynamicSharedMemorySize, SM_SMEM);
     done = true;
   }
-  dgemm_small_kernel<A_K, B_K><<<grid, 128, SM_SMEM, st>>>(mA, mB, C, ldc, (int)m, (int)n, (int)k, alpha, beta, mode,
-                                                           diag_off, err, guard, guard_limit, k_chunk, c_zstride);
+  FB_LAUNCH(launch_chain(dgemm_small_kernel<A_K, B_K>, dim3(grid), dim3(128), SM_SMEM, st,
+        mA, mB, C, ldc, (int)m, (int)n, (int)k, alpha, beta, mode,
+                                                           diag_off, err, guard, guard_limit, k_chunk, c_zstride));
 }
 
 // C := alpha * sum_z P_z + beta * C over the S partial products of a split-K
 // GEMM (P_z at P + z * zs, ld ldp), summed in z order (deterministic).
 __global__ void splitk_reduce_kernel(const double* __restrict__ P, long ldp, long zs, int S, int m, int n,
                                      double alpha, double beta, double* __restrict__ C, long ldc) {
+  chain_begin();
   const long total = (long)m * n;
   for (long e = blockIdx.x * (long)blockDim.x + threadIdx.x; e < total; e += (long)gridDim.x * blockDim.x) {
     const long i = e % m, j = e / m;
@@ -613,6 +619,7 @@ template <int D>
 __global__ void __launch_bounds__(256) gemm_tn_small_kernel(const double* __restrict__ A, long lda,
                                                             const double* __restrict__ B, long ldb, int m, int n,
                                                             long k, double* __restrict__ P) {
+  chain_begin();
   using T = TnSmall<D>;
   constexpr int KC = T::KC, LD = T::LD, NG = T::NG;
   extern __shared__ __align__(16) double tn_sm[];
@@ -656,6 +663,7 @@ __global__ void __launch_bounds__(256) gemm_tn_small_kernel(const double* __rest
     }
     __syncthreads();
   }
+  chain_next();
   // group sums: entry (i, j) of group grp at tn_sm[(grp D + j) (D + 1) + i]
 #pragma unroll
   for (int h = 0; h < 2; ++h)
@@ -680,6 +688,7 @@ __global__ void __launch_bounds__(256) gemm_tn_small_kernel(const double* __rest
 // a fixed shuffle tree (the same order on every run).
 __global__ void splitk_reduce_warp_kernel(const double* __restrict__ P, int S, int m, int n, double alpha,
                                           double beta, double* __restrict__ C, long ldc) {
+  chain_begin();
   const long e = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (e >= (long)m * n) return;
@@ -737,11 +746,14 @@ int gemm_tn_partials(cudaStream_t st, long m, long n, long k, const double* A, l
   }
   const int ps = prof_begin(st);
   if (D == 16)
-    gemm_tn_small_kernel<16><<<(unsigned)*S, 256, TnSmall<16>::SMEM, st>>>(A, lda, B, ldb, (int)m, (int)n, k, *P);
+    FB_LAUNCH(launch_chain(gemm_tn_small_kernel<16>, dim3((unsigned)*S), dim3(256), TnSmall<16>::SMEM, st,
+        A, lda, B, ldb, (int)m, (int)n, k, *P));
   else if (D == 32)
-    gemm_tn_small_kernel<32><<<(unsigned)*S, 256, TnSmall<32>::SMEM, st>>>(A, lda, B, ldb, (int)m, (int)n, k, *P);
+    FB_LAUNCH(launch_chain(gemm_tn_small_kernel<32>, dim3((unsigned)*S), dim3(256), TnSmall<32>::SMEM, st,
+        A, lda, B, ldb, (int)m, (int)n, k, *P));
   else
-    gemm_tn_small_kernel<64><<<(unsigned)*S, 256, TnSmall<64>::SMEM, st>>>(A, lda, B, ldb, (int)m, (int)n, k, *P);
+    FB_LAUNCH(launch_chain(gemm_tn_small_kernel<64>, dim3((unsigned)*S), dim3(256), TnSmall<64>::SMEM, st,
+        A, lda, B, ldb, (int)m, (int)n, k, *P));
   prof_end(ps, st, PROF_GEMM, 2.0 * (double)m * (double)n * (double)k);
   count_launch();
   FB_CK(cudaGetLastError());
@@ -769,8 +781,9 @@ int gemm_f64(cudaStream_t st, bool ta, bool tb, long m, long n, long k, double a
     double* Pz = nullptr;
     long S = 0;
     if (gemm_tn_partials(st, m, n, k, A, lda, B, ldb, &Pz, &S) != FLA_SUCCESS) return FLA_FAILURE;
-    splitk_reduce_warp_kernel<<<(unsigned)((m * n * 32 + 255) / 256), 256, 0, st>>>(Pz, (int)S, (int)m, (int)n,
-                                                                                   alpha, beta, C, ldc);
+    FB_LAUNCH(launch_chain(splitk_reduce_warp_kernel, dim3((unsigned)((m * n * 32 + 255) / 256)), dim3(256), 0, st,
+        Pz, (int)S, (int)m, (int)n,
+                                                                                   alpha, beta, C, ldc));
     count_launch();
     FB_CK(cudaGetLastError());
     return FLA_SUCCESS;
@@ -858,8 +871,8 @@ int gemm_f64(cudaStream_t st, bool ta, bool tb, long m, long n, long k, double a
   if (keep) *split->slices = S;
   if (S > 1 && !keep) {
     const long total = m * n;
-    splitk_reduce_kernel<<<(unsigned)std::min<long>(4L * sms, (total + 255) / 256), 256, 0, st>>>(
-        Pz, ldp, zs, (int)S, (int)m, (int)n, alpha, beta, C, ldc);
+    FB_LAUNCH(launch_chain(splitk_reduce_kernel, dim3((unsigned)std::min<long>(4L * sms, (total + 255) / 256)), dim3(256), 0, st,
+        Pz, ldp, zs, (int)S, (int)m, (int)n, alpha, beta, C, ldc));
     count_launch();
   }
   prof_end(pslot, st, PROF_GEMM,

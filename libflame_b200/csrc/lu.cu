@@ -240,6 +240,7 @@ __device__ void laswp_compose(const int* __restrict__ piv, int npiv, int reverse
 template <typename T, bool TR>
 __global__ void __launch_bounds__(256) laswp_apply_kernel(T* A, long ld, int row0, const int* __restrict__ piv,
                                                           int npiv, int reverse, int c0, int n0, int c1, int n1) {
+  chain_begin();
   __shared__ int s_piv[LASWP_MAXP];
   __shared__ int s_tgt[LASWP_MAXP];
   __shared__ int s_row[2 * LASWP_MAXP];
@@ -320,9 +321,11 @@ int laswp_blocked(T* A, long ld, int row0, const int* d_piv, int npiv, int c0, i
   const int ps = prof_begin(st);
   const unsigned grid = (unsigned)((ncols + LASWP_NC - 1) / LASWP_NC);
   if (tr)
-    laswp_apply_kernel<T, true><<<grid, 256, 0, st>>>(A, ld, row0, d_piv, npiv, reverse ? 1 : 0, c0, n0, c1, n1);
+    FB_LAUNCH(launch_chain(laswp_apply_kernel<T, true>, dim3(grid), dim3(256), 0, st,
+        A, ld, row0, d_piv, npiv, reverse ? 1 : 0, c0, n0, c1, n1));
   else
-    laswp_apply_kernel<T, false><<<grid, 256, 0, st>>>(A, ld, row0, d_piv, npiv, reverse ? 1 : 0, c0, n0, c1, n1);
+    FB_LAUNCH(launch_chain(laswp_apply_kernel<T, false>, dim3(grid), dim3(256), 0, st,
+        A, ld, row0, d_piv, npiv, reverse ? 1 : 0, c0, n0, c1, n1));
   prof_end(ps, st, PROF_SWAP, 0.0);
   count_launch();
   FB_CK(cudaGetLastError());

@@ -449,6 +449,7 @@ __device__ void rleaf_apply_pivots(const LeafArgs& a, const int* s_r, int c, int
 
 template <int W, int RPT>
 __global__ void __launch_bounds__(RLEAF_THREADS, 1) lu_leaf_reg_kernel(LeafArgs a) {
+  chain_begin();
   using Slot = RSlot<W>;
   extern __shared__ __align__(128) unsigned char rleaf_smem[];
   cg::cluster_group cluster = cg::this_cluster();
@@ -601,6 +602,7 @@ __global__ void __launch_bounds__(RLEAF_THREADS, 1) lu_leaf_reg_kernel(LeafArgs 
     // ---- 4. exchange, scale, update, next candidate
     rleaf_column_at<W, RPT>(j, rv, tid, r0, rows, r, u, oldj, 1.0 / piv, bv, bi, bk);
   }
+  chain_next();
   rleaf_store<W, RPT>(rv, a, r0, rows, tile, warp, lane);
   if (c == 0 && tid == 0 && first_null >= 0) atomicMin(a.info, a.gcol + first_null);
   if (done && a.pl + a.pr > 0) rleaf_apply_pivots<W>(a, s_r, c, C, reinterpret_cast<double*>(rleaf_smem + rleaf_tile_offset(W, C)));
@@ -715,7 +717,7 @@ int rleaf_launch(double* P, long ld, long M, int w, int* d_piv, int gcol, cudaSt
   la.pl = pl;
   la.pr = pr;
   cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = C;
   attr[0].val.clusterDim.y = 1;
@@ -725,7 +727,9 @@ int rleaf_launch(double* P, long ld, long M, int w, int* d_piv, int gcol, cudaSt
   cfg.dynamicSmemBytes = rleaf_smem_bytes(w, C);
   cfg.stream = st;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // see launch_chain
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.numAttrs = 2;
   const int ps = prof_begin(st);
   if (w == 8) FB_CK(cudaLaunchKernelEx(&cfg, lu_leaf_reg_kernel<8, 4>, la));
   else if (w == 16) FB_CK(cudaLaunchKernelEx(&cfg, lu_leaf_reg_kernel<16, 2>, la));

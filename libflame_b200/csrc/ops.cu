@@ -6,6 +6,7 @@
 #include <vector>
 
 #include "common.h"
+#include "dev_util.cuh"
 #include "mixed.h"
 
 namespace fb {
@@ -18,6 +19,7 @@ int laswp_dev(double* A, long ld, int row0, const int* d_piv, int npiv, int c0, 
 // triangle of dst (i <= j) is written.
 __global__ void transpose_kernel(const double* __restrict__ src, long lds, double* __restrict__ dst,
                                  long ldd, int m, int n, int tri) {
+  chain_begin();
   __shared__ double tile[32][33];
   const int bx = blockIdx.x * 32, by = blockIdx.y * 32;  // bx over src rows, by over src cols
   for (int j = threadIdx.y; j < 32; j += blockDim.y) {
@@ -35,7 +37,8 @@ int transpose_dev(const double* src, long lds, double* dst, long ldd, long m, lo
                   cudaStream_t st) {
   if (m <= 0 || n <= 0) return FLA_SUCCESS;
   dim3 grid((unsigned)((m + 31) / 32), (unsigned)((n + 31) / 32)), block(32, 8);
-  transpose_kernel<<<grid, block, 0, st>>>(src, lds, dst, ldd, (int)m, (int)n, upper_only ? 1 : 0);
+  FB_LAUNCH(launch_chain(transpose_kernel, dim3(grid), dim3(block), 0, st,
+        src, lds, dst, ldd, (int)m, (int)n, upper_only ? 1 : 0));
   count_launch();
   FB_CK(cudaGetLastError());
   return FLA_SUCCESS;

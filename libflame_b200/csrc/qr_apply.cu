@@ -19,7 +19,8 @@
 // Bound by the latency of that chain; before, each super-block had copies of
 // U and B, a Gram product with a 4-tile output, an inverse on one SM and a
 // reduction in it: m = 8192, k = 4096, 64 columns 2.88 ms,
-// now 1.56 ms (three launches of 8 to 16 us per super-block, 0.3 ms before).
+// now 1.38 ms (three launches of 8 to 16 us per super-block, 0.3 ms before
+// them).
 #include <algorithm>
 
 #include "common.h"
@@ -150,6 +151,7 @@ __global__ void __launch_bounds__(MID_THREADS) qr_apply_mid_kernel(const double*
                                                                    const double* __restrict__ P, long ldp, long zs,
                                                                    int nz, int transpose, double* B, long ldb, int nr,
                                                                    double* __restrict__ W2, long ldw) {
+  chain_begin();
   extern __shared__ __align__(16) double mid_sm[];
   double* sQ = mid_sm;                       // U1(i, j), i > j;  Ti(i, j), i <= j
   double* sB = sQ + AS * ALD;                // B1 columns
@@ -207,6 +209,7 @@ __global__ void __launch_bounds__(MID_THREADS) qr_apply_mid_kernel(const double*
     if (i < s && c < nc) W2[i + (long)(c0 + c) * ldw] = r[e];
   }
   __syncthreads();
+  chain_next();
   // U1 W2: U1(i, k), k < i, one at k = i
   mid_product([&](int k) { const int kk = k + t; return kk < i ? sQ[i + kk * ALD] : kk == i ? one : 0.0; }, zv, 0,
               i0 + 8, r);
@@ -283,9 +286,9 @@ int apply_q_blocks(DMat U, long k, DMat T, int b_alg, int S, DMat B, bool transp
     }
     ps = prof_begin(st);
     const long ldp = (s + 1) & ~1L;
-    qr_apply_mid_kernel<<<(unsigned)((nr + MID_COLS - 1) / MID_COLS), MID_THREADS, MID_SMEM, st>>>(
+    FB_LAUNCH(launch_chain(qr_apply_mid_kernel, dim3((unsigned)((nr + MID_COLS - 1) / MID_COLS)), dim3(MID_THREADS), MID_SMEM, st,
         Uq, U.ld, Ti + (size_t)q * S * S, S, s, h, P, ldp, ldp * nr, (int)slices, transpose_q ? 1 : 0, Bq, B.ld, (int)nr,
-        W2, ldw);
+        W2, ldw));
     prof_end(ps, st, PROF_TRSM, 3.0 * s * (double)s * nr);
     count_launch();
     FB_CK(cudaGetLastError());

@@ -93,6 +93,7 @@ __host__ __device__ inline size_t qleaf_smem_bytes(int W, int C) {
 
 template <int W>
 __global__ void __launch_bounds__(QL_THREADS, 1) qr_leaf_kernel(QrLeafArgs a) {
+  chain_begin();
   constexpr int G = 32 / W;   // row groups per warp
   constexpr int WR = 32 * G;  // rows per warp
   extern __shared__ __align__(128) unsigned char qleaf_smem[];
@@ -287,6 +288,7 @@ __global__ void __launch_bounds__(QL_THREADS, 1) qr_leaf_kernel(QrLeafArgs a) {
     }
     __syncwarp();  // xs is rewritten for the next column
   }
+  chain_next();
   // ---- store through the tile
   __syncwarp();
 #pragma unroll
@@ -380,7 +382,7 @@ int qleaf_launch(double* P, long ld, long M, int w, int W, double* T, long ldt, 
   la.ldu = ldu;
   la.err = ctx().d_status + ST_ERROR;
   cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = C;
   attr[0].val.clusterDim.y = 1;
@@ -390,7 +392,9 @@ int qleaf_launch(double* P, long ld, long M, int w, int W, double* T, long ldt, 
   cfg.dynamicSmemBytes = qleaf_smem_bytes(W, C);
   cfg.stream = st;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // see launch_chain
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.numAttrs = 2;
   const int ps = prof_begin(st);
   if (W == 8) FB_CK(cudaLaunchKernelEx(&cfg, qr_leaf_kernel<8>, la));
   else if (W == 16) FB_CK(cudaLaunchKernelEx(&cfg, qr_leaf_kernel<16>, la));
@@ -422,6 +426,7 @@ constexpr int RS_THREADS = 512, RS_COLS = 4;
 __global__ void __launch_bounds__(RS_THREADS) qr_reduce_solve_kernel(const double* __restrict__ P, int S, int w1,
                                                                      int w2, const double* __restrict__ T, long ldt,
                                                                      double* __restrict__ W, long ldw) {
+  chain_begin();
   __shared__ double sT[64 * 65];            // sT[j + i * 65] = T(j, i), j <= i
   __shared__ double sW[RS_THREADS];
   __shared__ double sr[64];
@@ -445,6 +450,7 @@ __global__ void __launch_bounds__(RS_THREADS) qr_reduce_solve_kernel(const doubl
   }
   sW[tid] = s;
   __syncthreads();
+  chain_next();
   if (warp < nc) {
     double r[2] = {0.0, 0.0};
 #pragma unroll
@@ -503,8 +509,8 @@ int panel_rec(double* P, long ld, long M, int w, double* Tb, long ldtb, double* 
       if (gemm_f64(st, true, false, w1, w2, M, 1.0, U, ldu, B, ld, 0.0, Pz, w1) != FLA_SUCCESS) return FLA_FAILURE;
     }
     const int ps = prof_begin(st);
-    qr_reduce_solve_kernel<<<(unsigned)((w2 + RS_COLS - 1) / RS_COLS), RS_THREADS, 0, st>>>(
-        Pz, (int)S, w1, w2, Tb, ldtb, W1, ldw);
+    FB_LAUNCH(launch_chain(qr_reduce_solve_kernel, dim3((unsigned)((w2 + RS_COLS - 1) / RS_COLS)), dim3(RS_THREADS), 0, st,
+        Pz, (int)S, w1, w2, Tb, ldtb, W1, ldw));
     prof_end(ps, st, PROF_TRSM, (double)w1 * w1 * w2);
     count_launch();
     FB_CK(cudaGetLastError());

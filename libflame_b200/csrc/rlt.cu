@@ -121,6 +121,7 @@ __device__ __forceinline__ void rlt_mul16(const double* Y, const double* Wm, dou
 template <int ROWS, bool UNIT, typename TX>
 __global__ void __launch_bounds__(R_THREADS) rlt_kernel(const double* __restrict__ Ls, long ld, TX* __restrict__ X,
                                                         long ldx, int b, long m, const int* guard, int guard_limit) {
+  chain_begin();
   constexpr int LDX = rlt_ldx<ROWS>();
   extern __shared__ __align__(16) double rlt_sm[];
   if (guard && *((volatile const int*)guard) < guard_limit) return;
@@ -207,6 +208,7 @@ __global__ void __launch_bounds__(R_THREADS) rlt_kernel(const double* __restrict
     rlt_update<ROWS>(sL, sX, kb, kb + RIB, (b8 - kb - RIB) / 8, warp, lane);
     __syncthreads();
   }
+  chain_next();
 #pragma unroll 4
   for (int e = tid; e < ROWS * b; e += R_THREADS) {
     const int r = e % ROWS, c = e / ROWS;
@@ -223,8 +225,8 @@ void rlt_launch(const double* L, long ld, TX* X, long ldx, int b, long m, const 
                          (int)rlt_smem<ROWS>(RB));
     attr = true;
   }
-  rlt_kernel<ROWS, UNIT, TX><<<(unsigned)((m + ROWS - 1) / ROWS), R_THREADS, rlt_smem<ROWS>(b), st>>>(
-      L, ld, X, ldx, b, m, guard, guard_limit);
+  FB_LAUNCH(launch_chain(rlt_kernel<ROWS, UNIT, TX>, dim3((unsigned)((m + ROWS - 1) / ROWS)), dim3(R_THREADS), rlt_smem<ROWS>(b), st,
+        L, ld, X, ldx, b, m, guard, guard_limit));
 }
 
 // Rows per CTA: the fewest that leave one wave (a 128-column triangle allows
