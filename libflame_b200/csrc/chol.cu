@@ -7,10 +7,10 @@
 //                               A22 -= A21 A21^T (lower) [DMMA GEMM engine]
 // with the next block column factored on a second stream while the rest of
 // the trailing update runs (chol_lower_enqueue).
-// The diagonal block is factored in shared memory in 32-column steps (the
-// reference's inner blocksize, FLA_Chol_cntl_init.c:23-61): a warp factors
-// each 32x32 block (the unblocked var2/var3 leaf), the rows below are solved
-// against it and the trailing part of the block is updated, all in SMEM.
+// The diagonal block is factored in shared memory in 8-column steps (the
+// reference's inner blocksize is 32, FLA_Chol_cntl_init.c:23-61): an 8 x 8
+// factor in registers, the rows below solved against it, the products with the
+// columns beyond.
 // A failing pivot (<= 0 or NaN, bl1_dsqrte in
 // src/base/flamec/blis/include/blis_macro_defs.h:134-136) records the
 // zero-based global column in the status block; every later kernel of the
@@ -28,67 +28,80 @@ namespace fb {
 namespace {
 
 constexpr int NB = 128;        // outer block
-constexpr int IB = CHOL_IB;    // inner block
 constexpr int LDS = NB + 4;    // SMEM leading dimension (= 4 mod 16: conflict-free DMMA fragments)
-constexpr int POTRF_THREADS = 256;
+constexpr int POTRF_THREADS = 512;
 constexpr int POTRF_SMEM = NB * LDS * 8;
+
 __device__ __forceinline__ bool guard_failed(const int* info) {
   return *((volatile const int*)info) != INT_MAX;
 }
 
 // Factor the b x b (b <= 128) lower-triangular diagonal block at A (ld) in
 // place.  gcol = global index of its first column for the info word.
-// Bound by the pivot chain of one warp: per column a reciprocal square root,
-// two products and a shuffle.  Everything else of a 32-column chunk runs
-// beside that chain:
-//   (a) warp 0 factors the 32 x 32 diagonal block, one row per lane in
-//       registers, and publishes each column in shared memory with a counter;
-//       warps 1-3 solve the rows below (one row per thread in registers,
-//       X := X inv(L11)^T, dtrsm's R,L,T,N order), one column behind warp 0;
-//       warps 4-7 subtract the previous chunk's products from the columns
-//       beyond this chunk;
-//   (b) all warps subtract this chunk's products from the next 32 columns.
-// The products run on the FP64 tensor cores.  The pivot chain carries register
-// values only: the next pivot is formed by its own lane from its own
-// multiplier (fma(-l, l, a)) and shuffled; each pivot's reciprocal square root
-// is one rsqrt, its square root d * rsqrt(d).
-// Measured (128 x 128): 40 us with the solve and the products between the
-// chunks' chains, 27 us in this form.
+// Bound by the pivot chain, so as little as possible hangs on it.  Steps of
+// eight columns; threads 0..127 own one row each:
+//   (a) every warp with rows reads the 8 x 8 diagonal block and factors it
+//       redundantly in registers (chol8: no exchange inside the chain, per
+//       column a reciprocal square root, a product and a fused multiply-add),
+//       then solves its own rows against it (dtrsm's R,L,T,N order); rows of
+//       the block itself come out of the same formulas;
+//       meanwhile the other warps subtract the previous step's products from the
+//       columns beyond this step on the FP64 tensor cores;
+//   (b) the rows lose this step's products in the next step's eight columns.
+// Measured, one call of FLA_Chol between events (about 6 us without a kernel):
+// n = 100 30.7 -> 26.2 us, n = 128 32.2 -> 30.6 us against 32-column blocks
+// factored by one warp (lane = row, the column through shared memory, about
+// 370 cycles a column); with four instead of twelve warps for the products
+// n = 128 took 32.4 us.
 __device__ __forceinline__ void cp_async8(double* dst, const double* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
 }
 
-// S(r, c) -= sum_{k < IB} S(r, jb + k) S(c, jb + k) for 8 x 8 tiles: rows
-// r_lo + 8 i, columns c_lo + 8 j (i < nti, j < ntj), tiles on or below the
-// diagonal only (r_lo, c_lo multiples of 8), dealt to the warps w, w + nw, ...
-// Entries above the diagonal of a diagonal tile are written too: nothing
-// reads them.
-__device__ __forceinline__ void syrk_tiles(double* S, int jb, int r_lo, int nti, int c_lo, int ntj, int w, int nw,
-                                           int lane) {
+// S(r, c) -= sum_{k < 8} S(r, jb + k) S(c, jb + k) for 8 x 8 tiles: rows and
+// columns from lo (a multiple of 8) to b8, tiles on or below the diagonal;
+// warp w of nw takes the column tiles w, w + nw, ..., four row tiles at a time
+// in flight.  Entries above the diagonal of a diagonal tile are written too:
+// nothing reads them.
+__device__ __forceinline__ void syrk8_tiles(double* S, int jb, int lo, int b8, int w, int nw, int lane) {
   const int g = lane >> 2, t = lane & 3;
-  for (int e = w; e < nti * ntj; e += nw) {
-    const int r = r_lo + 8 * (e % nti), c = c_lo + 8 * (e / nti);
-    if (r < c) continue;
-    const double* pa = S + r + g + (jb + t) * LDS;
+  for (int c = lo + 8 * w; c < b8; c += 8 * nw) {
     const double* pb = S + c + g + (jb + t) * LDS;
-    double d0[2] = {0.0, 0.0}, d1[2] = {0.0, 0.0};
+    const double b0 = pb[0], b1 = pb[4 * LDS];
+    for (int r = c; r < b8; r += 32) {
+      double a0[4], a1[4], o0[4], o1[4], d0[4], d1[4];
 #pragma unroll
-    for (int k = 0; k < IB; k += 8) {
-      dmma_884(d0[0], d0[1], pa[k * LDS], pb[k * LDS]);
-      dmma_884(d1[0], d1[1], pa[(k + 4) * LDS], pb[(k + 4) * LDS]);
+      for (int u = 0; u < 4; ++u) {
+        const int ru = min(r + 8 * u, b8 - 8);
+        const double* pa = S + ru + g + (jb + t) * LDS;
+        const double* o = S + ru + g + (c + 2 * t) * LDS;
+        a0[u] = pa[0];
+        a1[u] = pa[4 * LDS];
+        o0[u] = o[0];
+        o1[u] = o[LDS];
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        d0[u] = d1[u] = 0.0;
+        dmma_884(d0[u], d1[u], a0[u], b0);
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) dmma_884(d0[u], d1[u], a1[u], b1);
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (r + 8 * u < b8) {
+          double* o = S + r + 8 * u + g + (c + 2 * t) * LDS;
+          o[0] = o0[u] - d0[u];
+          o[LDS] = o1[u] - d1[u];
+        }
     }
-    double* o = S + r + g + (c + 2 * t) * LDS;
-    o[0] -= d0[0] + d1[0];
-    o[LDS] -= d0[1] + d1[1];
   }
 }
 
 __global__ void __launch_bounds__(POTRF_THREADS, 1) potrf_diag_kernel(double* A, long ld, int b, int gcol,
-                                                                   int* info, int* err) {
+                                                                   int* info) {
   chain_begin();
   extern __shared__ __align__(16) double S[];  // S[r + c*LDS]
-  __shared__ int s_fail, s_cnt;
-  __shared__ double s_rinv[2][IB];
+  __shared__ int s_fail;
   if (guard_failed(info)) return;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   // load the lower triangle (and diagonal) with asynchronous copies, all in
@@ -96,29 +109,50 @@ __global__ void __launch_bounds__(POTRF_THREADS, 1) potrf_diag_kernel(double* A,
   for (int c = warp; c < b; c += POTRF_THREADS / 32)
     for (int r = c + lane; r < b; r += 32) cp_async8(S + r + c * LDS, A + r + (long)c * ld);
   asm volatile("cp.async.wait_all;" ::: "memory");
-  if (tid == 0) {
-    s_fail = -1;
-    s_cnt = 0;
-  }
+  if (tid == 0) s_fail = -1;
   __syncthreads();
   const int b8 = (b + 7) & ~7;
-  for (int jb = 0; jb < b; jb += IB) {
-    const int w = min(IB, b - jb), r0 = jb + w;  // r0: first row below the block
-    // (a); the counter runs on over the chunks (base jb), s_rinv alternates
-    double* rinv = s_rinv[(jb / IB) & 1];
-    if (warp == 0) {
-      potrf_diag32<LDS>(S, jb, w, lane, rinv, &s_cnt, jb, &s_fail);
-    } else if (warp < 4) {
-      const int r = r0 + (warp - 1) * 32 + lane;
-      if (r < b) potrf_row<LDS>(S, jb, r, rinv, &s_cnt, jb, err);
-    } else if (jb > 0 && r0 < b) {
-      syrk_tiles(S, jb - IB, r0, (b8 - r0) / 8, r0, (b8 - r0) / 8, warp - 4, 4, lane);
+#pragma unroll 1
+  for (int jb = 0; jb < b; jb += 8) {
+    double x[8];
+    const bool own = warp < 4 && tid >= jb && tid < b8;  // this thread's row takes part
+    if (warp < 4) {
+      if ((warp << 5) + 31 >= jb) {  // (a) (warps whose rows are all done skip it)
+        double l[36], ri[8];
+        const int fail = chol8_load_factor(S + jb + jb * LDS, LDS, l, ri);
+        if (tid == jb && fail >= 0 && jb + fail < b) s_fail = jb + fail;  // rows past b: not pivots
+        if (own) {
+#pragma unroll
+          for (int k = 0; k < 8; ++k) x[k] = S[tid + (jb + k) * LDS];
+          chol8_solve(l, ri, x);
+#pragma unroll
+          for (int k = 0; k < 8; ++k) S[tid + (jb + k) * LDS] = x[k];
+        }
+      }
+    } else if (jb > 0 && jb + 8 < b8) {
+      syrk8_tiles(S, jb - 8, jb + 8, b8, warp - 4, POTRF_THREADS / 32 - 4, lane);
     }
     __syncthreads();
     if (s_fail >= 0) break;
-    // (b) the next chunk's columns
-    if (r0 < b) syrk_tiles(S, jb, r0, (b8 - r0) / 8, r0, min(IB, b8 - r0) / 8, warp, POTRF_THREADS / 32, lane);
-    __syncthreads();
+    if (warp < 4) {  // (b)
+      if (own && tid >= jb + 8) {
+        const double* row = S + jb + 8 + jb * LDS;  // rows jb + 8 .., this step's columns
+        double y[8];
+#pragma unroll
+        for (int c = 0; c < 8; ++c) y[c] = S[tid + (jb + 8 + c) * LDS];
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+#pragma unroll
+          for (int c = 0; c < 8; c += 2) {
+            const double2 v = *reinterpret_cast<const double2*>(row + c + k * LDS);
+            y[c] = fma(-x[k], v.x, y[c]);
+            y[c + 1] = fma(-x[k], v.y, y[c + 1]);
+          }
+#pragma unroll
+        for (int c = 0; c < 8; ++c) S[tid + (jb + 8 + c) * LDS] = y[c];
+      }
+      asm volatile("bar.sync 1, 128;" ::: "memory");
+    }
   }
   chain_next();
   // write back the lower triangle (the strictly upper part of A is untouched)
@@ -197,7 +231,7 @@ int chol_lower_enqueue(DMat A, cudaStream_t st) {
     const int b = (int)std::min<long>(NB, n - k);
     int ps = prof_begin(s);
     FB_LAUNCH(launch_chain(potrf_diag_kernel, dim3(1), dim3(POTRF_THREADS), POTRF_SMEM, s,
-        at(k, k), ld, b, (int)k, info, cx.d_status + ST_ERROR));
+        at(k, k), ld, b, (int)k, info));
     prof_end(ps, s, PROF_DIAG, (double)b * b * b / 3.0);
     count_launch();
     FB_CK(cudaGetLastError());
@@ -256,8 +290,7 @@ int potrf_diag_dev(double* A, long ld, int b, int gcol, cudaStream_t st) {
   set_attrs();
   int ps = prof_begin(st);
   FB_LAUNCH(launch_chain(potrf_diag_kernel, dim3(1), dim3(POTRF_THREADS), POTRF_SMEM, st,
-        A, ld, b, gcol, ctx().d_status + ST_INFO,
-                                                            ctx().d_status + ST_ERROR));
+        A, ld, b, gcol, ctx().d_status + ST_INFO));
   prof_end(ps, st, PROF_DIAG, (double)b * b * b / 3.0);
   count_launch();
   FB_CK(cudaGetLastError());
