@@ -32,7 +32,7 @@ namespace fb {
 
 namespace {
 
-constexpr int CW_ = CHOL_IB;      // panel width
+constexpr int CW_ = 32;           // panel width
 constexpr int CRHS = 8;           // right-hand sides
 
 template <int NT>
@@ -40,12 +40,49 @@ struct ChB {
   static constexpr int NW = NT / 32;
   static constexpr int LD = NT + 20;        // rows of the panel: NT, the right-hand sides, a tile's rest; = 4 mod 16
   static constexpr int LDR = NT;            // right-hand side q at sR[q * LDR]
-  static constexpr size_t SMEM = sizeof(double) * ((size_t)LD * CW_ + (size_t)CRHS * LDR + 2 * CW_ + CRHS * CW_);
+  static constexpr size_t SMEM = sizeof(double) * ((size_t)LD * CW_ + (size_t)CRHS * LDR + CW_);
   static constexpr int MINB = NT == 256 ? 2 : 1;
 };
 
 __device__ __forceinline__ void cp_async8(double* dst, const double* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+
+// Entries s .. s + 7 of row r of the panel less the products of its columns
+// before s with the diagonal block's rows.
+template <int LD>
+__device__ __forceinline__ void row_minus(const double* P, int r, int s, double (&x)[8]) {
+#pragma unroll
+  for (int c = 0; c < 8; ++c) x[c] = P[r + (s + c) * LD];
+#pragma unroll 4
+  for (int k = 0; k < s; ++k) {
+    const double v = P[r + k * LD];
+#pragma unroll
+    for (int c = 0; c < 8; c += 2) {
+      const double2 b = *reinterpret_cast<const double2*>(P + s + c + k * LD);
+      x[c] = fma(-v, b.x, x[c]);
+      x[c + 1] = fma(-v, b.y, x[c + 1]);
+    }
+  }
+}
+
+// x := x inv(L)^T for the factored 8 x 8 block at column s, its reciprocal
+// pivots in rinv.
+template <int LD>
+__device__ __forceinline__ void row_solve(const double* P, int s, const double* rinv, double (&x)[8]) {
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    x[k] *= rinv[s + k];
+    const double* col = P + s + (s + k) * LD;
+#pragma unroll
+    for (int c = k + 1; c < 8; ++c) x[c] = fma(-x[k], col[c], x[c]);
+  }
+}
+
+template <int LD>
+__device__ __forceinline__ void store8(double* P, int r, int s, const double (&x)[8]) {
+#pragma unroll
+  for (int c = 0; c < 8; ++c) P[r + (s + c) * LD] = x[c];
 }
 
 template <int NT>
@@ -55,9 +92,8 @@ __global__ void __launch_bounds__(NT, ChB<NT>::MINB) chol_batched_f64_kernel(Bat
   extern __shared__ __align__(16) double chb_sm[];
   double* P = chb_sm;                      // panel: row r (from the panel's first), column c at P[r + c * LD]
   double* sR = P + (size_t)LD * CW_;       // right-hand sides
-  double* s_rinv = sR + CRHS * LDR;        // [2][32], by panel parity
-  double* sx = s_rinv + 2 * CW_;           // [CRHS][32]
-  __shared__ int s_next, s_fail, s_cnt;
+  double* rinv = sR + CRHS * LDR;          // [32] the panel's reciprocal pivots
+  __shared__ int s_next, s_fail;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int g = lane >> 2, t = lane & 3;
   for (;;) {
@@ -65,7 +101,6 @@ __global__ void __launch_bounds__(NT, ChB<NT>::MINB) chol_batched_f64_kernel(Bat
     if (tid == 0) {
       s_next = atomicAdd(a.counter, 1);
       s_fail = -1;
-      s_cnt = 0;
     }
     __syncthreads();
     if (s_next >= a.count) break;
@@ -83,6 +118,11 @@ __global__ void __launch_bounds__(NT, ChB<NT>::MINB) chol_batched_f64_kernel(Bat
       const int RB = max(R, CW_);  // panel rows RB ..: the right-hand sides (past the whole diagonal block)
       for (int c = warp; c < w; c += NW)
         for (int r = c + lane; r < R; r += 32) cp_async8(P + r + c * LD, G + (long)(j + r) + (long)(j + c) * ld);
+      if (w < CW_)  // the last panel: unit pivots past the matrix
+        for (int e = tid; e < CW_ * CW_; e += NT) {
+          const int r = e % CW_, c = e / CW_;
+          if (r >= w && r >= c) P[r + c * LD] = r == c ? 1.0 : 0.0;
+        }
       asm volatile("cp.async.wait_all;" ::: "memory");
       __syncthreads();  // (the first time: the right-hand sides too)
       for (int e = tid; e < nrhs * CW_; e += NT) {
@@ -90,13 +130,40 @@ __global__ void __launch_bounds__(NT, ChB<NT>::MINB) chol_batched_f64_kernel(Bat
         P[RB + q + c * LD] = c < w ? sR[j + c + q * LDR] : 0.0;
       }
       __syncthreads();
-      // ---- panel; the counter runs on over the panels
-      double* rinv = s_rinv + ((j / CW_) & 1) * CW_;
-      if (warp == 0) {
-        potrf_diag32<LD>(P, 0, w, lane, rinv, &s_cnt, j, &s_fail);
-      } else {
-        for (int r = CW_ + (warp - 1) * 32 + lane; r < RB + nrhs; r += (NW - 1) * 32)
-          potrf_row<LD>(P, 0, r, rinv, &s_cnt, j, a.err);
+      // ---- panel, eight columns a step: warp 0 factors the 8 x 8 block and
+      // solves the rest of the diagonal block's rows; the rows below follow
+      // after the barrier, beside its next step
+      const int row = CW_ + (warp - 1) * 32 + lane;
+      for (int s = 0; s < CW_; s += 8) {
+        double x[8];
+        if (warp == 0) {
+          row_minus<LD>(P, lane, s, x);
+          if (lane >= s) store8<LD>(P, lane, s, x);
+          __syncwarp();
+          double l[36], ri[8];
+          const int f = chol8_load_factor(P + s + s * LD, LD, l, ri);
+          chol8_solve(l, ri, x);
+          __syncwarp();
+          if (lane >= s) store8<LD>(P, lane, s, x);
+          if (lane == 0) {
+            if (f >= 0 && s + f < w && s_fail < 0) s_fail = s + f;
+#pragma unroll
+            for (int k = 0; k < 8; ++k) rinv[s + k] = ri[k];
+          }
+        } else if (row < RB + nrhs) {
+          row_minus<LD>(P, row, s, x);
+        }
+        __syncthreads();
+        if (warp != 0 && row < RB + nrhs) {
+          row_solve<LD>(P, s, rinv, x);
+          store8<LD>(P, row, s, x);
+          // at most eight rows, in the first panel of the largest orders
+          if (const int r2 = row + (NW - 1) * 32; r2 < RB + nrhs) {
+            row_minus<LD>(P, r2, s, x);
+            row_solve<LD>(P, s, rinv, x);
+            store8<LD>(P, r2, s, x);
+          }
+        }
       }
       __syncthreads();
       if (s_fail >= 0) {
@@ -115,61 +182,65 @@ __global__ void __launch_bounds__(NT, ChB<NT>::MINB) chol_batched_f64_kernel(Bat
       // diagonal, then one strip of the right-hand sides' rows
       const int R2 = R - CW_;
       const int tr = (R2 + 15) / 16, tc = (R2 + 31) / 32;
-      const int strips = nrhs > 0 ? tc : 0;
-      for (int e = warp; e < tr * tc + strips; e += NW) {
-        const bool rhs = e >= tr * tc;
-        const int r0 = rhs ? R2 : (e % tr) * 16, c0 = (rhs ? e - tr * tc : e / tr) * 32;
-        if (!rhs && r0 + 15 < c0) continue;
-        double d[2][4][2];
+      int c32 = 0, e = warp;  // tile e of column tile c32 (row tiles 2 c32 ..)
+      for (;; e += NW) {
+        while (c32 < tc && e >= tr - 2 * c32) e -= tr - 2 * c32++;
+        if (c32 == tc) break;
+        const int r0 = (2 * c32 + e) * 16, c0 = c32 * 32;
+        double* C = G + (long)(j + CW_) + (long)(j + CW_) * ld;
+        double v[2][4][2], d[2][4][2];  // the tile's entries arrive during the products
 #pragma unroll
         for (int i = 0; i < 2; ++i)
 #pragma unroll
-          for (int c = 0; c < 4; ++c) d[i][c][0] = d[i][c][1] = 0.0;
+          for (int c = 0; c < 4; ++c)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              const int rw = r0 + 8 * i + g, col = c0 + 8 * c + 2 * t + h;
+              v[i][c][h] = (rw < R2 && col <= rw) ? C[rw + (long)col * ld] : 0.0;
+              d[i][c][h] = 0.0;
+            }
+        // rows past the matrix: whatever P holds there, never stored
         const double* pa = P + CW_ + r0 + g + t * LD;
         const double* pb = P + CW_ + c0 + g + t * LD;
-        const bool two = !rhs;  // eight right-hand sides: one row tile
-#pragma unroll 4
+#pragma unroll
         for (int k = 0; k < CW_; k += 4) {
-          const double a0 = pa[k * LD], a1 = two ? pa[8 + k * LD] : 0.0;
+          const double a0 = pa[k * LD], a1 = pa[8 + k * LD];
 #pragma unroll
           for (int c = 0; c < 4; ++c) {
-            // column tiles past the matrix: any finite or garbage row of P, never stored
-            const double b = c0 + 8 * c < R2 ? pb[8 * c + k * LD] : 0.0;
+            const double b = pb[8 * c + k * LD];
             dmma_884(d[0][c][0], d[0][c][1], a0, b);
-            if (two) dmma_884(d[1][c][0], d[1][c][1], a1, b);
+            dmma_884(d[1][c][0], d[1][c][1], a1, b);
           }
         }
-        if (rhs) {
-          if (g < nrhs)
 #pragma unroll
-            for (int c = 0; c < 4; ++c)
+        for (int i = 0; i < 2; ++i)
 #pragma unroll
-              for (int h = 0; h < 2; ++h) {
-                const int col = c0 + 8 * c + 2 * t + h;
-                if (col < R2) sR[j + CW_ + col + g * LDR] -= d[0][c][h];
-              }
-        } else {
-          double* C = G + (long)(j + CW_) + (long)(j + CW_) * ld;
-          double v[2][4][2];
+          for (int c = 0; c < 4; ++c)
 #pragma unroll
-          for (int i = 0; i < 2; ++i)
+            for (int h = 0; h < 2; ++h) {
+              const int rw = r0 + 8 * i + g, col = c0 + 8 * c + 2 * t + h;
+              if (rw < R2 && col <= rw) C[rw + (long)col * ld] = v[i][c][h] - d[i][c][h];
+            }
+      }
+      // the right-hand sides' rows: one row tile
+      for (int c0 = e * 32; nrhs > 0 && c0 < R2; c0 += NW * 32) {
+        double d[4][2];
 #pragma unroll
-            for (int c = 0; c < 4; ++c)
+        for (int c = 0; c < 4; ++c) d[c][0] = d[c][1] = 0.0;
+        const double* pa = P + CW_ + R2 + g + t * LD;
+        const double* pb = P + CW_ + c0 + g + t * LD;
 #pragma unroll
-              for (int h = 0; h < 2; ++h) {
-                const int row = r0 + 8 * i + g, col = c0 + 8 * c + 2 * t + h;
-                v[i][c][h] = (row < R2 && col <= row) ? C[row + (long)col * ld] : 0.0;
-              }
+        for (int k = 0; k < CW_; k += 4)
 #pragma unroll
-          for (int i = 0; i < 2; ++i)
+          for (int c = 0; c < 4; ++c) dmma_884(d[c][0], d[c][1], pa[k * LD], pb[8 * c + k * LD]);
+        if (g < nrhs)
 #pragma unroll
-            for (int c = 0; c < 4; ++c)
+          for (int c = 0; c < 4; ++c)
 #pragma unroll
-              for (int h = 0; h < 2; ++h) {
-                const int row = r0 + 8 * i + g, col = c0 + 8 * c + 2 * t + h;
-                if (row < R2 && col <= row) C[row + (long)col * ld] = v[i][c][h] - d[i][c][h];
-              }
-        }
+            for (int h = 0; h < 2; ++h) {
+              const int col = c0 + 8 * c + 2 * t + h;
+              if (col < R2) sR[j + CW_ + col + g * LDR] -= d[c][h];
+            }
       }
       __syncthreads();  // the next panel reads the update; P is reused
     }
@@ -186,42 +257,80 @@ __global__ void __launch_bounds__(NT, ChB<NT>::MINB) chol_batched_f64_kernel(Bat
     }
     // ---- backward substitution L^T x = y
     if (nrhs > 0 && fail < 0) {
-      double* sD = P;  // diagonal block, sD[r + c * 33]
-      for (int b0 = (n - 1) / CW_ * CW_; b0 >= 0; b0 -= CW_) {
-        const int w = min(CW_, n - b0);
-        __syncthreads();
-        for (int e = tid; e < CW_ * CW_; e += NT) {
-          const int r = e % CW_, c = e / CW_;
-          sD[r + c * 33] = r < w && c <= r ? G[(long)(b0 + r) + (long)(b0 + c) * ld] : (r == c ? 1.0 : 0.0);
+      double* sD = P;                       // [2] diagonal blocks, L(r, c) at r + 33 c
+      double* sS = P + 2 * CW_ * (CW_ + 1);  // [NW / 4][CRHS][32] partial products
+      const int last = (n - 1) / CW_ * CW_;
+      __syncthreads();
+      for (int e = tid; e < CW_ * CW_; e += NT) {
+        const int r = e % CW_, c = e / CW_, w = n - last;
+        sD[r + c * 33] = r < w && c <= r ? G[(long)(last + r) + (long)(last + c) * ld] : (r == c ? 1.0 : 0.0);
+      }
+      for (int b0 = last, i = 0; b0 >= 0; b0 -= CW_, i ^= 1) {
+        if (b0 > 0)  // the next diagonal block
+          for (int e = tid; e < CW_ * CW_; e += NT) {
+            const int r = e % CW_, c = e / CW_;
+            if (c <= r)
+              cp_async8(sD + (i ^ 1) * CW_ * (CW_ + 1) + r + c * 33,
+                        G + (long)(b0 - CW_ + r) + (long)(b0 - CW_ + c) * ld);
+          }
+        // L(below, block)^T times the solved rows: warp & 3 takes eight of the
+        // columns, warp >> 2 a share of the rows
+        const int cg = 8 * (warp & 3), ks = warp >> 2;
+        if (b0 < last) {
+          double d0 = 0.0, d1 = 0.0;
+          const double* gb = G + (long)(b0 + cg + g) * ld + t;
+          const double* ra = sR + t + g * LDR;
+          for (int k = b0 + CW_ + 4 * ks; k < n; k += 8 * NW) {
+            double av[8], bv[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+              const int kk = k + u * NW;
+              const bool in = kk + t < n;
+              bv[u] = in ? gb[kk] : 0.0;
+              av[u] = in ? ra[kk] : 0.0;
+            }
+#pragma unroll
+            for (int u = 0; u < 8; ++u) dmma_884(d0, d1, av[u], bv[u]);
+          }
+          double* o = sS + (ks * CRHS + g) * CW_ + cg + 2 * t;
+          o[0] = d0;
+          o[1] = d1;
         }
+        asm volatile("cp.async.wait_all;" ::: "memory");
         __syncthreads();
+        const int w = min(CW_, n - b0);
+        const double* D = sD + i * CW_ * (CW_ + 1);
         for (int q = warp; q < nrhs; q += NW) {
           double y = lane < w ? sR[b0 + lane + q * LDR] : 0.0;
-          const double rv = 1.0 / sD[lane + lane * 33];
-          for (int s = w - 1; s >= 0; --s) {
-            const double x = __shfl_sync(0xffffffffu, y * rv, s);
-            if (lane == s) y = x;
-            else if (lane < s) y = fma(-sD[s + lane * 33], x, y);
+          if (b0 < last) {
+            double u = 0.0;
+#pragma unroll
+            for (int k = 0; k < NW / 4; ++k) u += sS[(k * CRHS + q) * CW_ + lane];
+            y -= u;
           }
-          sx[q * CW_ + lane] = y;
-          if (lane < w) a.B[mi][(long)(b0 + lane) + (long)q * a.ldb[mi]] = y;
+          const double rv = 1.0 / D[lane + lane * 33];
+          double sol = 0.0;
+#pragma unroll
+          for (int s = CW_ - 8; s >= 0; s -= 8) {  // eight entries in every lane, then the lane's own
+            double x[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) x[k] = __shfl_sync(0xffffffffu, y, s + k);
+#pragma unroll
+            for (int k = 7; k >= 0; --k) {
+              x[k] *= __shfl_sync(0xffffffffu, rv, s + k);
+#pragma unroll
+              for (int c = 0; c < k; ++c) x[c] = fma(-D[s + k + (s + c) * 33], x[k], x[c]);
+              if (lane == s + k) sol = x[k];
+            }
+#pragma unroll
+            for (int k = 7; k >= 0; --k) y = fma(-D[s + k + lane * 33], x[k], y);  // only lanes below s count
+          }
+          if (lane < w) {
+            sR[b0 + lane + q * LDR] = sol;
+            a.B[mi][(long)(b0 + lane) + (long)q * a.ldb[mi]] = sol;
+          }
         }
         __syncthreads();
-        for (int r = tid; r < b0; r += NT) {
-          const double* p = G + (long)b0 + (long)r * ld;
-          double u[CW_];
-#pragma unroll
-          for (int s = 0; s < CW_; ++s) u[s] = s < w ? p[s] : 0.0;
-          for (int q = 0; q < nrhs; ++q) {
-            double y0 = sR[r + q * LDR], y1 = 0.0;
-#pragma unroll
-            for (int s = 0; s < CW_; s += 2) {
-              y0 = fma(-u[s], sx[q * CW_ + s], y0);
-              y1 = fma(-u[s + 1], sx[q * CW_ + s + 1], y1);
-            }
-            sR[r + q * LDR] = y0 + y1;
-          }
-        }
       }
     }
   }
