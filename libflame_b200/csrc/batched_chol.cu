@@ -9,19 +9,25 @@
 //
 // Right-looking in panels of 32 columns, in place (the matrices of the
 // resident CTAs stay in L2):
-//   panel   the block column in shared memory; one warp factors its 32 x 32
-//           diagonal block and publishes each column, the other warps solve
-//           the rows below one column behind it (chol_leaf.cuh);
+//   panel   the block column in shared memory, eight columns a step: one warp
+//           factors the 8 x 8 block in registers and solves the diagonal
+//           block's rows, the other warps the rows below beside its next step;
 //   update  A22 -= L21 L21^T (lower) on the FP64 tensor cores, 16 x 32 warp
 //           tiles, both operands from the panel in shared memory.
 // The right-hand sides are rows below the matrix (kept in shared memory), so
-// the forward substitution comes with the factorization.  Bound by the pivot
-// chain of the panels (about 0.13 us a column) and, for the large orders, the
-// FP64 rate.  Orders up to 256 run in CTAs of 256 threads, two per SM, so that
-// one matrix's chain overlaps the other's updates; 257 to 512 in CTAs of 512.
+// the forward substitution comes with the factorization; the backward one
+// takes L(below, block)^T x on the tensor cores, block by block.  Bound by the
+// update's tiles for the large orders (n = 512: 39 of 66 thousand cycles a
+// panel, the FP64 tensor pipe 34 % and the L1 data path 66 % of their rates
+// over the whole kernel), the panels' pivot chain (8 thousand cycles a panel)
+// for the small ones.  Orders up to 256 run in CTAs of 256 threads, two per
+// SM, so that one matrix's chain overlaps the other's updates; 257 to 512 in
+// CTAs of 512.
 // Measured: 2500 matrices, n uniform in 8..512, 4 right-hand sides: 11.9 ms
 // left-looking with one CTA of 512 threads per SM (chol_batched_dmma_kernel,
-// which keeps the orders above 512), 4.5 ms in this form.
+// which keeps the orders above 512); 4.5 ms right-looking with panels factored
+// column by column and a row per thread in the backward substitution; 3.9 ms
+// in this form.
 #include <algorithm>
 
 #include "batched.h"
