@@ -6,7 +6,7 @@
 // (src/lapack/dec/lu/piv/vars/flamec/FLA_LU_piv_blk_var5.c:13-114):
 //   for each block of nb columns:
 //     [A11;A21], p1 := LU_piv([A11;A21])   lu_panel_factor (lu_panel.cu)
-//     pivot [A10;A20] and [A12;A22]         laswp_compose/apply kernels
+//     pivot [A10;A20] and [A12;A22]         laswp_apply_kernel
 //     A12 := inv(tril_unit(A11)) A12         forward substitution, one launch
 //                                            (rlt_kernel, rlt.cu)
 //     A22 -= A21 A12                         DMMA GEMM engine
@@ -197,14 +197,14 @@ __global__ void __launch_bounds__(PANEL_THREADS) lu_panel_kernel(PanelArgs a) {
 constexpr int LASWP_MAXP = 128;
 constexpr int LASWP_NC = 16;  // columns per CTA (static SMEM < 48 KB)
 
-// Composition of the interchange sequence into slot rows and sources, in
-// shared memory (every CTA of the apply kernel forms it itself: the sequence
-// has at most LASWP_MAXP entries, and a separate launch would cost more).
-__device__ void laswp_compose(const int* __restrict__ piv, int npiv, int reverse, int* s_piv, int* s_tgt,
-                              int* s_row, int* s_src) {
+// Slots of the interchange sequence, in shared memory: s_tgt[i] is the slot
+// that interchange i exchanges with slot i, s_row the row offset of each slot
+// (-1: not used).  Every CTA of the apply kernel forms them itself: the
+// sequence has at most LASWP_MAXP entries, and a separate launch would cost
+// more.
+__device__ void laswp_slots(const int* __restrict__ piv, int npiv, int* s_piv, int* s_tgt, int* s_row) {
   const int tid = threadIdx.x;
-  const int nslot = 2 * npiv;
-  for (int s = tid; s < nslot; s += blockDim.x) s_row[s] = (s < npiv) ? s : -1;
+  for (int s = tid; s < 2 * npiv; s += blockDim.x) s_row[s] = (s < npiv) ? s : -1;
   for (int i = tid; i < npiv; i += blockDim.x) s_piv[i] = piv[i];
   __syncthreads();
   for (int i = tid; i < npiv; i += blockDim.x) {
@@ -224,19 +224,24 @@ __device__ void laswp_compose(const int* __restrict__ piv, int npiv, int reverse
     s_tgt[i] = slot;
   }
   __syncthreads();
-  if (tid == 0) {
-    for (int s = 0; s < nslot; ++s) s_src[s] = s;
-    for (int q = 0; q < npiv; ++q) {
-      const int i = reverse ? npiv - 1 - q : q;
-      const int a = i, b = s_tgt[i];
-      const int x = s_src[a];
-      s_src[a] = s_src[b];
-      s_src[b] = x;
-    }
-  }
-  __syncthreads();
 }
 
+// Slot whose value the whole sequence leaves in slot s: the interchanges
+// undone from the last one.
+__device__ __forceinline__ int laswp_source(const int* s_tgt, int npiv, int reverse, int s) {
+#pragma unroll 8
+  for (int q = npiv - 1; q >= 0; --q) {
+    const int a = reverse ? npiv - 1 - q : q, b = s_tgt[a];
+    s = s == a ? b : (s == b ? a : s);
+  }
+  return s;
+}
+
+// Bound by latency: the scan for the slots, the trace of the sequence (one
+// thread per slot, npiv steps, while the values are on their way) and one
+// round trip of loads.  Measured (the whole FLA_LU_piv): n = 3001 6.90 ->
+// 6.47 ms, 16384 123.6 -> 120.3, against one thread that composed the sequence
+// and loads one after another.
 template <typename T, bool TR>
 __global__ void __launch_bounds__(256) laswp_apply_kernel(T* A, long ld, int row0, const int* __restrict__ piv,
                                                           int npiv, int reverse, int c0, int n0, int c1, int n1) {
@@ -247,19 +252,30 @@ __global__ void __launch_bounds__(256) laswp_apply_kernel(T* A, long ld, int row
   __shared__ int s_src[2 * LASWP_MAXP];
   __shared__ T s_val[LASWP_NC][2 * LASWP_MAXP + 1];
   const int tid = threadIdx.x;
-  laswp_compose(piv, npiv, reverse, s_piv, s_tgt, s_row, s_src);
+  laswp_slots(piv, npiv, s_piv, s_tgt, s_row);
   const int nslot = 2 * npiv;
   const int ncols = n0 + n1;
   const int cbase = blockIdx.x * LASWP_NC;
   // load: consecutive threads take consecutive slots of one column
   // (consecutive columns of one slot when TR)
-  for (int e = tid; e < LASWP_NC * nslot; e += blockDim.x) {
+  constexpr int NE = LASWP_NC * 2 * LASWP_MAXP / 256;  // per thread
+  T v[NE];
+#pragma unroll
+  for (int u = 0; u < NE; ++u) {
+    const int e = tid + 256 * u;
     const int cl = TR ? e % LASWP_NC : e / nslot, s = TR ? e / LASWP_NC : e % nslot;
     const int t = cbase + cl;
-    if (t >= ncols || s_row[s] < 0) continue;
+    if (e >= LASWP_NC * nslot || t >= ncols || s_row[s] < 0) continue;
     const long col = t < n0 ? c0 + t : c1 + (t - n0);
     const long row = (long)row0 + s_row[s];
-    s_val[cl][s] = TR ? A[col + row * ld] : A[row + col * ld];
+    v[u] = TR ? A[col + row * ld] : A[row + col * ld];
+  }
+  for (int s = tid; s < nslot; s += blockDim.x) s_src[s] = laswp_source(s_tgt, npiv, reverse, s);
+#pragma unroll
+  for (int u = 0; u < NE; ++u) {
+    const int e = tid + 256 * u;
+    const int cl = TR ? e % LASWP_NC : e / nslot, s = TR ? e / LASWP_NC : e % nslot;
+    if (e < LASWP_NC * nslot) s_val[cl][s] = v[u];
   }
   __syncthreads();
   for (int e = tid; e < LASWP_NC * nslot; e += blockDim.x) {
@@ -599,9 +615,8 @@ int lu_piv_dev(DMat A, int* d_piv, int* info) {
   const int NBL = (int)std::min<long>(lu_blocksize(), mn);
   // Width of the panel starting at column k: twice NBL while more than
   // wide_rows rows remain (the trailing updates dominate there, and K = 2 NBL
-  // halves each update tile's fixed cost), NBL after (the panels dominate;
-  // at n = 16384 that is the last ~8000 rows, and an n = 8192 factorization
-  // is panel-bound from the start).  FLA_B200_LU_WIDE_ROWS overrides it.
+  // halves each update tile's fixed cost), NBL after (the panels dominate).
+  // FLA_B200_LU_WIDE_ROWS overrides it.
   static const long wide_rows = [] {
     long v = 8192;
     if (const char* e = std::getenv("FLA_B200_LU_WIDE_ROWS")) v = std::atol(e);
