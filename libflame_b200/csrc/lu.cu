@@ -616,9 +616,11 @@ int lu_piv_dev(DMat A, int* d_piv, int* info) {
   // Width of the panel starting at column k: twice NBL while more than
   // wide_rows rows remain (the trailing updates dominate there, and K = 2 NBL
   // halves each update tile's fixed cost), NBL after (the panels dominate).
-  // FLA_B200_LU_WIDE_ROWS overrides it.
+  // n = 16384 / 8192 / 6144 with the line at 8192 rows: 120.3 / 25.3 / 15.47
+  // ms; at 6144: 119.3 / 24.6 / 15.45 (5120 gains no more at 16384 and costs
+  // 0.4 % at 6144).  FLA_B200_LU_WIDE_ROWS overrides it.
   static const long wide_rows = [] {
-    long v = 8192;
+    long v = 6144;
     if (const char* e = std::getenv("FLA_B200_LU_WIDE_ROWS")) v = std::atol(e);
     return v;
   }();
