@@ -391,9 +391,9 @@ __device__ __forceinline__ void rleaf_store(const double (&rv)[RPT][W], const Le
 // the leaf and pr right of it (FLA_Apply_pivots on A10/A12 of the panel
 // recursion, done here instead of by separate launches).  The interchanges
 // move at most 2W rows: the W leaf rows and the distinct far targets.  Their
-// composition (the row that ends in each slot) is formed once; each CTA of
-// the cluster then gathers its share of the columns for those rows into
-// shared memory and writes them back permuted.  The leaf's own columns are
+// composition (the row that ends in each slot, traced back by a thread per
+// slot) is formed once; each CTA of the cluster gathers its share of the
+// columns for those rows into shared memory and writes them back permuted.  The leaf's own columns are
 // not touched, so no CTA waits for another.
 template <int W>
 __device__ void rleaf_apply_pivots(const LeafArgs& a, const int* s_r, int c, int C, double* buf) {
@@ -402,30 +402,25 @@ __device__ void rleaf_apply_pivots(const LeafArgs& a, const int* s_r, int c, int
   __shared__ int s_src[2 * W];   // slot whose original row ends in this slot
   const int tid = threadIdx.x;
   __syncthreads();  // s_r complete
-  for (int q = tid; q < 2 * W; q += blockDim.x) s_row[q] = q < W ? q : -1;
-  __syncthreads();
   if (tid < W) {
     const int t = s_r[tid];
-    int slot = t;
-    if (t >= W) {  // far target: the first interchange with it owns the slot
-      int first = tid;
-      for (int i2 = tid - 1; i2 >= 0; --i2) first = s_r[i2] == t ? i2 : first;
-      slot = W + first;
-      if (first == tid) s_row[slot] = t;
-    }
-    s_tgt[tid] = slot;
+    int first = tid;  // far target: the first interchange with it owns the slot
+#pragma unroll
+    for (int i2 = W - 1; i2 >= 0; --i2) first = (i2 < tid && s_r[i2] == t) ? i2 : first;
+    s_tgt[tid] = t < W ? t : W + first;
+    s_row[tid] = tid;
+    s_row[W + tid] = t >= W && first == tid ? t : -1;
   }
   __syncthreads();
-  if (tid == 0) {
-    for (int q = 0; q < 2 * W; ++q) s_src[q] = q;
-    for (int i = 0; i < W; ++i) {
+  if (tid < 2 * W) {  // the interchanges undone from the last one
+    int q = tid;
+#pragma unroll
+    for (int i = W - 1; i >= 0; --i) {
       const int b = s_tgt[i];
-      const int x = s_src[i];
-      s_src[i] = s_src[b];
-      s_src[b] = x;
+      q = q == i ? b : (q == b ? i : q);
     }
+    s_src[tid] = q;
   }
-  __syncthreads();
   const int tot = a.pl + a.pr;
   const int per = (tot + C - 1) / C;
   const int cb = c * per, ce = min(tot, cb + per);
