@@ -66,31 +66,48 @@ __device__ __forceinline__ double rleaf_pick_col(const double (&row)[W], int j) 
   return v;
 }
 
-// Column J of the leaf for the calling thread's rows, J a compile-time
-// constant so every register of a row is addressed directly: exchange
-// rows j and r, scale column J below the pivot (reciprocal multiply, as
-// bl1_dinvscalv), rank-1 update, and the candidate for column J + 1.
-template <int W, int RPT, int J>
-__device__ __forceinline__ void rleaf_column(double (&rv)[RPT][W], int tid, int r0, int rows, int r,
-                                             const double* u, const double* oldj, double rinv, double& bv,
-                                             int& bi, int& bk) {
+// Rows j and r of the leaf exchanged: the owner of row j takes the pivot row
+// u, the owner of row r the old row j.
+template <int W, int RPT>
+__device__ __forceinline__ void rleaf_exchange(int j, double (&rv)[RPT][W], int tid, int r0, int rows, int r,
+                                               const double* u, const double* oldj) {
+  if (r == j) return;
 #pragma unroll
   for (int k = 0; k < RPT; ++k) {
     const int i = tid + k * RLEAF_THREADS, gi = r0 + i;
-    if (i >= rows || gi < J) continue;
-    if (gi == J) {
-      if (r != J)
+    if (i < rows && (gi == j || gi == r)) {
+      const double* src = gi == j ? u : oldj;
 #pragma unroll
-        for (int q = 0; q < W; ++q) rv[k][q] = u[q];
-      continue;
+      for (int q = 0; q < W; q += 2) {
+        const double2 v = *reinterpret_cast<const double2*>(src + q);
+        rv[k][q] = v.x;
+        rv[k][q + 1] = v.y;
+      }
     }
-    if (gi == r)
+  }
+}
+
+// Column J of the leaf for the calling thread's rows, J a compile-time
+// constant so every register of a row is addressed directly: scale column J
+// below the pivot (reciprocal multiply, as bl1_dinvscalv), rank-1 update, and
+// the candidate for column J + 1.  A column's body runs once per leaf and
+// comes from beyond the SM's instruction caches, so it holds nothing that
+// could stand outside it.  LEAFFIG
+template <int W, int RPT, int J>
+__device__ __forceinline__ void rleaf_column(double (&rv)[RPT][W], int tid, int r0, int rows, const double* u,
+                                             double rinv, double& bv, int& bi, int& bk) {
 #pragma unroll
-      for (int q = 0; q < W; ++q) rv[k][q] = oldj[q];
+  for (int k = 0; k < RPT; ++k) {
+    const int i = tid + k * RLEAF_THREADS, gi = r0 + i;
+    if (i >= rows || gi <= J) continue;
     const double l = rv[k][J] * rinv;
     rv[k][J] = l;
 #pragma unroll
-    for (int q = J + 1; q < W; ++q) rv[k][q] = fma(-l, u[q], rv[k][q]);
+    for (int q = (J + 1) & ~1; q < W; q += 2) {
+      const double2 v = *reinterpret_cast<const double2*>(u + q);
+      if (q > J) rv[k][q] = fma(-l, v.x, rv[k][q]);
+      rv[k][q + 1] = fma(-l, v.y, rv[k][q + 1]);
+    }
     if constexpr (J + 1 < W) {
       const double t = fabs(rv[k][J + 1]);
       if (t > bv) { bv = t; bi = gi; bk = k; }
@@ -98,16 +115,18 @@ __device__ __forceinline__ void rleaf_column(double (&rv)[RPT][W], int tid, int 
   }
 }
 
-// Run-time column j to its compile-time body through one jump table.
+// The exchange, then run-time column j to its compile-time body through one
+// jump table.
 template <int W, int RPT>
 __device__ __forceinline__ void rleaf_column_at(int j, double (&rv)[RPT][W], int tid, int r0, int rows, int r,
                                                 const double* u, const double* oldj, double rinv, double& bv,
                                                 int& bi, int& bk) {
-  static_assert(W <= 32, "leaf width");
+  static_assert(W <= 32 && W % 2 == 0, "leaf width");
+  rleaf_exchange<W, RPT>(j, rv, tid, r0, rows, r, u, oldj);
   switch (j) {
 #define FB_RLEAF_CASE(J)                                                              \
   case J:                                                                             \
-    if constexpr (J < W) rleaf_column<W, RPT, J>(rv, tid, r0, rows, r, u, oldj, rinv, bv, bi, bk); \
+    if constexpr (J < W) rleaf_column<W, RPT, J>(rv, tid, r0, rows, u, rinv, bv, bi, bk); \
     break;
     FB_RLEAF_CASE(0) FB_RLEAF_CASE(1) FB_RLEAF_CASE(2) FB_RLEAF_CASE(3) FB_RLEAF_CASE(4) FB_RLEAF_CASE(5)
     FB_RLEAF_CASE(6) FB_RLEAF_CASE(7) FB_RLEAF_CASE(8) FB_RLEAF_CASE(9) FB_RLEAF_CASE(10) FB_RLEAF_CASE(11)
