@@ -387,13 +387,13 @@ __global__ void __launch_bounds__(NT, LuB<NT>::MINB) lu_batched_f64_kernel(Batch
         __syncthreads();
         if (tid < b0) {
           for (int q = 0; q < nrhs; ++q) {
-            double y0 = W[(long)tid * ldw + n32 + q], y1 = 0.0;
+            double y0 = 0.0, y1 = 0.0;  // summed apart: one rounding at the size of the entry
 #pragma unroll
             for (int s = 0; s < LW; s += 2) {  // entries past w meet zeros of the copy
-              y0 = fma(-u[s], sx[q * LW + s], y0);
-              y1 = fma(-u[s + 1], sx[q * LW + s + 1], y1);
+              y0 = fma(u[s], sx[q * LW + s], y0);
+              y1 = fma(u[s + 1], sx[q * LW + s + 1], y1);
             }
-            W[(long)tid * ldw + n32 + q] = y0 + y1;
+            W[(long)tid * ldw + n32 + q] -= y0 + y1;
           }
         }
       }
