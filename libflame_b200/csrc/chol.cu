@@ -28,8 +28,7 @@ namespace fb {
 namespace {
 
 constexpr int NB = 128;        // outer block
-constexpr int LDS = NB + 4;    // SMEM leading dimension (= 4 mod 16: conflict-free DMMA fragments)
-constexpr int POTRF_THREADS = 512;
+constexpr int LDS = POTRF_LD;  // SMEM leading dimension
 constexpr int POTRF_SMEM = NB * LDS * 8;
 
 __device__ __forceinline__ bool guard_failed(const int* info) {
@@ -44,10 +43,12 @@ __device__ __forceinline__ bool guard_failed(const int* info) {
 //       redundantly in registers (chol8: no exchange inside the chain, per
 //       column a reciprocal square root, a product and a fused multiply-add),
 //       then solves its own rows against it (dtrsm's R,L,T,N order); rows of
-//       the block itself come out of the same formulas;
+//       the block itself come out of the same formulas, but stay in registers:
+//       other warps may still be reading the block;
 //       meanwhile the other warps subtract the previous step's products from the
 //       columns beyond this step on the FP64 tensor cores;
-//   (b) the rows lose this step's products in the next step's eight columns.
+//   (b) after a barrier of all warps the block's own rows are stored, and the
+//       rows below lose this step's products in the next step's eight columns.
 // Measured, one call of FLA_Chol between events (about 6 us without a kernel):
 // n = 100 30.7 -> 26.2 us, n = 128 32.2 -> 30.6 us against 32-column blocks
 // factored by one warp (lane = row, the column through shared memory, about
@@ -57,51 +58,11 @@ __device__ __forceinline__ void cp_async8(double* dst, const double* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
 }
 
-// S(r, c) -= sum_{k < 8} S(r, jb + k) S(c, jb + k) for 8 x 8 tiles: rows and
-// columns from lo (a multiple of 8) to b8, tiles on or below the diagonal;
-// warp w of nw takes the column tiles w, w + nw, ..., four row tiles at a time
-// in flight.  Entries above the diagonal of a diagonal tile are written too:
-// nothing reads them.
-__device__ __forceinline__ void syrk8_tiles(double* S, int jb, int lo, int b8, int w, int nw, int lane) {
-  const int g = lane >> 2, t = lane & 3;
-  for (int c = lo + 8 * w; c < b8; c += 8 * nw) {
-    const double* pb = S + c + g + (jb + t) * LDS;
-    const double b0 = pb[0], b1 = pb[4 * LDS];
-    for (int r = c; r < b8; r += 32) {
-      double a0[4], a1[4], o0[4], o1[4], d0[4], d1[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int ru = min(r + 8 * u, b8 - 8);
-        const double* pa = S + ru + g + (jb + t) * LDS;
-        const double* o = S + ru + g + (c + 2 * t) * LDS;
-        a0[u] = pa[0];
-        a1[u] = pa[4 * LDS];
-        o0[u] = o[0];
-        o1[u] = o[LDS];
-      }
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        d0[u] = d1[u] = 0.0;
-        dmma_884(d0[u], d1[u], a0[u], b0);
-      }
-#pragma unroll
-      for (int u = 0; u < 4; ++u) dmma_884(d0[u], d1[u], a1[u], b1);
-#pragma unroll
-      for (int u = 0; u < 4; ++u)
-        if (r + 8 * u < b8) {
-          double* o = S + r + 8 * u + g + (c + 2 * t) * LDS;
-          o[0] = o0[u] - d0[u];
-          o[LDS] = o1[u] - d1[u];
-        }
-    }
-  }
-}
-
 __global__ void __launch_bounds__(POTRF_THREADS, 1) potrf_diag_kernel(double* A, long ld, int b, int gcol,
                                                                    int* info) {
   chain_begin();
   extern __shared__ __align__(16) double S[];  // S[r + c*LDS]
-  __shared__ int s_fail;
+  __shared__ int s_fail[2];
   if (guard_failed(info)) return;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   // load the lower triangle (and diagonal) with asynchronous copies, all in
@@ -109,56 +70,14 @@ __global__ void __launch_bounds__(POTRF_THREADS, 1) potrf_diag_kernel(double* A,
   for (int c = warp; c < b; c += POTRF_THREADS / 32)
     for (int r = c + lane; r < b; r += 32) cp_async8(S + r + c * LDS, A + r + (long)c * ld);
   asm volatile("cp.async.wait_all;" ::: "memory");
-  if (tid == 0) s_fail = -1;
+  if (tid < 2) s_fail[tid] = -1;
   __syncthreads();
-  const int b8 = (b + 7) & ~7;
-#pragma unroll 1
-  for (int jb = 0; jb < b; jb += 8) {
-    double x[8];
-    const bool own = warp < 4 && tid >= jb && tid < b8;  // this thread's row takes part
-    if (warp < 4) {
-      if ((warp << 5) + 31 >= jb) {  // (a) (warps whose rows are all done skip it)
-        double l[36], ri[8];
-        const int fail = chol8_load_factor(S + jb + jb * LDS, LDS, l, ri);
-        if (tid == jb && fail >= 0 && jb + fail < b) s_fail = jb + fail;  // rows past b: not pivots
-        if (own) {
-#pragma unroll
-          for (int k = 0; k < 8; ++k) x[k] = S[tid + (jb + k) * LDS];
-          chol8_solve(l, ri, x);
-#pragma unroll
-          for (int k = 0; k < 8; ++k) S[tid + (jb + k) * LDS] = x[k];
-        }
-      }
-    } else if (jb > 0 && jb + 8 < b8) {
-      syrk8_tiles(S, jb - 8, jb + 8, b8, warp - 4, POTRF_THREADS / 32 - 4, lane);
-    }
-    __syncthreads();
-    if (s_fail >= 0) break;
-    if (warp < 4) {  // (b)
-      if (own && tid >= jb + 8) {
-        const double* row = S + jb + 8 + jb * LDS;  // rows jb + 8 .., this step's columns
-        double y[8];
-#pragma unroll
-        for (int c = 0; c < 8; ++c) y[c] = S[tid + (jb + 8 + c) * LDS];
-#pragma unroll
-        for (int k = 0; k < 8; ++k)
-#pragma unroll
-          for (int c = 0; c < 8; c += 2) {
-            const double2 v = *reinterpret_cast<const double2*>(row + c + k * LDS);
-            y[c] = fma(-x[k], v.x, y[c]);
-            y[c + 1] = fma(-x[k], v.y, y[c + 1]);
-          }
-#pragma unroll
-        for (int c = 0; c < 8; ++c) S[tid + (jb + 8 + c) * LDS] = y[c];
-      }
-      asm volatile("bar.sync 1, 128;" ::: "memory");
-    }
-  }
+  const int fail = potrf_block(S, b, s_fail);
   chain_next();
   // write back the lower triangle (the strictly upper part of A is untouched)
   for (int c = warp; c < b; c += POTRF_THREADS / 32)
     for (int r = c + lane; r < b; r += 32) A[r + (long)c * ld] = S[r + c * LDS];
-  if (tid == 0 && s_fail >= 0) atomicMin(info, gcol + s_fail);
+  if (tid == 0 && fail >= 0) atomicMin(info, gcol + fail);
 }
 
 bool g_attr_done = false;

@@ -51,6 +51,109 @@ __device__ __forceinline__ void chol8_solve(const double (&l)[36], const double 
   }
 }
 
+constexpr int POTRF_MAX = 128;              // largest block of potrf_block
+constexpr int POTRF_LD = POTRF_MAX + 4;     // = 4 mod 16: conflict-free DMMA fragments
+constexpr int POTRF_THREADS = 512;
+
+// S(r, c) -= sum_{k < 8} S(r, jb + k) S(c, jb + k) for 8 x 8 tiles: rows and
+// columns from lo (a multiple of 8) to b8, tiles on or below the diagonal;
+// warp w of nw takes the column tiles w, w + nw, ..., four row tiles at a time
+// in flight.  Entries above the diagonal of a diagonal tile are written too:
+// nothing reads them.
+__device__ __forceinline__ void syrk8_tiles(double* S, int jb, int lo, int b8, int w, int nw, int lane) {
+  const int g = lane >> 2, t = lane & 3;
+  for (int c = lo + 8 * w; c < b8; c += 8 * nw) {
+    const double* pb = S + c + g + (jb + t) * POTRF_LD;
+    const double b0 = pb[0], b1 = pb[4 * POTRF_LD];
+    for (int r = c; r < b8; r += 32) {
+      double a0[4], a1[4], o0[4], o1[4], d0[4], d1[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int ru = min(r + 8 * u, b8 - 8);
+        const double* pa = S + ru + g + (jb + t) * POTRF_LD;
+        const double* o = S + ru + g + (c + 2 * t) * POTRF_LD;
+        a0[u] = pa[0];
+        a1[u] = pa[4 * POTRF_LD];
+        o0[u] = o[0];
+        o1[u] = o[POTRF_LD];
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        d0[u] = d1[u] = 0.0;
+        dmma_884(d0[u], d1[u], a0[u], b0);
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) dmma_884(d0[u], d1[u], a1[u], b1);
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (r + 8 * u < b8) {
+          double* o = S + r + 8 * u + g + (c + 2 * t) * POTRF_LD;
+          o[0] = o0[u] - d0[u];
+          o[POTRF_LD] = o1[u] - d1[u];
+        }
+    }
+  }
+}
+
+// The b x b (b <= 128) lower triangle in shared memory, S(r, c) at S[r + c *
+// POTRF_LD], := its Cholesky factor, by all POTRF_THREADS threads of the CTA.
+// Returns the first failing column, -1 if none, in every thread.  s_fail: two
+// words of shared memory, -1 (before a barrier).
+__device__ __forceinline__ int potrf_block(double* S, int b, int* s_fail) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int b8 = (b + 7) & ~7;
+#pragma unroll 1
+  for (int jb = 0; jb < b; jb += 8) {
+    double x[8];
+    const bool own = warp < 4 && tid >= jb && tid < b8;  // this thread's row takes part
+    if (warp < 4) {
+      if ((warp << 5) + 31 >= jb) {  // (a) (warps whose rows are all done skip it)
+        double l[36], ri[8];
+        const int fail = chol8_load_factor(S + jb + jb * POTRF_LD, POTRF_LD, l, ri);
+        if (tid == jb && fail >= 0 && jb + fail < b) s_fail[0] = jb + fail;  // rows past b: not pivots
+        if (own) {
+#pragma unroll
+          for (int k = 0; k < 8; ++k) x[k] = S[tid + (jb + k) * POTRF_LD];
+          chol8_solve(l, ri, x);
+          if (tid >= jb + 8) {
+#pragma unroll
+            for (int k = 0; k < 8; ++k) S[tid + (jb + k) * POTRF_LD] = x[k];
+          }
+        }
+      }
+    } else if (jb > 0 && jb + 8 < b8) {
+      syrk8_tiles(S, jb - 8, jb + 8, b8, warp - 4, POTRF_THREADS / 32 - 4, lane);
+    }
+    __syncthreads();
+    if (own && tid < jb + 8) {  // every warp has read the block
+#pragma unroll
+      for (int k = 0; k < 8; ++k) S[tid + (jb + k) * POTRF_LD] = x[k];
+    }
+    if (s_fail[0] >= 0) break;
+    if (warp < 4) {  // (b)
+      if (own && tid >= jb + 8) {
+        const double* row = S + jb + 8 + jb * POTRF_LD;  // rows jb + 8 .., this step's columns
+        double y[8];
+#pragma unroll
+        for (int c = 0; c < 8; ++c) y[c] = S[tid + (jb + 8 + c) * POTRF_LD];
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+#pragma unroll
+          for (int c = 0; c < 8; c += 2) {
+            const double2 v = *reinterpret_cast<const double2*>(row + c + k * POTRF_LD);
+            y[c] = fma(-x[k], v.x, y[c]);
+            y[c + 1] = fma(-x[k], v.y, y[c + 1]);
+          }
+#pragma unroll
+        for (int c = 0; c < 8; ++c) S[tid + (jb + 8 + c) * POTRF_LD] = y[c];
+      }
+      bar_sync(1, 128);
+    }
+  }
+  __syncthreads();  // the last block's rows
+  return s_fail[0];
+}
+
 }  // namespace
 
 }  // namespace fb

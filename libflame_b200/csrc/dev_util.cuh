@@ -95,6 +95,11 @@ __device__ __forceinline__ void dmma_884(double& d0, double& d1, double a, doubl
                : "d"(a), "d"(b));
 }
 
+// Named barrier `id` (1..15) of the CTA for `threads` threads (whole warps).
+__device__ __forceinline__ void bar_sync(int id, int threads) {
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+
 // Grid-wide barrier for cooperative launches: monotonically increasing
 // counter; barrier number `epoch` (1-based) completes when it reaches
 // nblocks*epoch.  Bounded: returns false (and sets *err) on timeout.
