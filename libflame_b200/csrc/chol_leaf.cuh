@@ -98,19 +98,22 @@ __device__ __forceinline__ void syrk8_tiles(double* S, int jb, int lo, int b8, i
 // The b x b (b <= 128) lower triangle in shared memory, S(r, c) at S[r + c *
 // POTRF_LD], := its Cholesky factor, by all POTRF_THREADS threads of the CTA.
 // Returns the first failing column, -1 if none, in every thread.  s_fail: two
-// words of shared memory, -1 (before a barrier).
+// words of shared memory, -1 (before a barrier); steps take them in turn, since
+// a warp may read a step's word while the next step is under way, and every
+// warp has to leave in the same step.
 __device__ __forceinline__ int potrf_block(double* S, int b, int* s_fail) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int b8 = (b + 7) & ~7;
 #pragma unroll 1
   for (int jb = 0; jb < b; jb += 8) {
     double x[8];
+    int* flag = s_fail + ((jb >> 3) & 1);
     const bool own = warp < 4 && tid >= jb && tid < b8;  // this thread's row takes part
     if (warp < 4) {
       if ((warp << 5) + 31 >= jb) {  // (a) (warps whose rows are all done skip it)
         double l[36], ri[8];
         const int fail = chol8_load_factor(S + jb + jb * POTRF_LD, POTRF_LD, l, ri);
-        if (tid == jb && fail >= 0 && jb + fail < b) s_fail[0] = jb + fail;  // rows past b: not pivots
+        if (tid == jb && fail >= 0 && jb + fail < b) *flag = jb + fail;  // rows past b: not pivots
         if (own) {
 #pragma unroll
           for (int k = 0; k < 8; ++k) x[k] = S[tid + (jb + k) * POTRF_LD];
@@ -129,7 +132,7 @@ __device__ __forceinline__ int potrf_block(double* S, int b, int* s_fail) {
 #pragma unroll
       for (int k = 0; k < 8; ++k) S[tid + (jb + k) * POTRF_LD] = x[k];
     }
-    if (s_fail[0] >= 0) break;
+    if (*flag >= 0) break;
     if (warp < 4) {  // (b)
       if (own && tid >= jb + 8) {
         const double* row = S + jb + 8 + jb * POTRF_LD;  // rows jb + 8 .., this step's columns
@@ -151,7 +154,7 @@ __device__ __forceinline__ int potrf_block(double* S, int b, int* s_fail) {
     }
   }
   __syncthreads();  // the last block's rows
-  return s_fail[0];
+  return max(s_fail[0], s_fail[1]);
 }
 
 }  // namespace

@@ -13,7 +13,8 @@ int main() {
   using namespace fb;
   std::mt19937_64 rng(5);
   std::normal_distribution<double> nd;
-  const int cases[][2] = {{1, -1}, {7, -1}, {8, -1}, {9, -1}, {32, -1}, {33, -1}, {63, -1}, {72, -1}, {100, -1}, {128, -1}};
+  const int cases[][2] = {{1, -1}, {7, -1}, {8, -1}, {9, -1}, {32, -1}, {33, -1}, {63, -1}, {72, -1}, {100, -1}, {128, -1},
+                          {9, 8}, {40, 0}, {72, 35}, {128, 7}, {128, 8}, {128, 77}, {128, 127}};
   for (auto& cs : cases) {
     const int b = cs[0], f = cs[1], ld = POTRF_LD;
     std::vector<double> G(b * b), S0(POTRF_MAX * ld, std::nan(""));

@@ -26,7 +26,7 @@ def test_potrf_block(tmp_path):
     """Diagonal block of the Cholesky (chol_leaf.cuh).  Error: at most b rounded
     operations on an entry of a factor whose condition is below 10, so 10 b eps."""
     lines = _run(tmp_path, "chol_leaf.cuh", "potrf_block.cpp").splitlines()
-    assert len(lines) == 10
+    assert len(lines) == 17
     for line in lines:
         b, f, ret, agree, bars, err = line.split()
         assert int(ret) == int(f), line
