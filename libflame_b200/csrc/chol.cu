@@ -43,17 +43,18 @@ __device__ __forceinline__ bool guard_failed(const int* info) {
 //       redundantly in registers (chol8: no exchange inside the chain, per
 //       column a reciprocal square root, a product and a fused multiply-add),
 //       then solves its own rows against it (dtrsm's R,L,T,N order); rows of
-//       the block itself come out of the same formulas, but stay in registers:
-//       other warps may still be reading the block;
+//       the block itself come out of the same formulas, and the warp that owns
+//       them stores them once the other warps have announced (bar.arrive) that
+//       they have read the block;
 //       meanwhile the other warps subtract the previous step's products from the
 //       columns beyond this step on the FP64 tensor cores;
-//   (b) after a barrier of all warps the block's own rows are stored, and the
-//       rows below lose this step's products in the next step's eight columns.
+//   (b) the rows lose this step's products in the next step's eight columns.
 // Measured, one call of FLA_Chol between events (about 6 us without a kernel):
 // n = 100 30.7 -> 26.2 us, n = 128 32.2 -> 30.6 us against 32-column blocks
 // factored by one warp (lane = row, the column through shared memory, about
 // 370 cycles a column); with four instead of twelve warps for the products
-// n = 128 took 32.4 us.
+// n = 128 took 32.4 us.  With the block's rows stored after the CTA barrier
+// instead of the arrivals, n = 1024 (eight blocks) took 336 us, now 325.
 __device__ __forceinline__ void cp_async8(double* dst, const double* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
 }

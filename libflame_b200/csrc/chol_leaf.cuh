@@ -12,8 +12,9 @@ namespace {
 // aligned, ld even) factored by every lane alike: l[i (i + 1) / 2 + k] =
 // L(i, k) off the diagonal, ri[k] = 1 / L(k, k).  Returns the first column
 // whose pivot is not > 0 (NaN included), -1 if none; what follows it is not
-// meaningful then.
-__device__ __forceinline__ int chol8_load_factor(const double* D, int ld, double (&l)[36], double (&ri)[8]) {
+// meaningful then.  loaded(): called between the loads and the factorization.
+template <class F>
+__device__ __forceinline__ int chol8_load_factor(const double* D, int ld, double (&l)[36], double (&ri)[8], F loaded) {
 #pragma unroll
   for (int k = 0; k < 8; ++k)
 #pragma unroll
@@ -22,6 +23,7 @@ __device__ __forceinline__ int chol8_load_factor(const double* D, int ld, double
       if (i >= k) l[i * (i + 1) / 2 + k] = v.x;
       l[(i + 1) * (i + 2) / 2 + k] = v.y;
     }
+  loaded();
   int fail = -1;
 #pragma unroll
   for (int k = 0; k < 8; ++k) {
@@ -112,26 +114,25 @@ __device__ __forceinline__ int potrf_block(double* S, int b, int* s_fail) {
     if (warp < 4) {
       if ((warp << 5) + 31 >= jb) {  // (a) (warps whose rows are all done skip it)
         double l[36], ri[8];
-        const int fail = chol8_load_factor(S + jb + jb * POTRF_LD, POTRF_LD, l, ri);
+        const int fail = chol8_load_factor(S + jb + jb * POTRF_LD, POTRF_LD, l, ri, [&] {
+          if (warp != jb >> 5) bar_arrive(2, 128 - (jb & ~31));
+        });
+        // the warp that owns the block's rows stores them below: not before
+        // the others have read the block
+        if (warp == jb >> 5) bar_sync(2, 128 - (jb & ~31));
         if (tid == jb && fail >= 0 && jb + fail < b) *flag = jb + fail;  // rows past b: not pivots
         if (own) {
 #pragma unroll
           for (int k = 0; k < 8; ++k) x[k] = S[tid + (jb + k) * POTRF_LD];
           chol8_solve(l, ri, x);
-          if (tid >= jb + 8) {
 #pragma unroll
-            for (int k = 0; k < 8; ++k) S[tid + (jb + k) * POTRF_LD] = x[k];
-          }
+          for (int k = 0; k < 8; ++k) S[tid + (jb + k) * POTRF_LD] = x[k];
         }
       }
     } else if (jb > 0 && jb + 8 < b8) {
       syrk8_tiles(S, jb - 8, jb + 8, b8, warp - 4, POTRF_THREADS / 32 - 4, lane);
     }
     __syncthreads();
-    if (own && tid < jb + 8) {  // every warp has read the block
-#pragma unroll
-      for (int k = 0; k < 8; ++k) S[tid + (jb + k) * POTRF_LD] = x[k];
-    }
     if (*flag >= 0) break;
     if (warp < 4) {  // (b)
       if (own && tid >= jb + 8) {
@@ -153,7 +154,6 @@ __device__ __forceinline__ int potrf_block(double* S, int b, int* s_fail) {
       bar_sync(1, 128);
     }
   }
-  __syncthreads();  // the last block's rows
   return max(s_fail[0], s_fail[1]);
 }
 

@@ -100,6 +100,12 @@ __device__ __forceinline__ void bar_sync(int id, int threads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }
 
+// Arrival at a named barrier without waiting for it: what this thread read
+// before stays valid for the threads that bar_sync on it.
+__device__ __forceinline__ void bar_arrive(int id, int threads) {
+  asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+
 // Grid-wide barrier for cooperative launches: monotonically increasing
 // counter; barrier number `epoch` (1-based) completes when it reaches
 // nblocks*epoch.  Bounded: returns false (and sets *err) on timeout.

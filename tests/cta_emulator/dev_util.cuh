@@ -61,9 +61,9 @@ inline void check(int bar) {
     release(BARRIER, 0, (int)th.size(), bar);
   }
 }
-inline void arrive(int bar, int n) {
+inline void arrive(int bar, int n, bool wait = true) {
   Thread& t = th[cur];
-  t.state = BARRIER;
+  if (wait) t.state = BARRIER;
   t.bar = bar;
   expected[bar] = n;
   if (bar == 0) ++t.syncs;
@@ -129,6 +129,7 @@ inline void __syncthreads() { emu::arrive(0, 0); }
 
 namespace fb {
 inline void bar_sync(int id, int threads) { emu::arrive(id, threads); }
+inline void bar_arrive(int id, int threads) { emu::arrive(id, threads, false); }
 // D(g, 2t..2t+1) += sum_k A(g, k) B(k, 2t..), lane = 4 g + t holding A(g, t), B(t, g)
 inline void dmma_884(double& d0, double& d1, double a, double b) {
   const int lane = emu::cur & 31, lo = emu::cur - lane, g = lane >> 2, t = lane & 3;
