@@ -7,20 +7,22 @@
 //             transposed storage U12^T is X and row i of L11 a contiguous
 //             column of A^T.
 //
-// By 32-column blocks: X_k := A_k inv(L_kk)^T, then the products of block k
-// are subtracted from the columns to its right, all on the FP64 tensor cores.
-// The inverses of the 32 x 32 diagonal blocks (zero above the diagonal) take
-// their place in shared memory first: eight warps invert the 16 x 16 blocks
-// by forward substitution, one column per lane, and each 32 x 32 one is
-// completed by I21 = -I22 (L21 I11).  A CTA holds the triangle and ROWS rows
-// of X; fewer rows per CTA when there are few rows, so that they spread over
-// the SMs.  Bound by the latency of the load, the 16 dependent steps of the
-// small inverses and four pairs of products.
-// Measured against forward substitution with a shuffle per column (a warp
-// per row group): 896 x 128 16.2 -> 10.2 us, the LU's joins (up to 128 x 128) 9.8 -> 7.2 us on
-// average; 8000 x 128 takes 18 us, less than inv(L11), a copy and a product.
-// (Substitution with a row per thread by 32-column blocks took 17.8 us: one
-// warp's 496 dependent loads and FMAs per block.)
+// By steps of 16 columns, the reference's order within a step: a thread per row
+// solves them by forward substitution in registers (dtrsm's R,L,T,N case), the
+// products with the columns beyond are subtracted on the FP64 tensor cores:
+// first those the next step needs, the rest beside its substitution.  A CTA
+// holds the triangle and ROWS rows of X; fewer rows per CTA when there are few
+// rows, so that they spread over the SMs.  Bound by the latency of the load and
+// the chain of steps; sixteen columns, because a step's 120 FMAs then just fill
+// the latency of its own chain of sixteen.
+// Substitution rather than products with inverted diagonal blocks: the error of
+// those grows with the condition of the block (n = 512, squared-exponential
+// kernel, nugget 1e-9: ||A - L L^T|| / ||A|| 2.6e-15 with 32 x 32 inverses,
+// 1.5e-16 so; an LU whose 32 x 32 blocks are near -1 below the diagonal 1.1e-8
+// and 1.2e-16), and an infinite entry spoils columns before its own.  FLA_Chol
+// n = 1024 takes 327 us with inverses, 335 us so; FLA_LU_piv n = 3001 6.24 ms
+// both ways.  (A shuffle per column, a warp per row group: 896 x 128
+// 16.2 us against 10.2 with the inverses; a row per thread by 32 columns 17.8.)
 #include <algorithm>
 
 #include "common.h"
@@ -31,7 +33,7 @@ namespace fb {
 namespace {
 
 constexpr int RB = 128;           // widest triangle
-constexpr int RIB = 32;           // columns per substitution step
+constexpr int RIB = 16;           // columns per substitution step
 constexpr int RLD = RB + 4;       // = 4 mod 16: conflict-free DMMA fragments
 constexpr int R_THREADS = 256;
 
@@ -39,96 +41,68 @@ template <int ROWS>
 constexpr int rlt_ldx() { return ROWS + 4; }  // = 4 mod 16
 template <int ROWS>
 size_t rlt_smem(int b) {
-  const int b32 = (b + RIB - 1) / RIB * RIB;
-  return sizeof(double) * ((size_t)b32 * RLD + (size_t)b32 * rlt_ldx<ROWS>() + RB);
+  const int bp = (b + RIB - 1) / RIB * RIB;
+  return sizeof(double) * ((size_t)bp * RLD + (size_t)bp * rlt_ldx<ROWS>() + RB);
 }
 
 __device__ __forceinline__ void cp_async8(double* dst, const double* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
 }
 
-// X(:, c_lo + 8 j) -= X(:, kb..kb+31) L(c, kb..kb+31)^T for ntj 8-column
-// tiles, the ROWS/8 x ntj tiles dealt to the warps.
+// X(:, c) -= X(:, kb..kb+15) L(c, kb..kb+15)^T for the 8-column tiles from c_lo
+// up to c_hi, the tiles of 8 rows dealt to nw warps, w the calling one.
 template <int ROWS>
-__device__ __forceinline__ void rlt_update(const double* sL, double* sX, int kb, int c_lo, int ntj, int w, int lane) {
+__device__ __forceinline__ void rlt_update(const double* sL, double* sX, int kb, int c_lo, int c_hi, int w, int nw, int lane) {
   constexpr int LDX = rlt_ldx<ROWS>(), TI = ROWS / 8;
   const int g = lane >> 2, t = lane & 3;
-  for (int e = w; e < TI * ntj; e += R_THREADS / 32) {
+  for (int e = w; e < TI * ((c_hi - c_lo) >> 3); e += nw) {
     const int r = 8 * (e % TI), c = c_lo + 8 * (e / TI);
     const double* pa = sX + r + g + (kb + t) * LDX;
     const double* pb = sL + c + g + (kb + t) * RLD;
-    double d0[2] = {0.0, 0.0}, d1[2] = {0.0, 0.0};
-#pragma unroll
-    for (int k = 0; k < RIB; k += 8) {
-      dmma_884(d0[0], d0[1], pa[k * LDX], pb[k * RLD]);
-      dmma_884(d1[0], d1[1], pa[(k + 4) * LDX], pb[(k + 4) * RLD]);
-    }
     double* o = sX + r + g + (c + 2 * t) * LDX;
-    o[0] -= d0[0] + d1[0];
-    o[LDX] -= d0[1] + d1[1];
-  }
-}
-
-// The 16 x 16 diagonal block at D := its inverse, zero above the diagonal.
-template <bool UNIT>
-__device__ __forceinline__ void rlt_invert16(double* D, const double* rinv, int lane) {
-  const int c = lane & 15;
-  double x[16];
+    const double o0 = o[0], o1 = o[LDX];
+    double d0[2] = {0.0, 0.0}, d1[2] = {0.0, 0.0};  // halves of the sixteen, in order
 #pragma unroll
-  for (int r = 0; r < 16; ++r) x[r] = r == c ? 1.0 : 0.0;
-#pragma unroll
-  for (int j = 0; j < 16; ++j) {
-    if (!UNIT) x[j] *= rinv[j];
-    double l[16];
-#pragma unroll
-    for (int r = (j + 1) & ~1; r < 16; r += 2) {
-      const double2 v = *reinterpret_cast<const double2*>(D + r + j * RLD);
-      l[r] = v.x;
-      l[r + 1] = v.y;
+    for (int k = 0; k < RIB / 2; k += 4) {
+      dmma_884(d0[0], d0[1], pa[k * LDX], pb[k * RLD]);
+      dmma_884(d1[0], d1[1], pa[(k + RIB / 2) * LDX], pb[(k + RIB / 2) * RLD]);
     }
-#pragma unroll
-    for (int r = j + 1; r < 16; ++r) x[r] = fma(-l[r], x[j], x[r]);
+    o[0] = o0 - (d0[0] + d1[0]);
+    o[LDX] = o1 - (d0[1] + d1[1]);
   }
-  __syncwarp();
-  if (lane < 16)
-#pragma unroll
-    for (int r = 0; r < 16; ++r) D[r + c * RLD] = r >= c ? x[r] : 0.0;
 }
 
-// Z := sgn Y W for 16 x 16 blocks in shared memory (ld RLD), by one warp; Z
-// may not overlap Y or W.
-__device__ __forceinline__ void rlt_mul16(const double* Y, const double* Wm, double* Z, double sgn, int lane) {
-  const int g = lane >> 2, t = lane & 3;
-  double d[2][2][2] = {};
+// x := x inv(D)^T for a row x of RIB entries, D the diagonal block at D (ld
+// RLD), its reciprocal pivots in rinv.
+template <bool UNIT>
+__device__ __forceinline__ void rlt_solve(const double* D, const double* rinv, double (&x)[RIB]) {
 #pragma unroll
-  for (int k = 0; k < 16; k += 4)
+  for (int k = 0; k < RIB; ++k) {
+    if (!UNIT) x[k] *= rinv[k];
+    if (k % 2 == 0) x[k + 1] = fma(-D[k + 1 + k * RLD], x[k], x[k + 1]);
 #pragma unroll
-    for (int i = 0; i < 2; ++i)
-#pragma unroll
-      for (int j = 0; j < 2; ++j)
-        dmma_884(d[i][j][0], d[i][j][1], Y[8 * i + g + (k + t) * RLD], Wm[k + t + (8 * j + g) * RLD]);
-#pragma unroll
-  for (int i = 0; i < 2; ++i)
-#pragma unroll
-    for (int j = 0; j < 2; ++j)
-#pragma unroll
-      for (int e = 0; e < 2; ++e) Z[8 * i + g + (8 * j + 2 * t + e) * RLD] = sgn * d[i][j][e];
+    for (int c = (k + 2) & ~1; c < RIB; c += 2) {
+      const double2 v = *reinterpret_cast<const double2*>(D + c + k * RLD);
+      x[c] = fma(-v.x, x[k], x[c]);
+      x[c + 1] = fma(-v.y, x[k], x[c + 1]);
+    }
+  }
 }
 
 // UNIT: unit L with L(i, j) at Ls[j + i ld]; else non-unit, L(i, j) at
 // Ls[i + j ld].  X(r, c) at X[r + c ldx].  Returns at once when *guard holds
 // a failing column below guard_limit.
 template <int ROWS, bool UNIT, typename TX>
-__global__ void __launch_bounds__(R_THREADS) rlt_kernel(const double* __restrict__ Ls, long ld, TX* __restrict__ X,
+__global__ void __launch_bounds__(R_THREADS, 1) rlt_kernel(const double* __restrict__ Ls, long ld, TX* __restrict__ X,
                                                         long ldx, int b, long m, const int* guard, int guard_limit) {
   chain_begin();
   constexpr int LDX = rlt_ldx<ROWS>();
   extern __shared__ __align__(16) double rlt_sm[];
   if (guard && *((volatile const int*)guard) < guard_limit) return;
-  const int b32 = (b + RIB - 1) / RIB * RIB, b8 = (b + 7) & ~7;
+  const int bp = (b + RIB - 1) / RIB * RIB;
   double* sL = rlt_sm;               // L(i, j) at sL[i + j * RLD]
-  double* sX = sL + b32 * RLD;       // X(r, c) at sX[r + c * LDX]
-  double* sR = sX + b32 * LDX;       // reciprocal pivots
+  double* sX = sL + bp * RLD;       // X(r, c) at sX[r + c * LDX]
+  double* sR = sX + bp * LDX;       // reciprocal pivots
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const long r0 = (long)blockIdx.x * ROWS;
   const int rows = (int)(m - r0 < ROWS ? m - r0 : ROWS);
@@ -152,60 +126,39 @@ __global__ void __launch_bounds__(R_THREADS) rlt_kernel(const double* __restrict
       sX[r + c * LDX] = r < rows ? (double)X[r0 + r + (long)c * ldx] : 0.0;
     }
   }
-  if (b < b32) {  // rows of the triangle and columns of X past b
-    for (int e = tid; e < b32 * (b32 - b); e += R_THREADS) sL[b + e % (b32 - b) + e / (b32 - b) * RLD] = 0.0;
-    for (int e = tid; e < ROWS * (b32 - b); e += R_THREADS) sX[e % ROWS + (b + e / ROWS) * LDX] = 0.0;
+  if (b < bp) {  // rows of the triangle and columns of X past b
+    for (int e = tid; e < bp * (bp - b); e += R_THREADS) sL[b + e % (bp - b) + e / (bp - b) * RLD] = 0.0;
+    for (int e = tid; e < ROWS * (bp - b); e += R_THREADS) sX[e % ROWS + (b + e / ROWS) * LDX] = 0.0;
   }
   asm volatile("cp.async.wait_all;" ::: "memory");
   __syncthreads();
   if (!UNIT) {
-    for (int j = tid; j < b32; j += R_THREADS) sR[j] = j < b ? 1.0 / sL[j + j * RLD] : 1.0;
+    for (int j = tid; j < bp; j += R_THREADS) sR[j] = j < b ? 1.0 / sL[j + j * RLD] : 1.0;
     __syncthreads();
   }
-  // inverses of the diagonal blocks, in place
-  if (16 * warp < b32) rlt_invert16<UNIT>(sL + 16 * warp * (1 + RLD), sR + 16 * warp, lane);
-  __syncthreads();
-  if (RIB * warp < b32) {
-    double* D = sL + RIB * warp * (1 + RLD);
-    double* Tm = D + 16 * RLD;  // the block's upper right quarter, for L21 I11
-    rlt_mul16(D + 16, D, Tm, 1.0, lane);
-    __syncwarp();
-    rlt_mul16(D + 16 * (1 + RLD), Tm, D + 16, -1.0, lane);
-    __syncwarp();
-    for (int e = lane; e < 256; e += 32) Tm[(e & 15) + (e >> 4) * RLD] = 0.0;
-  }
-  __syncthreads();
-  constexpr int TPW = (ROWS / 8) * (RIB / 8) / (R_THREADS / 32);  // tiles of X_k per warp
-  const int g = lane >> 2, t = lane & 3;
+  // row warps: a thread per row; the others subtract the products, with few
+  // rows without the one on the row warp's sub-partition
+  constexpr int RW = (ROWS + 31) / 32;
+  constexpr int UW = ROWS <= 32 ? 6 : R_THREADS / 32 - RW;
+  const int uw = ROWS <= 32 ? (warp & 3) - 1 + 3 * (warp >> 2) : warp - RW;  // UW update warps
+  const bool upd = ROWS <= 32 ? (warp & 3) != 0 : warp >= RW;
   for (int kb = 0; kb < b; kb += RIB) {
-    // X_k := A_k inv(L_kk)^T: tile (ri, cj), k up to the end of column tile cj
-    double x[TPW][2];
+    if (warp < RW) {
+      if (tid < ROWS) {
+        double x[RIB];
+        double* row = sX + tid + kb * LDX;
 #pragma unroll
-    for (int u = 0; u < TPW; ++u) {
-      const int e = warp + u * (R_THREADS / 32);
-      const int r = 8 * (e % (ROWS / 8)), c = 8 * (e / (ROWS / 8));
-      const double* pa = sX + r + g + (kb + t) * LDX;
-      const double* pb = sL + kb + c + g + (kb + t) * RLD;
-      double d0[2] = {0.0, 0.0}, d1[2] = {0.0, 0.0};
-      for (int k = 0; k <= c; k += 8) {
-        dmma_884(d0[0], d0[1], pa[k * LDX], pb[k * RLD]);
-        dmma_884(d1[0], d1[1], pa[(k + 4) * LDX], pb[(k + 4) * RLD]);
+        for (int c = 0; c < RIB; ++c) x[c] = row[c * LDX];
+        rlt_solve<UNIT>(sL + kb * (1 + RLD), sR + kb, x);
+#pragma unroll
+        for (int c = 0; c < RIB; ++c) row[c * LDX] = x[c];
       }
-      x[u][0] = d0[0] + d1[0];
-      x[u][1] = d0[1] + d1[1];
+    } else if (upd && kb > 0) {
+      rlt_update<ROWS>(sL, sX, kb - RIB, kb + RIB, bp, uw, UW, lane);
     }
     __syncthreads();
-#pragma unroll
-    for (int u = 0; u < TPW; ++u) {
-      const int e = warp + u * (R_THREADS / 32);
-      const int r = 8 * (e % (ROWS / 8)), c = 8 * (e / (ROWS / 8));
-      double* o = sX + r + g + (kb + c + 2 * t) * LDX;
-      o[0] = x[u][0];
-      o[LDX] = x[u][1];
-    }
-    __syncthreads();
-    if (kb + RIB >= b8) break;
-    rlt_update<ROWS>(sL, sX, kb, kb + RIB, (b8 - kb - RIB) / 8, warp, lane);
+    if (kb + RIB >= b) break;
+    rlt_update<ROWS>(sL, sX, kb, kb + RIB, kb + 2 * RIB, warp, R_THREADS / 32, lane);
     __syncthreads();
   }
   chain_next();
@@ -229,8 +182,8 @@ void rlt_launch(const double* L, long ld, TX* X, long ldx, int b, long m, const 
         L, ld, X, ldx, b, m, guard, guard_limit));
 }
 
-// Rows per CTA: the fewest that leave one wave (a 128-column triangle allows
-// one CTA per SM, a 64-column one three).
+// Rows per CTA: the fewest that leave one wave (shared memory allows one CTA per
+// SM with a 128-column triangle, two with a 64-column one).
 template <bool UNIT, typename TX>
 int rlt_any(const double* L, long ld, TX* X, long ldx, int b, long m, const int* guard, int guard_limit,
             cudaStream_t st) {
@@ -239,7 +192,7 @@ int rlt_any(const double* L, long ld, TX* X, long ldx, int b, long m, const int*
     set_last_error("triangular solve: triangle wider than 128");
     return FLA_FAILURE;
   }
-  const long wave = (long)ctx().num_sms * (b <= 64 ? 3 : 1);
+  const long wave = (long)ctx().num_sms * (b <= 64 ? 2 : 1);
   const int ps = prof_begin(st);
   if (m <= 16 * wave) rlt_launch<16, UNIT, TX>(L, ld, X, ldx, b, m, guard, guard_limit, st);
   else if (m <= 32 * wave) rlt_launch<32, UNIT, TX>(L, ld, X, ldx, b, m, guard, guard_limit, st);
