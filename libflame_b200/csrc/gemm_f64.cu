@@ -303,20 +303,23 @@ __global__ void __launch_bounds__(Tile<BM_, BN_>::THREADS, Tile<BM_, BN_>::MINB)
 // leaves most SMs idle and a chain of such products (the factorizations'
 // panel joins and lookahead updates, the solves) waits for one tile's k
 // loop: 32 x 32 tiles, four times as many CTAs, and the four warps of a CTA
-// share each 16 of k (warp w takes 4w..4w+3 for the whole tile), so these cost
-// each SM sub-partition 16 DMMAs instead of 64.  The four partial tiles are
-// added through shared memory in warp order.  Four stages of 32 k (64 KB,
-// three CTAs per SM): a depth of 128 is in flight at once, and a barrier wait
-// is paid every 32 k only.  C is read into registers
-// before the k loop.  Measured, one call between events (an empty one is
-// about 5 us), 64 x 64 tiles against these: 896 x 128 x 128 16.8 -> 8.9 us,
-// 768 x 256 x 256 25.1 -> 12.8, 1536 x 256 x 128 16.7 -> 11.2; past the
-// limit 2048 x 768 x 128 (384 tiles) 25.9 -> 31.6.
-constexpr int SM_T = 32, SM_STAGES = 4, SM_BK = 2 * BK;
-constexpr int SM_A_BYTES = SM_T * BK * 8, SM_HALF_BYTES = 2 * SM_A_BYTES, SM_STAGE_BYTES = 2 * SM_HALF_BYTES;
-constexpr int SM_SMEM = SM_STAGES * SM_STAGE_BYTES + 2048 /*align*/ + 256 /*barriers*/;
+// share k, so these cost each SM sub-partition a quarter of the DMMAs.  Warp w
+// takes the w-th quarter of k, in order: in a factorization the sum over a run
+// of k is the difference of two Schur complements, which are bounded where the
+// sum over every fourth k is not (A22 of a 256 x 256 LU: 1.53e-15 off per entry
+// with k dealt round, 1.28e-15 in one chain).  Each warp has its own ring of
+// boxes of 16 k (TMA, one barrier per box, no exchange between the warps before
+// the end); 64 KB, three CTAs per SM, a depth of 128 in flight.  The four
+// partial tiles are added through shared memory in warp order.  C is read into
+// registers before the k loop.  Measured, one call between events (an empty one
+// is about 5 us), 64 x 64 tiles against these: 896 x 128 x 128 18.2 -> 9.4 us,
+// 768 x 256 x 256 25.8 -> 13.6, 1536 x 256 x 128 17.8 -> 13.2, 128 x 128 x 2048
+// 39.2 -> 16.6; past the limit 2048 x 768 x 128 (384 tiles) 25.9 -> 31.6.
+constexpr int SM_T = 32, SM_WARPS = 4, SM_RING = 2;
+constexpr int SM_A_BYTES = SM_T * BK * 8, SM_BOX_BYTES = 2 * SM_A_BYTES;
+constexpr int SM_SMEM = SM_WARPS * SM_RING * SM_BOX_BYTES + 2048 /*align*/ + 256 /*barriers*/;
 template <bool A_K, bool B_K>
-__global__ void __launch_bounds__(128) dgemm_small_kernel(const __grid_constant__ CUtensorMap mapA,
+__global__ void __launch_bounds__(32 * SM_WARPS, 3) dgemm_small_kernel(const __grid_constant__ CUtensorMap mapA,
                                                           const __grid_constant__ CUtensorMap mapB,
                                                           double* __restrict__ C, long ldc, int M, int N, int K,
                                                           double alpha, double beta, int mode, long diag_off, int* err,
@@ -327,17 +330,20 @@ __global__ void __launch_bounds__(128) dgemm_small_kernel(const __grid_constant_
   const uintptr_t base = (reinterpret_cast<uintptr_t>(smem_raw) + 2047) & ~uintptr_t(2047);
   unsigned char* sm = reinterpret_cast<unsigned char*>(base);
   const uint32_t sm_base = smem_u32(sm);
-  const uint32_t full0 = sm_base + SM_STAGES * SM_STAGE_BYTES, empty0 = full0 + 8 * SM_STAGES;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const uint32_t box0 = sm_base + warp * SM_RING * SM_BOX_BYTES;  // this warp's ring
+  const uint32_t full0 = sm_base + SM_WARPS * SM_RING * SM_BOX_BYTES + 8 * SM_RING * warp;
   const int ks = blockIdx.z * k_chunk;
   const int Kz = k_chunk ? min(K - ks, k_chunk) : K;
   C += (long)blockIdx.z * c_zstride;
-  const int KT = (Kz + SM_BK - 1) / SM_BK;
+  // boxes of 16 k (the last one's rest is filled with zeros: slices are whole
+  // boxes), and this warp's steps of four k: whole boxes when there are enough
+  const int KB = (Kz + BK - 1) / BK, steps = (Kz + 3) / 4;
+  const int q4 = KB <= 2 ? (steps + SM_WARPS - 1) / SM_WARPS : (KB + SM_WARPS - 1) / SM_WARPS * 4;
+  const int step0 = min(warp * q4, steps), step1 = min(step0 + q4, steps);
+  const int kb0 = step0 >> 2, nbox = ((step1 + 3) >> 2) - kb0;
   if (tid == 0) {
-    for (int s = 0; s < SM_STAGES; ++s) {
-      mbar_init(full0 + 8 * s, 1);
-      mbar_init(empty0 + 8 * s, 4);
-    }
+    for (int i = 0; i < SM_WARPS * SM_RING; ++i) mbar_init(sm_base + SM_WARPS * SM_RING * SM_BOX_BYTES + 8 * i, 1);
     fence_barrier_init();
     prefetch_tmap(&mapA);
     prefetch_tmap(&mapB);
@@ -346,34 +352,28 @@ __global__ void __launch_bounds__(128) dgemm_small_kernel(const __grid_constant_
   if (guard && *((volatile const int*)guard) < guard_limit) return;
   if (mode == GEMM_LOWER && (long)tile_m + SM_T - 1 - tile_n < diag_off) return;
   __syncthreads();
-  // stage: two 16-wide k halves, each A (32 x 16) then B; a half past the end
-  // of k reads zeros (the map's fill), one inside another slice its values,
-  // so slices are multiples of SM_BK
-  auto issue = [&](int kt) {
-    const int st = kt % SM_STAGES;
-    const uint32_t fb_ = full0 + 8 * st;
-    mbar_arrive_expect_tx(fb_, SM_STAGE_BYTES);
-#pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      const uint32_t dA = sm_base + st * SM_STAGE_BYTES + u * SM_HALF_BYTES, dB = dA + SM_A_BYTES;
-      const int k0 = ks + kt * SM_BK + u * BK;
-      if (A_K) {
-        tma_load_2d(dA, &mapA, k0, tile_m, fb_);  // box {16 k, 32 m}
-      } else {
-        tma_load_2d(dA, &mapA, tile_m, k0, fb_);
-        tma_load_2d(dA + BK * 128, &mapA, tile_m + 16, k0, fb_);
-      }
-      if (B_K) {
-        tma_load_2d(dB, &mapB, k0, tile_n, fb_);
-      } else {
-        tma_load_2d(dB, &mapB, tile_n, k0, fb_);
-        tma_load_2d(dB + BK * 128, &mapB, tile_n + 16, k0, fb_);
-      }
+  // box i of this warp: A (32 x 16) then B
+  auto issue = [&](int i) {
+    const uint32_t fb_ = full0 + 8 * (i % SM_RING);
+    const uint32_t dA = box0 + (i % SM_RING) * SM_BOX_BYTES, dB = dA + SM_A_BYTES;
+    const int k0 = ks + (kb0 + i) * BK;
+    mbar_arrive_expect_tx(fb_, SM_BOX_BYTES);
+    if (A_K) {
+      tma_load_2d(dA, &mapA, k0, tile_m, fb_);  // box {16 k, 32 m}
+    } else {
+      tma_load_2d(dA, &mapA, tile_m, k0, fb_);
+      tma_load_2d(dA + BK * 128, &mapA, tile_m + 16, k0, fb_);
+    }
+    if (B_K) {
+      tma_load_2d(dB, &mapB, k0, tile_n, fb_);
+    } else {
+      tma_load_2d(dB, &mapB, tile_n, k0, fb_);
+      tma_load_2d(dB + BK * 128, &mapB, tile_n + 16, k0, fb_);
     }
   };
-  int issued = 0;
-  if (tid == 0)
-    for (; issued < SM_STAGES && issued < KT; ++issued) issue(issued);
+  int issued = min(SM_RING, nbox);  // lane 0's copies
+  if (lane == 0)
+    for (int i = 0; i < issued; ++i) issue(i);
   // this thread's elements of C: row tile_m + lane, columns tile_n + warp + 4 q
   const int row = tile_m + lane;
   double cv[8];
@@ -390,10 +390,8 @@ __global__ void __launch_bounds__(128) dgemm_small_kernel(const __grid_constant_
   for (int f = 0; f < 4; ++f) {
     const int ra = A_K ? (8 * f + perm8_tab(g)) : (16 * (f >> 1) + perm16_tab(f & 1, g));
     const int rb = B_K ? (8 * f + perm8_tab(g)) : (16 * (f >> 1) + perm16_tab(f & 1, g));
-    const uint32_t xa = A_K ? (uint32_t)(warp << 5) : (uint32_t)((warp << 9) | ((warp & 1) << 6));
-    const uint32_t xb = B_K ? (uint32_t)(warp << 5) : (uint32_t)((warp << 9) | ((warp & 1) << 6));
-    aoff[f] = (A_K ? base_kcontig(ra, t) : base_rcontig(ra, t)) ^ xa;
-    boff[f] = SM_A_BYTES + ((B_K ? base_kcontig(rb, t) : base_rcontig(rb, t)) ^ xb);
+    aoff[f] = A_K ? base_kcontig(ra, t) : base_rcontig(ra, t);
+    boff[f] = SM_A_BYTES + (B_K ? base_kcontig(rb, t) : base_rcontig(rb, t));
   }
   double acc[4][4][2];
 #pragma unroll
@@ -401,41 +399,39 @@ __global__ void __launch_bounds__(128) dgemm_small_kernel(const __grid_constant_
 #pragma unroll
     for (int j = 0; j < 4; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
   bool ok = true;
-  for (int kt = 0; kt < KT; ++kt) {
-    const int s = kt % SM_STAGES;
-    if (!mbar_wait(full0 + 8 * s, (kt / SM_STAGES) & 1, err, 12)) { ok = false; break; }
-    const uint32_t tS = sm_base + s * SM_STAGE_BYTES;
-    double a[2][4], b[2][4];
+  for (int i = 0; i < nbox; ++i) {
+    ok = __all_sync(0xffffffffu, mbar_wait(full0 + 8 * (i % SM_RING), (i / SM_RING) & 1, err, 12));
+    if (!ok) break;
+    const uint32_t tS = box0 + (i % SM_RING) * SM_BOX_BYTES;
+    const int lo = step0 - 4 * (kb0 + i), hi = step1 - 4 * (kb0 + i);  // this warp's steps of the box
 #pragma unroll
-    for (int u = 0; u < 2; ++u)
+    for (int kk = 0; kk < BK / 4; ++kk) {
+      if (kk < lo || kk >= hi) continue;
+      double a[4], b[4];
 #pragma unroll
       for (int f = 0; f < 4; ++f) {
-        a[u][f] = lds_f64(tS + u * SM_HALF_BYTES + aoff[f]);
-        b[u][f] = lds_f64(tS + u * SM_HALF_BYTES + boff[f]);
+        a[f] = lds_f64((tS + aoff[f]) ^ kk_xor<A_K>(kk));
+        b[f] = lds_f64((tS + boff[f]) ^ kk_xor<B_K>(kk));
       }
 #pragma unroll
-    for (int u = 0; u < 2; ++u)
+      for (int x = 0; x < 4; ++x)
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) dmma_884(acc[i][j][0], acc[i][j][1], a[u][i], b[u][j]);
-    if (kt + SM_STAGES < KT) {
-      // this stage is refilled (see dgemm_tma_kernel for the fences)
+        for (int y = 0; y < 4; ++y) dmma_884(acc[x][y][0], acc[x][y][1], a[x], b[y]);
+    }
+    if (i + SM_RING < nbox) {
+      // this box is refilled (see dgemm_tma_kernel for the fences)
       __threadfence_block();
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       __syncwarp();
-      if (lane == 0) mbar_arrive(empty0 + 8 * s);
-      if (tid == 0) {
-        if (!mbar_wait(empty0 + 8 * s, (kt / SM_STAGES) & 1, err, 11)) { ok = false; break; }
-        issue(issued);
-        ++issued;
-      }
+      if (lane == 0) issue(i + SM_RING);
+      ++issued;
     }
   }
   if (!__syncthreads_and(ok ? 1 : 0)) {
-    if (tid == 0)
-      for (int kt = (issued > SM_STAGES ? issued - SM_STAGES : 0); kt < issued; ++kt)
-        mbar_wait(full0 + 8 * (kt % SM_STAGES), (kt / SM_STAGES) & 1, nullptr, 0);
+    // a wait ran out: each warp drains (bounded) the copies it has in flight
+    if (!ok && lane == 0)
+      for (int i = max(0, issued - SM_RING); i < issued; ++i)
+        mbar_wait(full0 + 8 * (i % SM_RING), (i / SM_RING) & 1, nullptr, 0);
     return;
   }
   chain_next();
@@ -827,7 +823,7 @@ int gemm_f64(cudaStream_t st, bool ta, bool tb, long m, long n, long k, double a
     if (capped) S = std::min<long>(std::max<long>(S, (k + kmax - 1) / kmax), 64);
   }
   if (S > 1) {
-    kc = ((k + S - 1) / S + SM_BK - 1) / SM_BK * SM_BK;
+    kc = ((k + S - 1) / S + 2 * BK - 1) / (2 * BK) * (2 * BK);
     S = (k + kc - 1) / kc;
   }
   if (S > 1) {
