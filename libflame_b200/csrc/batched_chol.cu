@@ -5,7 +5,8 @@
 // Semantics of FLA_Chol per matrix (src/lapack/dec/chol/front/flamec/
 // FLA_Chol.c:16-29): lower triangle only, stopping at the first pivot that is
 // not > 0 (NaN included), its zero-based column reported; a matrix that fails
-// keeps its right-hand sides.
+// holds L in the columns before it (of the failing panel, the diagonal block's
+// rows), the failing pivot at its place, and keeps its right-hand sides.
 //
 // Right-looking in panels of 32 columns, in place (the matrices of the
 // resident CTAs stay in L2):
@@ -173,7 +174,22 @@ __global__ void __launch_bounds__(NT, ChB<NT>::MINB) chol_batched_f64_kernel(Bat
       }
       __syncthreads();
       if (s_fail >= 0) {
-        fail = j + s_fail;
+        // as far as the leading minor goes: the diagonal block's columns before
+        // the failing one, and what is left of its others
+        const int f = s_fail;
+        for (int e = tid; e < w * w; e += NT) {
+          const int r = e % w, c = e / w;
+          if (r < c) continue;
+          double* d = G + (long)(j + r) + (long)(j + c) * ld;
+          if (c < f) {
+            *d = P[r + c * LD];
+          } else {
+            double v = *d;
+            for (int k = 0; k < f; ++k) v = fma(-P[r + k * LD], P[c + k * LD], v);
+            *d = v;
+          }
+        }
+        fail = j + f;
         break;
       }
       // ---- back to memory, and the right-hand sides' entries
