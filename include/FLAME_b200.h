@@ -133,10 +133,12 @@ FLA_Error     FLA_B200_Chol_batched_logdet( int count, const int* n, double** A,
 /* Autotuner of the batched kernels: per size bin (orders 1-32, 33-64,
  * 65-128, 129-256, 257-512) times the panel widths 8, 16, 24, 32 on
  * `samples` scratch matrices and keeps the fastest for later calls on this
- * device (lu: 0 Cholesky, 1 LU; f64: 0 FP32, 1 FP64).  times (optional, 20
- * doubles) receives the bin x width timings in ms. */
+ * device (lu: 0 Cholesky, 1 LU; f64: 0 FP32, 1 FP64).  The FP64 kernels have
+ * one panel width, 32: it is timed and nothing changes.  times (optional, 20
+ * doubles) receives the bin x width timings in ms (FP64: the same for every
+ * width). */
 int           FLA_B200_batched_tune( int lu, int f64, int samples, double* times );
-/* Panel width the batched kernels use for order n. */
+/* Panel width the batched kernels use for order n (FP64: 32). */
 int           FLA_B200_batched_nb( int lu, int f64, int n );
 
 /* ---- Differentiation (no counterpart in the reference) ----

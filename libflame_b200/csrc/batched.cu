@@ -694,17 +694,19 @@ int launch_batched(bool lu, BatchArgs<T> args, cudaStream_t st) {
   }
 }
 
-// per-device panel width by matrix order (autotuned), index 0..BMAXN
+// Panel width of the FP32 kernels by matrix order (autotuned), index 0..BMAXN.
+// The FP64 kernels' panels are 32 columns wide for every order: their register
+// and tile layouts are built on that width.
 struct NbTable {
   std::vector<int> host;
   int* dev = nullptr;
-  bool tuned = false;
 };
-NbTable g_nb[2][2];  // [lu][fp64]
+NbTable g_nb[2];  // [lu]
 std::mutex g_nb_mu;
+constexpr int NB_F64 = 32;
 
-int* nb_table(bool lu, bool f64) {
-  NbTable& t = g_nb[lu ? 1 : 0][f64 ? 1 : 0];
+int* nb_table(bool lu) {
+  NbTable& t = g_nb[lu ? 1 : 0];
   if (!t.dev) {
     t.host.assign(BMAXN + 1, 32);
     for (int n = 0; n <= BMAXN; ++n) t.host[n] = n <= 32 ? 16 : 32;  // default before tuning
@@ -745,8 +747,7 @@ int batched_factor(bool lu, int count, const int* h_n, T** d_A, const long* d_ld
   a.info = d_info;
   a.logdet = d_logdet;
   a.err = ctx().d_status + ST_ERROR;
-  a.nb_of_size = nb_table(lu, sizeof(T) == 8);
-  if (!a.nb_of_size) return FLA_FAILURE;
+  if (sizeof(T) == 4 && !(a.nb_of_size = nb_table(lu))) return FLA_FAILURE;
   // the host order must stay valid until the copy is done
   FB_CK(cudaStreamSynchronize(st));
   if constexpr (sizeof(T) == 8) {
@@ -785,8 +786,8 @@ template int batched_factor<float>(bool, int, const int*, float**, const long*, 
 // fastest; bins are the orders 1-32, 33-64, 65-128, 129-256, 257-512.
 int batched_tune(bool lu, bool f64, int samples_per_bin, double* times_out) {
   std::lock_guard<std::mutex> lk(g_nb_mu);
-  NbTable& t = g_nb[lu ? 1 : 0][f64 ? 1 : 0];
-  if (!nb_table(lu, f64)) return FLA_FAILURE;
+  NbTable& t = g_nb[lu ? 1 : 0];
+  if (!f64 && !nb_table(lu)) return FLA_FAILURE;
   const int bins[6] = {1, 33, 65, 129, 257, 513};
   const int cands[4] = {8, 16, 24, 32};
   cudaStream_t st = ctx().stream;
@@ -829,11 +830,18 @@ int batched_tune(bool lu, bool f64, int samples_per_bin, double* times_out) {
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
     float best = 1e30f;
-    int bestnb = t.host[hi];
+    int bestnb = f64 ? NB_F64 : t.host[hi];
     for (int ci = 0; ci < 4; ++ci) {
       const int c = cands[ci];
-      for (int nn = lo; nn <= hi; ++nn) t.host[nn] = c;
-      FB_CK(cudaMemcpy(t.dev, t.host.data(), sizeof(int) * (BMAXN + 1), cudaMemcpyHostToDevice));
+      if (f64) {  // one width: every column of `times` holds its time
+        if (ci > 0) {
+          if (times_out) times_out[b * 4 + ci] = times_out[b * 4];
+          continue;
+        }
+      } else {
+        for (int nn = lo; nn <= hi; ++nn) t.host[nn] = c;
+        FB_CK(cudaMemcpy(t.dev, t.host.data(), sizeof(int) * (BMAXN + 1), cudaMemcpyHostToDevice));
+      }
       float ms = 1e30f;
       for (int rep = 0; rep < 2; ++rep) {
         if (batched_fill_dominant(f64, cnt, dA, dn, dld, st) != FLA_SUCCESS) return FLA_FAILURE;
@@ -855,18 +863,20 @@ int batched_tune(bool lu, bool f64, int samples_per_bin, double* times_out) {
         bestnb = c;
       }
     }
-    for (int nn = lo; nn <= hi; ++nn) t.host[nn] = bestnb;
-    FB_CK(cudaMemcpy(t.dev, t.host.data(), sizeof(int) * (BMAXN + 1), cudaMemcpyHostToDevice));
+    if (!f64) {
+      for (int nn = lo; nn <= hi; ++nn) t.host[nn] = bestnb;
+      FB_CK(cudaMemcpy(t.dev, t.host.data(), sizeof(int) * (BMAXN + 1), cudaMemcpyHostToDevice));
+    }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
   }
-  t.tuned = true;
   return FLA_SUCCESS;
 }
 
 int batched_nb(bool lu, bool f64, int n) {
-  NbTable& t = g_nb[lu ? 1 : 0][f64 ? 1 : 0];
-  if (t.host.empty()) nb_table(lu, f64);
+  if (f64) return NB_F64;
+  NbTable& t = g_nb[lu ? 1 : 0];
+  if (t.host.empty()) nb_table(lu);
   return t.host.empty() ? 0 : t.host[std::min(std::max(n, 0), BMAXN)];
 }
 
@@ -1017,8 +1027,8 @@ FLA_Error FLA_B200_LU_piv_batched_f32(int count, const int* n, float** A, const 
 // Autotuner of the batched kernels: for each size bin (orders 1-32, 33-64,
 // 65-128, 129-256, 257-512) times the panel widths 8, 16, 24, 32 on
 // `samples` scratch matrices and keeps the fastest for later calls on this
-// device.  times (optional, 20 doubles) receives the bin x width timings
-// in ms.
+// device (FP32; the FP64 kernels have one width, 32, which is timed and left).
+// times (optional, 20 doubles) receives the bin x width timings in ms.
 int FLA_B200_batched_tune(int lu, int f64, int samples, double* times) {
   if (!fb::ctx().initialized) FLA_Init();
   return fb::batched_tune(lu != 0, f64 != 0, samples, times);

@@ -17,7 +17,7 @@ struct BatchArgs {
   T** B = nullptr;
   const long* ldb = nullptr;
   int* info = nullptr;          // per matrix: -1 or the failing / first zero-pivot column
-  const int* nb_of_size = nullptr;  // panel width by order
+  const int* nb_of_size = nullptr;  // panel width by order (FP32)
   T* logdet = nullptr;          // optional: per matrix sum_i log L(i, i) (FP64 Cholesky)
   int* err = nullptr;           // status word for wait timeouts (FP64 Cholesky)
 };
