@@ -239,10 +239,12 @@ int apply_q_blocks(DMat U, long k, DMat T, int b_alg, int S, DMat B, bool transp
   // Gram slices per super-block: about two CTAs per SM over all of them, no
   // more than slabs
   const int nz = (int)std::max<long>(1, std::min<long>(std::min<long>(2L * sms / nsb, 16), (m + GK - 1) / GK));
-  constexpr long kMaxSlices = 32;  // the small kernel adds them
+  // Slices of U2^T B2: no more than the split fills the GPU with (four 64-column
+  // tiles per SM), and at most 32: the small kernel adds them
+  const long max_slices = std::max<long>(1, std::min<long>(32, 4L * sms / (((S + 127) / 128) * ((nr + 63) / 64))));
   const long ldw = (S + 1) & ~1L;
   const size_t n_gram = (size_t)nsb * nz * AS * AS, n_t = (size_t)nsb * S * (S + 1);
-  const size_t n_p = (size_t)kMaxSlices * ldw * nr;
+  const size_t n_p = (size_t)max_slices * ldw * nr;
   double* ws = (double*)ws_get(WS_QR_W, sizeof(double) * (std::max(n_gram, n_p) + n_t + (size_t)nsb * S * S +
                                                           (size_t)ldw * nr + 8));
   if (!ws) return FLA_FAILURE;
@@ -278,7 +280,7 @@ int apply_q_blocks(DMat U, long k, DMat T, int b_alg, int S, DMat B, bool transp
     if (M2 > 0) {
       sp.p = P;
       sp.elems = n_p;
-      sp.max_slices = kMaxSlices;
+      sp.max_slices = max_slices;
       sp.slices = &slices;
       if (gemm_f64(st, true, false, s, nr, M2, 1.0, Uq + h, U.ld, Bq + h, B.ld, 0.0, nullptr, 0, GEMM_FULL, 0, nullptr,
                    0, 0, &sp) != FLA_SUCCESS)

@@ -1,0 +1,46 @@
+"""Device memory that calls keep for later ones (until FLA_Finalize)."""
+import os
+import subprocess
+import sys
+
+import pytest
+
+from conftest import ROOT
+
+pytestmark = pytest.mark.gpu
+
+HEAD = """
+import sys
+sys.path.insert(0, %r)
+import torch, libflame_b200 as F
+F.init()
+def colmajor(m, n, fill=0.0):
+    return torch.full((n, m), fill, dtype=torch.float64, device="cuda").t()
+def held():
+    torch.cuda.synchronize()
+    return torch.cuda.mem_get_info()[0]
+""" % ROOT
+
+
+def _run(code):
+    """The last printed number of a fresh process (workspaces only grow)."""
+    p = subprocess.run([sys.executable, "-c", HEAD + code], capture_output=True, text=True, timeout=300, cwd=ROOT,
+                       env=dict(os.environ))
+    assert p.returncode == 0, p.stderr[-2000:]
+    return int(p.stdout.split()[-1])
+
+
+def test_apply_q_many_columns(cuda, flame):
+    """512 x 256 reflectors on 16384 columns (64 MB): the slices of the split
+    products take a few times a 128 x 16384 block (16 MB), not 32 times."""
+    grown = _run("""
+A = torch.randn((256, 512), dtype=torch.float64, device="cuda").t()
+T = colmajor(32, 256)
+assert F.qr_ut(A, T) == F.FLA_SUCCESS
+B = torch.randn((16384, 512), dtype=torch.float64, device="cuda").t()
+assert F.apply_q_ut(A, T, B[:, :1], F.FLA_CONJ_TRANSPOSE) == F.FLA_SUCCESS
+a = held()
+assert F.apply_q_ut(A, T, B, F.FLA_CONJ_TRANSPOSE) == F.FLA_SUCCESS
+print(a - held())
+""")
+    assert grown < 128 << 20, grown
