@@ -237,12 +237,16 @@ bool g_adj_attr = false;
 
 // Scratch of chol_adjoint_dev for order n, in doubles: the inverses of all
 // diagonal blocks, two W (ldw x AB each: S over Cbar, of two consecutive
-// blocks), the product Cbar^T C, and the partial products of `splits` slices
-// of an AB-row GEMM for either stream.
+// blocks), the product Cbar^T C, and room for either stream's partial products:
+// `splits` slices of an AB-row GEMM, but no more than a split that fills the
+// GPU (four 64 x 64 tiles per SM) ever has.
 static long adj_ldw(long n) { return (n + AB + 1) & ~1L; }
+static size_t adj_split_elems(long n, int splits) {
+  return std::min((size_t)splits * AB * (size_t)(n + AB), (size_t)4 * ctx().num_sms * 64 * 64);
+}
 size_t chol_adjoint_scratch(long n, int splits) {
   const size_t nblk = (size_t)((n + AB - 1) / AB);
-  return nblk * AB * AB + 2 * (size_t)adj_ldw(n) * AB + (size_t)AB * AB + 2 * (size_t)splits * AB * (size_t)(n + AB);
+  return nblk * AB * AB + 2 * (size_t)adj_ldw(n) * AB + (size_t)AB * AB + 2 * adj_split_elems(n, splits);
 }
 
 // In place over Lb (lower triangle); L lower Cholesky factor; n x n, ld.
@@ -269,7 +273,7 @@ int chol_adjoint_dev(const double* L, double* Lb, long ld, long n, cudaStream_t 
   double* G = W2 + 2 * (size_t)ldw * AB;
   GemmSplit sp_chain, sp_rest;
   sp_chain.p = G + (size_t)AB * AB;
-  sp_chain.elems = sp_rest.elems = (size_t)splits * AB * (size_t)(n + AB);
+  sp_chain.elems = sp_rest.elems = adj_split_elems(n, splits);
   sp_rest.p = sp_chain.p + sp_chain.elems;
   auto Lat = [&](long i, long j) { return L + i + j * ld; };
   auto Bat = [&](long i, long j) { return Lb + i + j * ld; };

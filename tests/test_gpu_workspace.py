@@ -44,3 +44,18 @@ assert F.apply_q_ut(A, T, B, F.FLA_CONJ_TRANSPOSE) == F.FLA_SUCCESS
 print(a - held())
 """)
     assert grown < 128 << 20, grown
+
+
+def test_adjoint_scratch(cuda, flame):
+    """n = 8192: the inverses of the diagonal blocks, two block columns and two
+    splits' partial products, 65 MB in all, rather than 32 KB per row."""
+    grown = _run("""
+n = 8192
+L, Lb = colmajor(n, n), colmajor(n, n, 1.0)
+L.diagonal().fill_(2.0)
+assert F.chol_adjoint(L[:256, :256], Lb[:256, :256]) == F.FLA_SUCCESS
+a = held()
+assert F.chol_adjoint(L, Lb) == F.FLA_SUCCESS
+print(a - held())
+""")
+    assert grown < 128 << 20, grown
