@@ -422,11 +422,17 @@ int lub_launch(const BatchArgs<double>& a, double* ws, size_t stride, int grid, 
 int batched_lu_f64(BatchArgs<double> a, int big, int maxn, cudaStream_t st) {
   Context& cx = ctx();
   const int sms = cx.num_sms;
-  const int g_big = std::min(sms, big), g_small = std::min(2 * sms, a.count - big);
+  int g_big = std::min(sms, big), g_small = std::min(2 * sms, a.count - big);
   const size_t s_big = (lub_ws(maxn) + 1) & ~size_t(1);
   const size_t s_small = (lub_ws(std::min(maxn, 256)) + 1) & ~size_t(1);
-  double* ws = (double*)ws_get(WS_REPACK, sizeof(double) * (s_big * g_big + s_small * g_small));
-  if (!ws) return FLA_FAILURE;
+  // a CTA's copy is 2.2 MB at order 512, 0.5 GB in all for a full GPU; with
+  // less memory to be had, fewer CTAs take the matrices
+  double* ws;
+  while (!(ws = (double*)ws_get(WS_REPACK, sizeof(double) * (s_big * g_big + s_small * g_small)))) {
+    if (g_big <= 1 && g_small <= 1) return FLA_FAILURE;
+    g_big = (g_big + 1) / 2;
+    g_small = (g_small + 1) / 2;
+  }
   const int ps = prof_begin(st);
   if (g_small > 0 && g_big > 0) {
     // beside the large ones: their CTAs take the SMs the others leave
