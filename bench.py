@@ -207,6 +207,17 @@ def lu_config(n, world):
             "l2": "inputs (2 GiB at n=16384) larger than L2; the per-step restore of A also flushes L2"}
 
 
+REF_OPENBLAS = os.path.join(ROOT, "oracle", "_ref", "libflame_ref_openblas.so")
+
+
+def reference_missing():
+    """Why the reference over OpenBLAS cannot be run here; None if it can."""
+    if os.path.exists(REF_OPENBLAS):
+        return None
+    return "%s has not been built (oracle/build_ref.py builds it from the reference's sources)" % os.path.relpath(
+        REF_OPENBLAS, ROOT)
+
+
 def reference_lu_openblas(n, nthreads):
     """The reference libflame's flat FLA_LU_piv over OpenBLAS
     (oracle/_ref/libflame_ref_openblas.so) on `nthreads` host threads, one
@@ -244,6 +255,9 @@ def pick_reference_n(n_full, nthreads, runs, budget_s):
 
 def run_reference(args, rank):
     if rank != 0:
+        return
+    if reference_missing():
+        print(json.dumps({"impl": "reference", "unavailable": reference_missing()}), flush=True)
         return
     nthreads = host_threads()
     n, _ = pick_reference_n(args.n, nthreads, args.warmup + args.steps, 200.0)
@@ -384,6 +398,8 @@ def reference_ir_cpu(kind, A, B):
     """The reference's own mixed-precision drivers (dsposv_ / dsgesv_: FP32
     factorization, FP64 refinement) beside its FP64 solvers (dposv_ /
     dgesv_), all from the reference built over OpenBLAS, on the host cores."""
+    if reference_missing():
+        return {"unavailable": reference_missing()}
     sys.path.insert(0, os.path.join(ROOT, "oracle"))
     import refbind as R
     nthreads = host_threads()
