@@ -117,7 +117,6 @@ enum WsSlot : int {
   WS_MISC2,
   WS_LP0,           // mixed-precision solvers: low-precision factor
   WS_LP1,           //   packed 16-bit operands
-  WS_LP2,
   WS_LP3,           //   FP64 panel / inverses
   WS_LP4,           //   inverse blocks kept for the correction solves
   WS_IR0,           //   refinement vectors (FP64 / FP32)
@@ -281,10 +280,6 @@ int tri_inverse_blocks_bs(const double* T, long ldt, long n, int bs, bool lower,
                           cudaStream_t st);
 // X := inv(T), T b x b triangular (lower or upper; unit diagonal if unit).
 int tri_inverse(const double* T, long ldt, int b, bool lower, bool unit, double* X, long ldx, cudaStream_t st);
-// X := X inv(op(T)) ^T row by row: every row x of the m x b block X is
-// replaced by the solution of op(T) y = x (b <= 128).
-int trsm_right_block(const double* T, long ldt, double* X, long ldx, long m, int b, bool lower, bool trans,
-                     bool unit, cudaStream_t st);
 // dst := src^T for an m x n src (dst n x m); upper_only writes i <= j only.
 int transpose_dev(const double* src, long lds, double* dst, long ldd, long m, long n, bool upper_only,
                   cudaStream_t st);
@@ -310,11 +305,5 @@ int potrf_diag_dev(double* A, long ld, int b, int gcol, cudaStream_t st);
 // LU panel on the transposed matrix: the M x w panel of A whose element
 // (i, j) is at P[i * ld + j] (rows of A are the columns of AT).
 int lu_panel_factor_t(double* P, long ld, long M, int w, int* d_piv, int gcol, cudaStream_t st);
-// LU panel: factor the M x w panel at P with partial pivoting (M >= w);
-// d_piv gets w relative pivots; gcol = global index of the first column.
-int lu_panel_factor(double* P, long ld, long M, int w, int* d_piv, int gcol, cudaStream_t st);
-// X := X inv(L)^T for an m x b block (b <= 128); no-op once *guard != INT_MAX.
-int trsm_right_lt_block(const double* L, long ldl, double* X, long ldx, long m, int b, const int* guard,
-                        cudaStream_t st);
 
 }  // namespace fb

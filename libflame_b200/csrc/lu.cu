@@ -5,7 +5,7 @@
 // Blocked right-looking algorithm with the reference's structure
 // (src/lapack/dec/lu/piv/vars/flamec/FLA_LU_piv_blk_var5.c:13-114):
 //   for each block of nb columns:
-//     [A11;A21], p1 := LU_piv([A11;A21])   lu_panel_factor (lu_panel.cu)
+//     [A11;A21], p1 := LU_piv([A11;A21])   lu_panel_factor_t (lu_panel.cu)
 //     pivot [A10;A20] and [A12;A22]         laswp_apply_kernel
 //     A12 := inv(tril_unit(A11)) A12         forward substitution, one launch
 //                                            (rlt_kernel, rlt.cu)
@@ -288,38 +288,6 @@ __global__ void __launch_bounds__(256) laswp_apply_kernel(T* A, long ld, int row
   }
 }
 
-__global__ void laswp_kernel(double* A, long ld, int row0, const int* __restrict__ piv, int npiv,
-                             int c0, int n0, int c1, int n1, int reverse) {
-  extern __shared__ int sp[];
-  for (int i = threadIdx.x; i < npiv; i += blockDim.x) sp[i] = piv[i];
-  __syncthreads();
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= n0 + n1) return;
-  const int col = t < n0 ? c0 + t : c1 + (t - n0);
-  double* a = A + (long)col * ld;
-  if (!reverse) {
-    for (int i = 0; i < npiv; ++i) {
-      const int p = sp[i];
-      if (p != 0) {
-        const long r1 = row0 + i, r2 = r1 + p;
-        const double x = a[r1];
-        a[r1] = a[r2];
-        a[r2] = x;
-      }
-    }
-  } else {
-    for (int i = npiv - 1; i >= 0; --i) {
-      const int p = sp[i];
-      if (p != 0) {
-        const long r1 = row0 + i, r2 = r1 + p;
-        const double x = a[r1];
-        a[r1] = a[r2];
-        a[r2] = x;
-      }
-    }
-  }
-}
-
 bool g_attrs = false;
 void set_attrs() {
   if (g_attrs) return;
@@ -348,19 +316,15 @@ int laswp_blocked(T* A, long ld, int row0, const int* d_piv, int npiv, int c0, i
   return FLA_SUCCESS;
 }
 
+// At most LASWP_MAXP interchanges.
 int laswp_dev(double* A, long ld, int row0, const int* d_piv, int npiv, int c0, int n0, int c1,
               int n1, bool reverse, cudaStream_t st) {
-  const int ncols = n0 + n1;
-  if (ncols <= 0 || npiv <= 0) return FLA_SUCCESS;
-  if (npiv <= LASWP_MAXP) return laswp_blocked<double>(A, ld, row0, d_piv, npiv, c0, n0, c1, n1, reverse, false, st);
-  const int threads = 128;
-  const int ps = prof_begin(st);
-  laswp_kernel<<<(ncols + threads - 1) / threads, threads, npiv * sizeof(int), st>>>(
-      A, ld, row0, d_piv, npiv, c0, n0, c1, n1, reverse ? 1 : 0);
-  prof_end(ps, st, PROF_SWAP, 0.0);
-  count_launch();
-  FB_CK(cudaGetLastError());
-  return FLA_SUCCESS;
+  if (n0 + n1 <= 0 || npiv <= 0) return FLA_SUCCESS;
+  if (npiv > LASWP_MAXP) {
+    set_last_error("row interchanges: more than one block of them");
+    return FLA_FAILURE;
+  }
+  return laswp_blocked<double>(A, ld, row0, d_piv, npiv, c0, n0, c1, n1, reverse, false, st);
 }
 
 // Row interchanges on a transposed matrix (see laswp_apply_kernel<T, true>),

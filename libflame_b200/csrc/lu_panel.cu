@@ -23,7 +23,7 @@
 // hardware, so the leaf can run on a second stream beside the trailing
 // update without any co-residency assumption, and the barrier is not a spin.
 //
-// Recursion (lu_panel_factor): a panel too wide for the cluster's shared
+// Recursion (lu_panel_factor_t): a panel too wide for the cluster's shared
 // memory is split in two halves: factor the left half, swap the right half's
 // rows, solve its top block, update the rest with the DMMA GEMM engine,
 // factor the lower right half, and swap the left half's lower rows.  The
@@ -75,9 +75,8 @@ __host__ __device__ inline size_t leaf_smem_bytes(int lds, int w, int C) {
   return sizeof(double) * ((size_t)lds * w + 2 * (size_t)C * w + 2 * C + 2 * w) + sizeof(int) * 2 * C + 64;
 }
 
-// RM: the panel is stored transposed (element (i, col) at P[i * ld + col],
-// rows of A being columns of A^T); otherwise column-major.
-template <bool RM>
+// The panel is stored transposed (element (i, col) at P[i * ld + col], rows of A
+// being columns of A^T).
 __global__ void __launch_bounds__(LEAF_THREADS, 1) lu_leaf_cluster_kernel(LeafArgs a) {
   extern __shared__ double S[];
   __shared__ double s_rv[LEAF_THREADS / 32];
@@ -97,31 +96,26 @@ __global__ void __launch_bounds__(LEAF_THREADS, 1) lu_leaf_cluster_kernel(LeafAr
 
   const int r0 = c * a.R;
   const int rows = max(0, min(a.R, a.M - r0));
-  if (RM) {
-    // eight independent loads in flight per thread
-    const int tot = rows * w;
-    for (int e0 = tid; e0 < tot; e0 += 8 * LEAF_THREADS) {
-      double v[8];
+  // eight independent loads in flight per thread
+  const int tot = rows * w;
+  for (int e0 = tid; e0 < tot; e0 += 8 * LEAF_THREADS) {
+    double v[8];
 #pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        const int e = e0 + k * LEAF_THREADS;
-        if (e < tot) {
-          const int i = e / w, col = e - i * w;
-          v[k] = a.P[(long)(r0 + i) * a.ld + col];
-        }
-      }
-#pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        const int e = e0 + k * LEAF_THREADS;
-        if (e < tot) {
-          const int i = e / w, col = e - i * w;
-          slab[i + col * lds] = v[k];
-        }
+    for (int k = 0; k < 8; ++k) {
+      const int e = e0 + k * LEAF_THREADS;
+      if (e < tot) {
+        const int i = e / w, col = e - i * w;
+        v[k] = a.P[(long)(r0 + i) * a.ld + col];
       }
     }
-  } else {
-    for (int col = 0; col < w; ++col)
-      for (int i = tid; i < rows; i += LEAF_THREADS) slab[i + col * lds] = a.P[(long)(r0 + i) + (long)col * a.ld];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const int e = e0 + k * LEAF_THREADS;
+      if (e < tot) {
+        const int i = e / w, col = e - i * w;
+        slab[i + col * lds] = v[k];
+      }
+    }
   }
   __syncthreads();
 
@@ -284,14 +278,9 @@ __global__ void __launch_bounds__(LEAF_THREADS, 1) lu_leaf_cluster_kernel(LeafAr
     }
   }
   __syncthreads();
-  if (RM) {
-    for (int e = tid; e < rows * w; e += LEAF_THREADS) {
-      const int i = e / w, col = e - i * w;
-      a.P[(long)(r0 + i) * a.ld + col] = slab[i + col * lds];
-    }
-  } else {
-    for (int col = 0; col < w; ++col)
-      for (int i = tid; i < rows; i += LEAF_THREADS) a.P[(long)(r0 + i) + (long)col * a.ld] = slab[i + col * lds];
+  for (int e = tid; e < rows * w; e += LEAF_THREADS) {
+    const int i = e / w, col = e - i * w;
+    a.P[(long)(r0 + i) * a.ld + col] = slab[i + col * lds];
   }
   if (c == 0 && tid == 0 && first_null >= 0) atomicMin(a.info, a.gcol + first_null);
 }
@@ -617,10 +606,9 @@ int leaf_setup() {
   if (g_leaf.ready) return FLA_SUCCESS;
   Context& cx = ctx();
   g_leaf.smem_cap = std::min<size_t>(cx.smem_optin, 227 * 1024) - 1024;
-  for (auto kern : {lu_leaf_cluster_kernel<false>, lu_leaf_cluster_kernel<true>}) {
-    FB_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g_leaf.smem_cap));
-    FB_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-  }
+  FB_CK(cudaFuncSetAttribute(lu_leaf_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)g_leaf.smem_cap));
+  FB_CK(cudaFuncSetAttribute(lu_leaf_cluster_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
   // Largest cluster (16, else 8, 4 ...) that can be resident with a full
   // shared-memory slab per CTA.
   g_leaf.max_cluster = 1;
@@ -637,7 +625,7 @@ int leaf_setup() {
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     int nclusters = 0;
-    if (cudaOccupancyMaxActiveClusters(&nclusters, lu_leaf_cluster_kernel<false>, &cfg) == cudaSuccess &&
+    if (cudaOccupancyMaxActiveClusters(&nclusters, lu_leaf_cluster_kernel, &cfg) == cudaSuccess &&
         nclusters > 0) {
       g_leaf.max_cluster = cs;
       break;
@@ -771,7 +759,7 @@ bool leaf_geometry(long M, int w, int* C, int* R, int* lds, size_t* smem) {
   return false;
 }
 
-int leaf_launch(double* P, long ld, long M, int w, int* d_piv, int gcol, bool rm, cudaStream_t st) {
+int leaf_launch(double* P, long ld, long M, int w, int* d_piv, int gcol, cudaStream_t st) {
   int C = 0, R = 0, lds = 0;
   size_t smem = 0;
   if (!leaf_geometry(M, w, &C, &R, &lds, &smem)) {
@@ -802,10 +790,7 @@ int leaf_launch(double* P, long ld, long M, int w, int* d_piv, int gcol, bool rm
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   const int ps = prof_begin(st);
-  if (rm)
-    FB_CK(cudaLaunchKernelEx(&cfg, lu_leaf_cluster_kernel<true>, la));
-  else
-    FB_CK(cudaLaunchKernelEx(&cfg, lu_leaf_cluster_kernel<false>, la));
+  FB_CK(cudaLaunchKernelEx(&cfg, lu_leaf_cluster_kernel, la));
   prof_end(ps, st, PROF_PANEL, 0.0);
   count_launch();
   return FLA_SUCCESS;
@@ -813,37 +798,11 @@ int leaf_launch(double* P, long ld, long M, int w, int* d_piv, int gcol, bool rm
 
 }  // namespace
 
-// Factor the M x w panel at P (ld) with partial pivoting; d_piv receives w
-// relative pivots; gcol is the global index of the panel's first column.
-int lu_panel_factor(double* P, long ld, long M, int w, int* d_piv, int gcol, cudaStream_t st) {
-  if (leaf_setup() != FLA_SUCCESS) return FLA_FAILURE;
-  if (w <= 0 || M <= 0) return FLA_SUCCESS;
-  int C, R, lds;
-  size_t smem;
-  if (leaf_geometry(M, w, &C, &R, &lds, &smem) || w <= 2) return leaf_launch(P, ld, M, w, d_piv, gcol, false, st);
-  // split: left half a multiple of 2 columns (keeps 16-byte alignment)
-  const int w1 = std::max(2, (w / 2) & ~1);
-  const int w2 = w - w1;
-  if (lu_panel_factor(P, ld, M, w1, d_piv, gcol, st) != FLA_SUCCESS) return FLA_FAILURE;
-  double* P12 = P + (long)w1 * ld;
-  if (laswp_dev(P, ld, 0, d_piv, w1, w1, w2, 0, 0, false, st) != FLA_SUCCESS) return FLA_FAILURE;
-  if (trsm_block(P, ld, P12, ld, w1, w2, true, false, true, st) != FLA_SUCCESS) return FLA_FAILURE;
-  if (M > w1) {
-    if (gemm_f64(st, false, false, M - w1, w2, w1, -1.0, P + w1, ld, P12, ld, 1.0, P12 + w1, ld) != FLA_SUCCESS)
-      return FLA_FAILURE;
-    if (lu_panel_factor(P12 + w1, ld, M - w1, w2, d_piv + w1, gcol + w1, st) != FLA_SUCCESS) return FLA_FAILURE;
-    if (laswp_dev(P, ld, w1, d_piv + w1, (int)std::min<long>(w2, M - w1), 0, w1, 0, 0, false, st) != FLA_SUCCESS)
-      return FLA_FAILURE;
-  }
-  return FLA_SUCCESS;
-}
-
-
-// The same recursion on a panel stored transposed (element (i, j) of the
-// panel at P[i * ld + j]): row interchanges move contiguous pieces of
-// columns of A^T, the top-right solve is a row-wise solve with L11 (held as
-// the upper triangle L11^T), and the update is A22^T -= U12^T A21^T.
-// Panel recursion in which every leaf is register-resident and applies its
+// Panel recursion on the transposed storage (element (i, j) of the panel at
+// P[i * ld + j]): row interchanges move contiguous pieces of columns of A^T, the
+// top-right solve is a row-wise solve with L11 (held as the upper triangle
+// L11^T), and the update is A22^T -= U12^T A21^T.
+// Here the form in which every leaf is register-resident and applies its
 // row interchanges to the other columns of the panel itself (pl columns left
 // of this sub-panel, pr right of it): the joins need no interchange launches.
 int panel_rec_reg(double* P, long ld, long M, int w, int* d_piv, int gcol, int pl, int pr, cudaStream_t st) {
@@ -883,7 +842,7 @@ int lu_panel_factor_t(double* P, long ld, long M, int w, int* d_piv, int gcol, c
   int C, R, lds;
   size_t smem;
   if (rleaf_geometry(M, w, &C, &R)) return rleaf_launch(P, ld, M, w, d_piv, gcol, st);
-  if (leaf_geometry(M, w, &C, &R, &lds, &smem) || w <= 2) return leaf_launch(P, ld, M, w, d_piv, gcol, true, st);
+  if (leaf_geometry(M, w, &C, &R, &lds, &smem) || w <= 2) return leaf_launch(P, ld, M, w, d_piv, gcol, st);
   const int w1 = std::max(2, (w / 2) & ~1);
   const int w2 = w - w1;
   if (lu_panel_factor_t(P, ld, M, w1, d_piv, gcol, st) != FLA_SUCCESS) return FLA_FAILURE;

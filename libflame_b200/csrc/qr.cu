@@ -175,20 +175,6 @@ __global__ void __launch_bounds__(QR_THREADS) qr_panel_kernel(QrPanelArgs a) {
     for (int i = tid; i < rows; i += QR_THREADS) a.P[(long)(r0 + i) + (long)col * a.ld] = S[i + col * lds];
 }
 
-// Uw (M x b, ld ldu) := unit lower trapezoid of P (M x b): ones on the
-// diagonal, zeros above, P below.
-__global__ void form_unit_lower_kernel(const double* __restrict__ P, long ldp, double* __restrict__ U,
-                                       long ldu, int M, int b) {
-  const long idx = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long total = (long)M * b;
-  if (idx >= total) return;
-  const int col = (int)(idx / M), row = (int)(idx % M);
-  double v = 0.0;
-  if (row > col) v = P[row + (long)col * ldp];
-  else if (row == col) v = 1.0;
-  U[row + (long)col * ldu] = v;
-}
-
 // Copy the b_alg x b_alg diagonal blocks of Tbig (cols x cols, ld ldb)
 // into T's columns [k, k+cols) (T is b_alg x n, ld ldt); only the upper
 // triangles.

@@ -38,29 +38,22 @@ __device__ __forceinline__ double coef(const double* S, int r, int j) {
   return TRANS ? S[j + r * LDT] : S[r + j * LDT];
 }
 
-template <bool LOWER, bool TRANS, bool UNIT, bool RIGHT>
+template <bool LOWER, bool TRANS, bool UNIT>
 __global__ void __launch_bounds__(THREADS) trsm_tile_kernel(const double* __restrict__ T, long ldt,
                                                             double* __restrict__ X, long ldx, int b,
-                                                            int nvec, const int* guard) {
+                                                            int nvec) {
   extern __shared__ double sm[];
   double* ST = sm;                    // b x b triangle (stored part only)
   double* SX = ST + TB * LDT;         // NV right-hand sides, SX[r + v*LDX]
   double* sx = SX + NV * LDX;         // scaled current unknown per rhs
   double* sd = sx + NV;               // reciprocal diagonal
-  if (guard && *((volatile const int*)guard) != 0x7fffffff) return;
   constexpr bool FWD = (LOWER != TRANS);
   const int tid = threadIdx.x;
   const int v0 = blockIdx.x * NV;
   const int nv = min(NV, nvec - v0);
   load_block_f64<THREADS, true>(T, ldt, b, ST, LDT, [](int r, int c) { return LOWER ? (r >= c) : (r <= c); });
-  // right-hand side v, unknown r: left -> X(r, v0+v); right -> X(v0+v, r)
-  if (!RIGHT) {
-    for (int v = tid >> 5; v < nv; v += THREADS / 32)
-      for (int r = tid & 31; r < b; r += 32) SX[r + v * LDX] = X[r + (long)(v0 + v) * ldx];
-  } else {
-    for (int r = tid >> 6; r < b; r += THREADS / 64)
-      for (int v = tid & 63; v < nv; v += 64) SX[r + v * LDX] = X[(long)(v0 + v) + (long)r * ldx];
-  }
+  for (int v = tid >> 5; v < nv; v += THREADS / 32)
+    for (int r = tid & 31; r < b; r += 32) SX[r + v * LDX] = X[r + (long)(v0 + v) * ldx];
   __syncthreads();
   if (!UNIT)
     for (int j = tid; j < b; j += THREADS) sd[j] = 1.0 / ST[j + j * LDT];
@@ -92,13 +85,8 @@ __global__ void __launch_bounds__(THREADS) trsm_tile_kernel(const double* __rest
     }
     __syncthreads();
   }
-  if (!RIGHT) {
-    for (int v = tid >> 5; v < nv; v += THREADS / 32)
-      for (int r = tid & 31; r < b; r += 32) X[r + (long)(v0 + v) * ldx] = SX[r + v * LDX];
-  } else {
-    for (int r = tid >> 6; r < b; r += THREADS / 64)
-      for (int v = tid & 63; v < nv; v += 64) X[(long)(v0 + v) + (long)r * ldx] = SX[r + v * LDX];
-  }
+  for (int v = tid >> 5; v < nv; v += THREADS / 32)
+    for (int r = tid & 31; r < b; r += 32) X[r + (long)(v0 + v) * ldx] = SX[r + v * LDX];
 }
 
 // X := inv(T) for a b x b triangular T (b <= 128), one warp per column of X.
@@ -385,30 +373,22 @@ __global__ void __launch_bounds__(256, 2) trsm_sweep_kernel(SweepArgs<TF, TV> a)
   }
 }
 
-template <bool L, bool T, bool U, bool R>
+template <bool L, bool T, bool U>
 void set_attr_one() {
-  cudaFuncSetAttribute(trsm_tile_kernel<L, T, U, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM);
+  cudaFuncSetAttribute(trsm_tile_kernel<L, T, U>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM);
 }
 
 bool g_attr = false;
 void set_attrs() {
   if (g_attr) return;
-  set_attr_one<true, false, true, false>();
-  set_attr_one<true, false, false, false>();
-  set_attr_one<true, true, true, false>();
-  set_attr_one<true, true, false, false>();
-  set_attr_one<false, false, true, false>();
-  set_attr_one<false, false, false, false>();
-  set_attr_one<false, true, true, false>();
-  set_attr_one<false, true, false, false>();
-  set_attr_one<true, false, false, true>();
-  set_attr_one<true, false, true, true>();
-  set_attr_one<true, true, false, true>();
-  set_attr_one<true, true, true, true>();
-  set_attr_one<false, false, false, true>();
-  set_attr_one<false, false, true, true>();
-  set_attr_one<false, true, false, true>();
-  set_attr_one<false, true, true, true>();
+  set_attr_one<true, false, true>();
+  set_attr_one<true, false, false>();
+  set_attr_one<true, true, true>();
+  set_attr_one<true, true, false>();
+  set_attr_one<false, false, true>();
+  set_attr_one<false, false, false>();
+  set_attr_one<false, true, true>();
+  set_attr_one<false, true, false>();
   cudaFuncSetAttribute(tri_inv_kernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)INV_SMEM);
   cudaFuncSetAttribute(tri_inv_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)INV_SMEM);
   cudaFuncSetAttribute(tri_inv_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)INV_SMEM);
@@ -503,7 +483,7 @@ int trsm_block(const double* T, long ldt, double* B, long ldb, int b, long n, bo
   const unsigned grid = (unsigned)((n + NV - 1) / NV);
   const int ps = prof_begin(st);
 #define FB_TRSM_LAUNCH(L, T_, U) \
-  trsm_tile_kernel<L, T_, U, false><<<grid, THREADS, SMEM, st>>>(T, ldt, B, ldb, b, (int)n, nullptr)
+  trsm_tile_kernel<L, T_, U><<<grid, THREADS, SMEM, st>>>(T, ldt, B, ldb, b, (int)n)
   if (lower) {
     if (!trans) { if (unit) FB_TRSM_LAUNCH(true, false, true); else FB_TRSM_LAUNCH(true, false, false); }
     else        { if (unit) FB_TRSM_LAUNCH(true, true, true);  else FB_TRSM_LAUNCH(true, true, false); }
@@ -513,22 +493,6 @@ int trsm_block(const double* T, long ldt, double* B, long ldb, int b, long n, bo
   }
 #undef FB_TRSM_LAUNCH
   prof_end(ps, st, PROF_TRSM, (double)b * (double)b * (double)n);
-  count_launch();
-  FB_CK(cudaGetLastError());
-  return FLA_SUCCESS;
-}
-
-// X := X inv(L)^T for an m x b block X, L b x b lower non-unit (b <= 128);
-// the kernel returns at once when *guard no longer holds INT_MAX.
-int trsm_right_lt_block(const double* L, long ldl, double* X, long ldx, long m, int b, const int* guard,
-                        cudaStream_t st) {
-  set_attrs();
-  if (m <= 0 || b <= 0) return FLA_SUCCESS;
-  const unsigned grid = (unsigned)((m + NV - 1) / NV);
-  const int ps = prof_begin(st);
-  // X L^T = B  <=>  L X^T = B^T: a forward solve with L per row of X
-  trsm_tile_kernel<true, false, false, true><<<grid, THREADS, SMEM, st>>>(L, ldl, X, ldx, b, (int)m, guard);
-  prof_end(ps, st, PROF_TRSM, (double)m * (double)b * (double)b);
   count_launch();
   FB_CK(cudaGetLastError());
   return FLA_SUCCESS;
@@ -551,30 +515,6 @@ int tri_inverse_lower(const double* L, long ldl, int b, bool unit, double* X, lo
   return tri_inverse(L, ldl, b, true, unit, X, ldx, st);
 }
 
-
-// Every row x of the m x b block X := solution y of op(T) y = x, i.e.
-// X := X inv(op(T))^T (T b x b, b <= 128).
-int trsm_right_block(const double* T, long ldt, double* X, long ldx, long m, int b, bool lower, bool trans,
-                     bool unit, cudaStream_t st) {
-  set_attrs();
-  if (m <= 0 || b <= 0) return FLA_SUCCESS;
-  const unsigned grid = (unsigned)((m + NV - 1) / NV);
-  const int ps = prof_begin(st);
-#define FB_TRSM_R(L, T_, U) \
-  trsm_tile_kernel<L, T_, U, true><<<grid, THREADS, SMEM, st>>>(T, ldt, X, ldx, b, (int)m, nullptr)
-  if (lower) {
-    if (!trans) { if (unit) FB_TRSM_R(true, false, true); else FB_TRSM_R(true, false, false); }
-    else        { if (unit) FB_TRSM_R(true, true, true);  else FB_TRSM_R(true, true, false); }
-  } else {
-    if (!trans) { if (unit) FB_TRSM_R(false, false, true); else FB_TRSM_R(false, false, false); }
-    else        { if (unit) FB_TRSM_R(false, true, true);  else FB_TRSM_R(false, true, false); }
-  }
-#undef FB_TRSM_R
-  prof_end(ps, st, PROF_TRSM, (double)m * (double)b * (double)b);
-  count_launch();
-  FB_CK(cudaGetLastError());
-  return FLA_SUCCESS;
-}
 
 // X := inv(T) for a b x b triangular T: one warp per column when b <= 128,
 // else X := I and the blocked left solve.
