@@ -117,15 +117,12 @@ __global__ void __cluster_dims__(ADJ_CL, 1, 1) __launch_bounds__(ADJ_THREADS)
       const int i = (e & (AB / 2 - 1)) * 2, j = e >> 6;
       double* d = sX + i + j * ADJ_LD;
       if (vec && i > j && i + 1 < w) {
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(d)), "l"(src + i + (long)j * lds)
-                     : "memory");
+        cp_async16(d, src + i + (long)j * lds, 16);
       } else {
 #pragma unroll
         for (int u = 0; u < 2; ++u) {
           if (in(i + u, j))
-            asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(d + u)),
-                         "l"(src + i + u + (long)j * lds)
-                         : "memory");
+            cp_async8(d + u, src + i + u + (long)j * lds);
           else d[u] = 0.0;
         }
       }

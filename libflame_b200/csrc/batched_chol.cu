@@ -51,10 +51,6 @@ struct ChB {
   static constexpr int MINB = NT == 256 ? 2 : 1;
 };
 
-__device__ __forceinline__ void cp_async8(double* dst, const double* src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
-}
-
 // Entries s .. s + 7 of row r of the panel less the products of its columns
 // before s with the diagonal block's rows.
 template <int LD>

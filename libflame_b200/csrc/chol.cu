@@ -55,10 +55,6 @@ __device__ __forceinline__ bool guard_failed(const int* info) {
 // 370 cycles a column); with four instead of twelve warps for the products
 // n = 128 took 32.4 us.  With the block's rows stored after the CTA barrier
 // instead of the arrivals, n = 1024 (eight blocks) took 336 us, now 325.
-__device__ __forceinline__ void cp_async8(double* dst, const double* src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
-}
-
 __global__ void __launch_bounds__(POTRF_THREADS, 1) potrf_diag_kernel(double* A, long ld, int b, int gcol,
                                                                    int* info) {
   chain_begin();

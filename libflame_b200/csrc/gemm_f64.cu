@@ -626,9 +626,7 @@ __global__ void __launch_bounds__(256) gemm_tn_small_kernel(const double* __rest
     for (int e = tid; e < KC * D; e += 256) {
       const int r = e % KC, c = e / KC;
       if (r < rows && c < cols)
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(S + r + c * LD)),
-                     "l"(X + (k0 + r) + (long)c * ldx)
-                     : "memory");
+        cp_async8(S + r + c * LD, X + (k0 + r) + (long)c * ldx);
       else
         S[r + c * LD] = 0.0;
     }

@@ -39,10 +39,6 @@ constexpr int MID_THREADS = 512;
 constexpr int MID_COLS = 8;
 constexpr size_t MID_SMEM = sizeof(double) * ((size_t)AS * ALD + 3 * MID_COLS * ALD);
 
-__device__ __forceinline__ void cp_async8(double* dst, const double* src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
-}
-
 // Partial Gram matrices: slice z = blockIdx.x of super-block q = blockIdx.y
 // adds U(rows, :)^T U(rows, :) over the slabs z, z + gridDim.x, ... of GK
 // rows of its trapezoid (unit diagonal, zeros above) and writes the tiles on

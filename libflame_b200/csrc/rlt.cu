@@ -45,10 +45,6 @@ size_t rlt_smem(int b) {
   return sizeof(double) * ((size_t)bp * RLD + (size_t)bp * rlt_ldx<ROWS>() + RB);
 }
 
-__device__ __forceinline__ void cp_async8(double* dst, const double* src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
-}
-
 // X(:, c) -= X(:, kb..kb+15) L(c, kb..kb+15)^T for the 8-column tiles from c_lo
 // up to c_hi, the tiles of 8 rows dealt to nw warps, w the calling one.
 template <int ROWS>

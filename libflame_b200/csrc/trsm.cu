@@ -190,11 +190,6 @@ struct SweepTile {
   static constexpr size_t SMEM = sizeof(TF) * (2 * HALF + FULL) + sizeof(double) * 2 * SC * SLD;
 };
 
-// 16 bytes, the first `bytes` of them from src, the rest zero
-__device__ __forceinline__ void cp_async16(void* dst, const void* src, int bytes) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(bytes) : "memory");
-}
-
 template <typename TF, typename TV>
 struct SweepArgs {
   const TF* T;     // n x n triangle, ld ldt
