@@ -144,7 +144,7 @@ __global__ void __launch_bounds__(NT, ChB<NT>::MINB) chol_batched_f64_kernel(Bat
           if (lane >= s) store8<LD>(P, lane, s, x);
           __syncwarp();
           double l[36], ri[8];
-          const int f = chol8_load_factor(P + s + s * LD, LD, l, ri, [] {});
+          const int f = chol8_load_factor(P + s + s * LD, LD, l, ri);
           chol8_solve(l, ri, x);
           __syncwarp();
           if (lane >= s) store8<LD>(P, lane, s, x);

@@ -45,7 +45,7 @@ __device__ __forceinline__ bool guard_failed(const int* info) {
 //       then solves its own rows against it (dtrsm's R,L,T,N order); rows of
 //       the block itself come out of the same formulas, and the warp that owns
 //       them stores them once the other warps have announced (bar.arrive) that
-//       they have read the block;
+//       they have factored the block, every entry read and used;
 //       meanwhile the other warps subtract the previous step's products from the
 //       columns beyond this step on the FP64 tensor cores;
 //   (b) the rows lose this step's products in the next step's eight columns.
@@ -54,7 +54,8 @@ __device__ __forceinline__ bool guard_failed(const int* info) {
 // factored by one warp (lane = row, the column through shared memory, about
 // 370 cycles a column); with four instead of twelve warps for the products
 // n = 128 took 32.4 us.  With the block's rows stored after the CTA barrier
-// instead of the arrivals, n = 1024 (eight blocks) took 336 us, now 325.
+// instead of the arrivals, n = 1024 (eight blocks) took 336 us, 330 so (324 to
+// 328 with the arrivals right after the loads).
 __global__ void __launch_bounds__(POTRF_THREADS, 1) potrf_diag_kernel(double* A, long ld, int b, int gcol,
                                                                    int* info) {
   chain_begin();

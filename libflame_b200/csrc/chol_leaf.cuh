@@ -12,9 +12,8 @@ namespace {
 // aligned, ld even) factored by every lane alike: l[i (i + 1) / 2 + k] =
 // L(i, k) off the diagonal, ri[k] = 1 / L(k, k).  Returns the first column
 // whose pivot is not > 0 (NaN included), -1 if none; what follows it is not
-// meaningful then.  loaded(): called between the loads and the factorization.
-template <class F>
-__device__ __forceinline__ int chol8_load_factor(const double* D, int ld, double (&l)[36], double (&ri)[8], F loaded) {
+// meaningful then.
+__device__ __forceinline__ int chol8_load_factor(const double* D, int ld, double (&l)[36], double (&ri)[8]) {
 #pragma unroll
   for (int k = 0; k < 8; ++k)
 #pragma unroll
@@ -23,7 +22,6 @@ __device__ __forceinline__ int chol8_load_factor(const double* D, int ld, double
       if (i >= k) l[i * (i + 1) / 2 + k] = v.x;
       l[(i + 1) * (i + 2) / 2 + k] = v.y;
     }
-  loaded();
   int fail = -1;
 #pragma unroll
   for (int k = 0; k < 8; ++k) {
@@ -114,12 +112,11 @@ __device__ __forceinline__ int potrf_block(double* S, int b, int* s_fail) {
     if (warp < 4) {
       if ((warp << 5) + 31 >= jb) {  // (a) (warps whose rows are all done skip it)
         double l[36], ri[8];
-        const int fail = chol8_load_factor(S + jb + jb * POTRF_LD, POTRF_LD, l, ri, [&] {
-          if (warp != jb >> 5) bar_arrive(2, 128 - (jb & ~31));
-        });
+        const int fail = chol8_load_factor(S + jb + jb * POTRF_LD, POTRF_LD, l, ri);
         // the warp that owns the block's rows stores them below: not before
         // the others have read the block
         if (warp == jb >> 5) bar_sync(2, 128 - (jb & ~31));
+        else bar_arrive(2, 128 - (jb & ~31));
         if (tid == jb && fail >= 0 && jb + fail < b) *flag = jb + fail;  // rows past b: not pivots
         if (own) {
 #pragma unroll

@@ -1,8 +1,6 @@
-// Triangular solves with one diagonal block (b <= 128) on the GPU.
-//
-//   left:  X := inv(op(T)) X   for a b x n block X      (LU: A12 := inv(L11) A12,
-//                                                      solves, QR: W := T^-T W)
-//   right: X := X inv(L)^T     for an m x b block X      (Chol: A21 := A21 inv(L11)^T)
+// Left triangular solves X := inv(op(T)) X on the GPU: with one diagonal block
+// (b <= 128, trsm_block), of a whole triangle in one launch (trsm_sweep), and
+// the inverses of triangles and of their diagonal blocks.
 //
 // Replaces the dtrsm_ calls of the reference's blocked algorithms
 // (FLA_Trsm_external, src/base/flamec/wrappers/blas/3/external/
@@ -11,11 +9,10 @@
 // multiplication by the reciprocal of the pivot (as dtrsm's R,L,T,N case,
 // src/flablas/f2c/dtrsm.c).
 //
-// One CTA owns 64 right-hand sides (columns of X for left, rows for right),
-// kept in shared memory with the triangle, and sweeps the b steps: scale the
-// current unknown (one thread per right-hand side), then update the
-// remaining unknowns (all threads).  The step loop is not unrolled, so the
-// kernel stays small in the instruction cache.
+// trsm_block: one CTA owns 64 columns of X, kept in shared memory with the
+// triangle, and sweeps the b steps: scale the current unknown (one thread per
+// right-hand side), then update the remaining unknowns (all threads).  The step
+// loop is not unrolled, so the kernel stays small in the instruction cache.
 #include <algorithm>
 
 #include "common.h"
@@ -321,8 +318,10 @@ __global__ void __launch_bounds__(256, 2) trsm_sweep_kernel(SweepArgs<TF, TV> a)
       }
       if (u & 1) {
         // a tile's sum leaves the right-hand side at once: one sum over all
-        // tiles doubles the error of the solution at n = 8192 (6.4e-13 against
-        // 3.0e-13; 3.2e-13 with the blocked updates this kernel replaced)
+        // tiles doubled the error of the solution (one matrix of n = 8192:
+        // 6.4e-13 against 3.0e-13).  Over eight matrices, factor and solve
+        // together: backward error 1.07e-15, 1.29e-15 with the blocked updates
+        // this kernel replaced
 #pragma unroll
         for (int h = 0; h < 2; ++h)
 #pragma unroll
