@@ -54,8 +54,11 @@ def parse():
     ap.add_argument("--batch-count", type=int, default=10000)
     ap.add_argument("--ir-n", type=int, default=16384)
     ap.add_argument("--profile-op", default=None,
-                    choices=["lu", "chol", "qr", "apply_q", "mixed_spd", "mixed_general", "batched_chol"],
+                    choices=["lu", "chol", "qr", "apply_q", "mixed_spd", "mixed_general", "batched_chol", "batched_lu",
+                             "lu_solve", "adjoint"],
                     help="run one operation twice at order --n (for ncu captures) and exit")
+    ap.add_argument("--batch-order", type=int, default=0,
+                    help="order of every matrix of a profiled batch (0: uniform in 8..512)")
     return ap.parse_args()
 
 
@@ -64,7 +67,10 @@ def profile_op(args):
     would look at), for ncu: lu / chol (FLA_LU_piv / FLA_Chol on n x n),
     qr / apply_q (FLA_QR_UT on 2n x n, then FLA_Apply_Q_UT on 64 columns),
     mixed_spd / mixed_general (the default mixed solvers, 32 right-hand
-    sides, kappa 1e2), batched_chol (n matrices of orders U{8..512}).
+    sides, kappa 1e2), batched_chol / batched_lu (n matrices of orders
+    U{8..512}, or of order --batch-order, 4 right-hand sides), lu_solve
+    (FLA_LU_piv, then FLA_LU_piv_solve of 32 right-hand sides), adjoint
+    (FLA_Chol, then FLA_Chol_adjoint).
     Prints one JSON line with the device times of the calls."""
     import torch
     import libflame_b200 as F
@@ -108,14 +114,31 @@ def profile_op(args):
                 r = F.chol_solve_mixed(A, B, X, F.FLA_LOWER_TRIANGULAR)[0]
             else:
                 r = F.lu_piv_solve_mixed(A, B, X)[0]
+        elif args.profile_op == "lu_solve":
+            A = colmajor(torch.rand((n, n), dtype=torch.float64, device=dev, generator=g) * 2 - 1)
+            p = torch.zeros(n, dtype=torch.int32, device=dev)
+            r = F.lu_piv(A, p)
+            B = colmajor(torch.randn((n, 32), dtype=torch.float64, device=dev, generator=g))
+            if r == F.FLA_SUCCESS:
+                r = F.lu_piv_solve(A, p, B, torch.empty_like(B))
+        elif args.profile_op == "adjoint":
+            G = torch.randn((n, n), dtype=torch.float64, device=dev, generator=g)
+            A = colmajor(G @ G.t() / n + torch.eye(n, dtype=torch.float64, device=dev))
+            r = F.chol(A)
+            if r == F.FLA_SUCCESS:
+                r = F.chol_adjoint(A, colmajor(torch.randn((n, n), dtype=torch.float64, device=dev, generator=g)))
         else:
+            kind = args.profile_op.split("_")[1]
             rng = np.random.default_rng(5)
-            mats = []
-            for m in rng.integers(8, 513, size=n):
-                m = int(m)
+            sizes = [args.batch_order] * n if args.batch_order else rng.integers(8, 513, size=n).tolist()
+            mats, rhs = [], []
+            for m in sizes:
                 G = torch.randn((m, m), dtype=torch.float64, device=dev, generator=g)
-                mats.append(colmajor(G @ G.t() / m + torch.eye(m, dtype=torch.float64, device=dev)))
-            r = F.batched("chol", mats)[0]
+                mats.append(colmajor(G @ G.t() / m + torch.eye(m, dtype=torch.float64, device=dev))
+                            if kind == "chol" else colmajor(G))
+                rhs.append(colmajor(torch.randn((m, 4), dtype=torch.float64, device=dev, generator=g)))
+            pivs = [torch.zeros(m, dtype=torch.int32, device=dev) for m in sizes]
+            r = F.batched(kind, mats, pivs=pivs if kind == "lu" else None, rhs=rhs)[0]
         torch.cuda.synchronize()
         if r != F.FLA_SUCCESS:
             raise RuntimeError("%s failed: %s" % (args.profile_op, F.last_error()))
