@@ -508,7 +508,7 @@ def batched_section(torch, dev, F, count):
                     "failed": int((info != -1).sum())}
         del src, work, bsrc, bwork, pivbuf
         torch.cuda.empty_cache()
-    out["note"] = ("FP64 Cholesky: DMMA (FP64 tensor-core) left-looking kernel; FP32 Cholesky and LU: SIMT FMA "
+    out["note"] = ("FP64 Cholesky and LU: right-looking kernels, updates on DMMA (FP64 tensor cores); FP32: SIMT FMA "
                    "kernels; one CTA per matrix, persistent grid, largest first; tflops includes the solves")
     return out
 

@@ -1,5 +1,7 @@
 // Batched Cholesky and LU with partial pivoting (+ solves) for many small
-// matrices of uneven sizes (n <= 512) in one persistent launch.
+// matrices of uneven sizes: the dispatch, the FP32 kernels (orders up to 512)
+// and the FP64 Cholesky of orders 513 to 1024.  FP64 to order 512 is in
+// batched_chol.cu and batched_lu.cu.
 //
 // No counterpart in the reference (which factors one FLA_Obj at a time:
 // FLA_Chol, src/lapack/dec/chol/front/flamec/FLA_Chol.c:16-29; FLA_LU_piv,
@@ -9,11 +11,12 @@
 // LU with the largest-magnitude pivot, the first row among equals, zero
 // pivot columns left unscaled and the first reported, relative pivots.
 //
-// Design: a persistent grid (one CTA per SM) takes matrices from an atomic
-// counter in a host-chosen order (largest first, so the tail of the
-// schedule holds the small ones).  A CTA factors one matrix at a time,
-// left-looking in panels of nb columns (nb per size bin, from the batched
-// autotuner): the panel is loaded into shared memory, updated by all the
+// Every kernel is a persistent grid that takes matrices from an atomic counter
+// in a host-chosen order (largest first, so the tail of the schedule holds the
+// small ones).  FP64: up to three launches on the two streams (orders above
+// 512, 257 to 512, up to 256 with two CTAs per SM).  FP32: one launch, one CTA
+// per SM; a CTA factors one matrix at a time, left-looking in panels of nb
+// columns (nb per size bin, from the batched autotuner): the panel is loaded into shared memory, updated by all the
 // previous columns with register-tiled FMAs (the previous columns streamed
 // through shared memory in chunks of 8), factored there, and written back;
 // every matrix is read from HBM about n/(2 nb) times instead of n/nb times
@@ -165,7 +168,7 @@ __device__ void block_solve(const T* F, long ld, int n, T* X, int nrhs, bool low
 }
 
 // ---------------------------------------------------------------------------
-// Cholesky
+// Cholesky (FP32)
 // ---------------------------------------------------------------------------
 template <typename T>
 __global__ void __launch_bounds__(BT, 1) chol_batched_kernel(BatchArgs<T> a) {
@@ -249,7 +252,7 @@ __global__ void __launch_bounds__(BT, 1) chol_batched_kernel(BatchArgs<T> a) {
 }
 
 // ---------------------------------------------------------------------------
-// FP64 Cholesky, orders up to 1024, updates on the FP64 tensor cores
+// FP64 Cholesky, orders 513 to 1024, updates on the FP64 tensor cores
 // ---------------------------------------------------------------------------
 // One CTA of 16 warps per matrix (persistent over the schedule), left-looking
 // in panels of 32 columns:
@@ -495,7 +498,7 @@ __global__ void __launch_bounds__(DT, 1) chol_batched_dmma_kernel(BatchArgs<doub
 }
 
 // ---------------------------------------------------------------------------
-// LU with partial pivoting
+// LU with partial pivoting (FP32)
 // ---------------------------------------------------------------------------
 template <typename T>
 __global__ void __launch_bounds__(BT, 1) lu_batched_kernel(BatchArgs<T> a) {
@@ -658,7 +661,7 @@ template <typename T>
 int launch_batched(bool lu, BatchArgs<T> args, cudaStream_t st) {
   const int grid = std::min(ctx().num_sms, std::max(1, args.count));
   if constexpr (sizeof(T) == 8) {
-    // FP64 Cholesky: the DMMA kernel (orders up to 1024); the FP64 LU is
+    // FP64 Cholesky: the DMMA kernel (orders above 512); the FP64 LU is
     // batched_lu_f64
     static bool dattr = false;
     if (!dattr) {
@@ -933,7 +936,7 @@ int batched_entry(bool lu, int count, const int* n, T** A, const int* lda, int**
     set_last_error("batched: nrhs must be 0.." + std::to_string(BMAXRHS));
     return FLA_FAILURE;
   }
-  const int maxn = (!lu && sizeof(T) == 8) ? DMAXN : BMAXN;  // FP64 Cholesky: the DMMA kernel
+  const int maxn = (!lu && sizeof(T) == 8) ? DMAXN : BMAXN;  // FP64 Cholesky
   for (int i = 0; i < count; ++i) {
     if (n[i] < 0 || n[i] > maxn || lda[i] < std::max(1, n[i]) || (nrhs > 0 && ldb[i] < std::max(1, n[i]))) {
       set_last_error("batched: matrix " + std::to_string(i) + " has n outside 0.." + std::to_string(maxn) +

@@ -8,7 +8,8 @@
 // relative pivots.
 //
 // Right-looking in panels of 32 columns on a row-major copy of [A | B] in the
-// CTA's own workspace (at most 2.3 MB, so the copies of all CTAs stay in L2):
+// CTA's own workspace (the copies of all CTAs fit in L2 up to order 200 with two
+// CTAs per SM, from 257 to 310 with one; at order 512 they are 325 MB):
 //   panel      rows j..n in registers, one row per thread (lu_leaf.cuh): per
 //              column two CTA barriers and an update without memory traffic;
 //   exchanges  the composition of the panel's interchanges moves whole rows
@@ -18,9 +19,10 @@
 //              L21 and a chunk of U12 in shared memory).
 // The right-hand sides are columns of the copy, so the forward substitution
 // and the row exchanges come with the factorization; the backward one follows.
-// HBM sees each matrix once in and once out.  Bound by the latency of the
-// panels' columns (about 0.5 us each) and, for the large orders, the FP64
-// rate.  Orders up to 256 run in CTAs of 256 threads, two per SM, so that one
+// Bound by the latency of the panels' columns (1 us each at order 512) and, for
+// the large orders, the copies' traffic: 148 matrices of order 512 move 5.4 GB
+// through HBM (0.6 GB in and out would do; 52 % of the accesses hit L2), 2.5 ms
+// at 27 % of its bandwidth.  Orders up to 256 run in CTAs of 256 threads, two per SM, so that one
 // matrix's panel overlaps the other's updates; larger ones in CTAs of 512.
 // Measured: 2500 matrices, n uniform in 8..512, 4 right-hand sides: 47.4 ms
 // with a left-looking panel in shared memory on FP64 FMAs (ten barriers and a

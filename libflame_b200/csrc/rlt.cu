@@ -20,9 +20,10 @@
 // kernel, nugget 1e-9: ||A - L L^T|| / ||A|| 2.6e-15 with 32 x 32 inverses,
 // 1.5e-16 so; an LU whose 32 x 32 blocks are near -1 below the diagonal 1.1e-8
 // and 1.2e-16), and an infinite entry spoils columns before its own.  FLA_Chol
-// n = 1024 takes 327 us with inverses, 335 us so; FLA_LU_piv n = 3001 6.24 ms
-// both ways.  (A shuffle per column, a warp per row group: 896 x 128
-// 16.2 us against 10.2 with the inverses; a row per thread by 32 columns 17.8.)
+// n = 1024 takes 327 us with inverses, 335 us so (eight solves); FLA_LU_piv
+// n = 3001 6.24 ms both ways.  (A shuffle per column, a warp per row group:
+// 896 x 128 16.2 us against 10.2 with the inverses; a row per thread by 32
+// columns 17.8.)
 #include <algorithm>
 
 #include "common.h"
