@@ -62,21 +62,21 @@ print(a - held())
 
 
 def test_batched_lu_short_of_memory(cuda, flame):
-    """With 96 MB left the batched LU runs in fewer CTAs instead of failing."""
+    """With 192 MB left for 318 MB of copies the batched LU runs in fewer CTAs instead of failing."""
     ok = _run("""
-n, count = 500, 64
+n, count = 500, 148
 A = [torch.rand((n, n), dtype=torch.float64, device="cuda").t() for _ in range(count)]
 A0 = [a.t().clone().t() for a in A]
 P = [torch.zeros(n, dtype=torch.int32, device="cuda") for _ in range(count)]
 W = [a.t().clone().t()[:8, :8] for a in A[:2]]
 assert F.batched("lu", W, pivs=P[:2])[0] == F.FLA_SUCCESS
 x = A[0].t().clone().t() @ A0[0][:, 0]  # the products below: loaded before memory is short
-hog = torch.empty((torch.cuda.mem_get_info()[0] - (96 << 20)) // 8, dtype=torch.float64, device="cuda")
+hog = torch.empty((torch.cuda.mem_get_info()[0] - (192 << 20)) // 8, dtype=torch.float64, device="cuda")
 r, info = F.batched("lu", A, pivs=P)
 del hog
 assert r == F.FLA_SUCCESS and info == [-1] * count, F.last_error()
 worst = 0.0
-for a, a0, p in list(zip(A, A0, P))[::9]:
+for a, a0, p in list(zip(A, A0, P))[::21]:
     perm = list(range(n))
     for i, q in enumerate(p.tolist()):
         perm[i], perm[i + q] = perm[i + q], perm[i]
