@@ -53,6 +53,11 @@ int           FLA_B200_dgemm( int transa, int transb, long m, long n, long k, do
  * (about 3 m n doubles) and frees them before returning. */
 int           FLA_B200_gemm_concurrency_check( long m, long n, long k, int iters,
                                                unsigned long long* mismatches );
+/* Self-test of the time limit on the waits of the one-launch triangular
+ * solves: a small solve whose first block is left out runs into the limit (two
+ * seconds) and *expired becomes 1 when the library reports it; the solve after
+ * it has to succeed.  FLA_FAILURE if that one is wrong or reported. */
+int           FLA_B200_solve_wait_check( int* expired );
 
 /* No counterpart in the reference libflame.  LU factorization with partial
  * pivoting of one m x n panel (n <= 128, m >= n) held in device memory (A,

@@ -266,7 +266,7 @@ int laswp_dev(double* A, long ld, int row0, const int* d_piv, int npiv, int c0, 
 int trsm_left_dev(DMat T, DMat B, bool lower, bool trans, bool unit, cudaStream_t st);
 int trsm_block(const double* T, long ldt, double* B, long ldb, int b, long n, bool lower,
                bool trans, bool unit, cudaStream_t st);
-int trsm_sweep(DMat T, DMat B, bool lower, bool trans, bool unit, cudaStream_t st);
+int trsm_sweep(DMat T, DMat B, bool lower, bool trans, bool unit, cudaStream_t st, int first_task = 0);
 int trsm_sweep_f32(const float* F, long ldf, const float* Inv, const float* Y, float* X, long ldb, long n, long nr,
                    bool trans, bool bwd, cudaStream_t st);
 // X := inv(L), L b x b lower triangular (unit diagonal if unit), X ld ldx.

@@ -1,4 +1,7 @@
-// Concurrency self-test of the FP64 GEMM engine.
+// Self-tests: the FP64 GEMM engine beside panel work, and the time limit of the
+// triangular solve's waits (solve_wait_check, below).
+//
+// Concurrency of the GEMM engine.
 //
 // The factorizations run their trailing-update GEMM on the main stream
 // while the next panel is factored on the second stream, so the GEMM's CTAs
@@ -34,6 +37,11 @@ __global__ void st_fill_kernel(double* p, long n, unsigned seed, double scale) {
 __global__ void st_spd_kernel(double* p, int b) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < b) p[i + (long)i * b] += 2.0 * b;
+}
+
+__global__ void st_unit_diagonal_kernel(double* p, int n) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) p[i + (long)i * n] = 1.0;
 }
 
 __global__ void st_compare_kernel(const double* __restrict__ C, const double* __restrict__ R, long total,
@@ -143,9 +151,49 @@ int gemm_concurrency_check(long m, long n, long k, int iters, unsigned long long
   return FLA_SUCCESS;
 }
 
+// The waits of the one-launch triangular solve: a solve whose first block is
+// left out, so that every other block's wait for it runs out (2 s), is reported
+// as a failure by the synchronization that follows, and the next solve is
+// neither reported nor wrong.
+int solve_wait_check(int* expired) {
+  Context& cx = ctx();
+  cudaStream_t st = cx.stream;
+  const int n = 192;  // three blocks
+  Buffers mem;
+  double *T = mem.get((size_t)n * n), *B = mem.get((size_t)n * n), *X = mem.get((size_t)n * n);
+  unsigned long long* count = (unsigned long long*)mem.get(1);
+  if (!T || !B || !X || !count) {
+    set_last_error("FLA_B200_solve_wait_check: device allocation failed");
+    return FLA_FAILURE;
+  }
+  const size_t bytes = sizeof(double) * (size_t)n * n;
+  FB_CK(cudaMemsetAsync(T, 0, bytes, st));
+  st_unit_diagonal_kernel<<<1, n, 0, st>>>(T, n);
+  st_fill_kernel<<<64, 256, 0, st>>>(B, (long)n * n, 7, 1.0);
+  count_launch(2);
+  const DMat t{T, n, n, n}, x{X, n, n, 16};
+  FB_CK(cudaMemcpyAsync(X, B, bytes, cudaMemcpyDeviceToDevice, st));
+  if (trsm_sweep(t, x, true, false, false, st, 1) != FLA_SUCCESS) return FLA_FAILURE;
+  op_end(st);
+  *expired = sync_all() == FLA_FAILURE;
+  FB_CK(cudaMemcpyAsync(X, B, bytes, cudaMemcpyDeviceToDevice, st));
+  FB_CK(cudaMemsetAsync(count, 0, sizeof(*count), st));
+  if (trsm_sweep(t, x, true, false, false, st) != FLA_SUCCESS) return FLA_FAILURE;
+  st_compare_kernel<<<64, 256, 0, st>>>(X, B, (long)n * n, count);  // T is the identity
+  count_launch();
+  unsigned long long wrong = 0;
+  FB_CK(cudaMemcpyAsync(&wrong, count, sizeof(wrong), cudaMemcpyDeviceToHost, st));
+  if (sync_all() != FLA_SUCCESS) return FLA_FAILURE;
+  if (wrong != 0) {
+    set_last_error("FLA_B200_solve_wait_check: the solve after the one that was cut short is wrong");
+    return FLA_FAILURE;
+  }
+  return FLA_SUCCESS;
+}
+
 }  // namespace fb
 
-// C-ABI entry (include/FLAME_b200.h).
+// C-ABI entries (include/FLAME_b200.h).
 extern "C" int FLA_B200_gemm_concurrency_check(long m, long n, long k, int iters, unsigned long long* mismatches) {
   if (!mismatches || m <= 0 || n <= 0 || k <= 0 || iters < 0) {
     fb::set_last_error("FLA_B200_gemm_concurrency_check: invalid argument");
@@ -154,6 +202,18 @@ extern "C" int FLA_B200_gemm_concurrency_check(long m, long n, long k, int iters
   if (!fb::ctx().initialized) FLA_Init();
   fb::op_begin(fb::ctx().stream);  // also orders the call after the caller's default-stream work
   const int r = fb::gemm_concurrency_check(m, n, k, iters, mismatches);
+  if (r != FLA_SUCCESS) fb::sync_all();
+  return r;
+}
+
+extern "C" int FLA_B200_solve_wait_check(int* expired) {
+  if (!expired) {
+    fb::set_last_error("FLA_B200_solve_wait_check: invalid argument");
+    return FLA_FAILURE;
+  }
+  if (!fb::ctx().initialized) FLA_Init();
+  fb::op_begin(fb::ctx().stream);
+  const int r = fb::solve_wait_check(expired);
   if (r != FLA_SUCCESS) fb::sync_all();
   return r;
 }

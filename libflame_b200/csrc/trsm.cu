@@ -200,6 +200,7 @@ struct SweepArgs {
   double* XB;      // exchange buffer, nblk * SB x nr, all ones
   int n, nr, nblk;
   int* err;
+  int first;       // first task: 0 (the check of the waits leaves the first block unsolved)
 };
 
 // TRANS: op(T)(r, c) = T(c, r), op(Inv) alike.  BWD: blocks solved last to
@@ -280,7 +281,7 @@ __global__ void __launch_bounds__(256, 2) trsm_sweep_kernel(SweepArgs<TF, TV> a)
     *reinterpret_cast<double2*>(d) = make_double2(v[0], v[1]);
     *reinterpret_cast<double2*>(d + 2) = make_double2(v[2], v[3]);
   };
-  for (int task = blockIdx.x; task < nblk * ngrp; task += gridDim.x) {
+  for (int task = blockIdx.x + a.first; task < nblk * ngrp; task += gridDim.x) {
     const int q = task / ngrp, col0 = (task % ngrp) * SC, nc = min(SC, nr - col0);
     const int bi = BWD ? nblk - 1 - q : q, r0 = bi * SB;
     auto blk = [&](int j) { return BWD ? nblk - 1 - j : j; };
@@ -425,8 +426,9 @@ int sweep_launch(SweepArgs<TF, TV> a, bool trans, bool bwd, cudaStream_t st) {
 }
 
 // B := inv(op(T)) B by trsm_sweep_kernel: T n x n, B n x nr, T 16-byte
-// aligned with an even leading dimension.
-int trsm_sweep(DMat T, DMat B, bool lower, bool trans, bool unit, cudaStream_t st) {
+// aligned with an even leading dimension.  first_task > 0: only for
+// solve_wait_check.
+int trsm_sweep(DMat T, DMat B, bool lower, bool trans, bool unit, cudaStream_t st, int first_task) {
   const long n = T.m, nblk = (n + SB - 1) / SB;
   double* Inv = (double*)ws_get(WS_TRINV, sizeof(double) * (size_t)nblk * SB * SB);
   if (!Inv) return FLA_FAILURE;
@@ -443,6 +445,7 @@ int trsm_sweep(DMat T, DMat B, bool lower, bool trans, bool unit, cudaStream_t s
   a.ldb = B.ld;
   a.n = (int)n;
   a.nr = (int)B.n;
+  a.first = first_task;
   return sweep_launch(a, trans, lower == trans, st);
 }
 
